@@ -6,7 +6,8 @@
 //   k_fx       pre-scale by gsig, zero-pad in x, forward x-FFT          x   -> U1[kx][y][zc]
 //   k_fy       zero-pad in y, forward y-FFT, scatter to (q,r,slot)      U1  -> Uhat[q][r][4][zc]
 //   contraction per (q,r): 6 Green's blocks applied to the 4 points (+-kx,+-ky)   Uhat in place
-//              (contract.cu, TMA-pipelined; k_contract below is the generic fallback)
+//              (contract_mma.cu on the tensor cores; contract.cu's FP kernels as variants; k_contract below is the
+//              plain form, GIEM2G_GENERIC_CONTRACT=1)
 //   k_by       inverse y-FFT, crop y<Ny                                 Uhat -> U1
 //   k_bx       inverse x-FFT, crop x<Nx, post-combine                   U1  -> y
 // The transforms are four-step register FFTs (fft4.cuh) with one shared-memory transpose; zc = c*Nz+z
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fx(con
 template <typename R, int L, int CAP>
 __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(const CT<R> *__restrict__ U1, CT<R> *__restrict__ Uh,
                                                  const CT<R> *__restrict__ twg, int Nx, int Ny, int Nz, int NL,
-                                                 int nv, const int *gate)
+                                                 int nv, int pitch, const int *gate)
 {
     if (gate && *gate == 0) return;
     using C = CT<R>;
@@ -109,6 +110,9 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(con
     C *tw = reinterpret_cast<C *>(smem_raw);
     C *sm = tw + L;
     const int Z3 = nv * 3 * Nz, zc0 = blockIdx.x * NL, kx = blockIdx.y;  // Z3: lines of all vectors
+    // in the spectrum a vector's 3Nz lines are `pitch` elements apart from the next vector's
+    const int ZP = nv * pitch, gap = pitch - 3 * Nz;
+    auto zpos = [&](int t) { return zc0 + t + (zc0 + t >= 3 * Nz ? gap : 0); };
     const int nl = min(NL, Z3 - zc0);
     int q, sx;
     kx_to_slot(kx, Nx, q, sx);
@@ -117,19 +121,19 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(con
             const int t = i % nl, ky = i / nl;
             int r, sy;
             ky_to_slot(ky, Ny, r, sy);
-            Uh[(((size_t)q * Ny + r) * 4 + sx * 2 + sy) * Z3 + zc0 + t] = czero<C>();
+            Uh[(((size_t)q * Ny + r) * 4 + sx * 2 + sy) * ZP + zpos(t)] = czero<C>();
         }
         return;
     }
     load_tw(tw, twg, L);
     __syncthreads();
     const C *col = U1 + kx * Ny * Z3 + zc0;
-    C *dst = Uh + q * Ny * 4 * Z3 + sx * 2 * Z3 + zc0;
+    C *dst = Uh + q * Ny * 4 * ZP + sx * 2 * ZP;
     auto load = [&](int t, int yy) -> C { return col[yy * Z3 + t]; };
     auto store = [&](int t, int ky, C v) {
         int r, sy;
         ky_to_slot(ky, L / 2, r, sy);  // L = 2Ny: with the output index's range known, this folds per output
-        dst[(r * 4 + sy) * Z3 + t] = v;
+        dst[(r * 4 + sy) * ZP + zpos(t)] = v;
     };
     auto off = [&](int t, int n1, int k2) { return t + NL * (n1 + N1 * k2); };
     fft4step<C, N1, N2, false, true, false, true, true>(sm, nl, ilog2(NL), tw, load, store, off);
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(con
 template <typename R, int L, int CAP>
 __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_by(const CT<R> *__restrict__ Uh, CT<R> *__restrict__ U1,
                                                  const CT<R> *__restrict__ twg, int Nx, int Ny, int Nz, int NL,
-                                                 int nv, const int *gate)
+                                                 int nv, int pitch, const int *gate)
 {
     if (gate && *gate == 0) return;
     using C = CT<R>;
@@ -148,18 +152,21 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_by(con
     C *tw = reinterpret_cast<C *>(smem_raw);
     C *sm = tw + L;
     const int Z3 = nv * 3 * Nz, zc0 = blockIdx.x * NL, kx = blockIdx.y;  // Z3: lines of all vectors
+    // in the spectrum a vector's 3Nz lines are `pitch` elements apart from the next vector's
+    const int ZP = nv * pitch, gap = pitch - 3 * Nz;
+    auto zpos = [&](int t) { return zc0 + t + (zc0 + t >= 3 * Nz ? gap : 0); };
     if (kx == Nx) return;  // x-Nyquist column is read as zero by k_bx
     const int nl = min(NL, Z3 - zc0);
     int q, sx;
     kx_to_slot(kx, Nx, q, sx);
     load_tw(tw, twg, L);
     __syncthreads();
-    const C *src = Uh + q * Ny * 4 * Z3 + sx * 2 * Z3 + zc0;
+    const C *src = Uh + q * Ny * 4 * ZP + sx * 2 * ZP;
     C *col = U1 + kx * Ny * Z3 + zc0;
     auto load = [&](int t, int ky) -> C {
         int r, sy;
         ky_to_slot(ky, L / 2, r, sy);  // L = 2Ny: folds per input at compile time
-        return src[(r * 4 + sy) * Z3 + t];
+        return src[(r * 4 + sy) * ZP + zpos(t)];
     };
     auto store = [&](int t, int yy, C v) { col[yy * Z3 + t] = v; };
     auto off = [&](int t, int n1, int k2) { return t + NL * (n1 + N1 * k2); };
@@ -307,6 +314,7 @@ __global__ void k_sigma(const double2 *__restrict__ csiga, const double2 *__rest
 template <typename R> struct Bufs;
 template <> struct Bufs<double> {
     static const double2 *G(IeOp *o) { return o->d_tensor64; }
+    static const double2 *plain(IeOp *o) { return o->d_plain64; }
     static const double2 *gsig(IeOp *o) { return o->d_gsig64; }
     static const double2 *asig(IeOp *o) { return o->d_asig64; }
     static const double *post(IeOp *o) { return o->d_post64; }
@@ -315,6 +323,7 @@ template <> struct Bufs<double> {
 };
 template <> struct Bufs<float> {
     static const float2 *G(IeOp *o) { return o->d_tensor32; }
+    static const float2 *plain(IeOp *o) { return o->d_plain32; }
     static const float2 *gsig(IeOp *o) { return o->d_gsig32; }
     static const float2 *asig(IeOp *o) { return o->d_asig32; }
     static const float *post(IeOp *o) { return o->d_post32; }
@@ -331,9 +340,14 @@ static bool uses_ypipe(const IeOp *op, int form)
 
 int ie_kernel_launch_count_apply(const IeOp *op, int form) { return uses_ypipe(op, form) ? 3 : 5; }
 
-// elements of the spectrum of one vector, and the pipelined pass's counters after it (in 8-byte units, so
+bool ie_uses_mma(const IeOp *op, int form)
+{
+    return op->use_fast_contract && op->contract_variant[form] < 0 && !uses_ypipe(op, form);
+}
+
+// elements of the spectrum of one vector (at the larger of the two row pitches), and the pipelined pass's counters after it (in 8-byte units, so
 // the same count covers them behind a complex64 or a complex128 spectrum)
-static size_t spectrum_elems(const IeOp *op) { return (size_t)op->Nx * op->Ny * 4 * 3 * op->Nz; }
+static size_t spectrum_elems(const IeOp *op) { return (size_t)op->Nx * op->Ny * 4 * ie_spectrum_pitch(op->Nz); }
 static size_t ystate_elems(const IeOp *op) { return (ie_ypipe_state_bytes(op->Nx) + 7) / 8; }
 
 // lines per CTA: tile of at most ~100 KB of shared memory, power of two, <= 32
@@ -397,26 +411,26 @@ static void launch_x(bool fwd, IeOp *op, const VecSet<CT<R>> &vs, CT<R> *U1, cud
 }
 
 template <typename R, int L, int CAP>
-static void launch_y_k(bool fwd, IeOp *op, int nv, CT<R> *U1, CT<R> *Uh, cudaStream_t st, const int *gate,
+static void launch_y_k(bool fwd, IeOp *op, int nv, int pitch, CT<R> *U1, CT<R> *Uh, cudaStream_t st, const int *gate,
                        dim3 grid, int nt, size_t sm, int NL)
 {
     const int Nx = op->Nx, Ny = op->Ny, Nz = op->Nz;
     static bool attr = false;
     if (!attr) { big_smem(k_fy<R, L, CAP>); big_smem(k_by<R, L, CAP>); attr = true; }
-    if (fwd) k_fy<R, L, CAP><<<grid, nt, sm, st>>>(U1, Uh, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, gate);
-    else k_by<R, L, CAP><<<grid, nt, sm, st>>>(Uh, U1, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, gate);
+    if (fwd) k_fy<R, L, CAP><<<grid, nt, sm, st>>>(U1, Uh, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, pitch, gate);
+    else k_by<R, L, CAP><<<grid, nt, sm, st>>>(Uh, U1, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, pitch, gate);
 }
 
 template <typename R, int L>
-static void launch_y(bool fwd, IeOp *op, int nv, CT<R> *U1, CT<R> *Uh, cudaStream_t st, const int *gate)
+static void launch_y(bool fwd, IeOp *op, int nv, int pitch, CT<R> *U1, CT<R> *Uh, cudaStream_t st, const int *gate)
 {
     const int Nz = op->Nz, ZL = nv * 3 * Nz;
     const size_t es = sizeof(CT<R>);
     const int NL = lines_for(L, es, op->fft_lines[es == sizeof(double2) ? 0 : 1]), nt = threads_for(L, NL);
     const size_t sm = (size_t)(NL * (L + 1) + L) * es;
     dim3 grid((ZL + NL - 1) / NL, 2 * op->Nx);
-    if (use_cap<R, L>(nt)) launch_y_k<R, L, 1>(fwd, op, nv, U1, Uh, st, gate, grid, nt, sm, NL);
-    else launch_y_k<R, L, 0>(fwd, op, nv, U1, Uh, st, gate, grid, nt, sm, NL);
+    if (use_cap<R, L>(nt)) launch_y_k<R, L, 1>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, nt, sm, NL);
+    else launch_y_k<R, L, 0>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, nt, sm, NL);
 }
 
 template <typename R>
@@ -435,18 +449,18 @@ static void dispatch_x(bool fwd, IeOp *op, const VecSet<CT<R>> &vs, CT<R> *U1, c
     }
 }
 template <typename R>
-static void dispatch_y(bool fwd, IeOp *op, int nv, CT<R> *U1, CT<R> *Uh, cudaStream_t st, const int *gate)
+static void dispatch_y(bool fwd, IeOp *op, int nv, int pitch, CT<R> *U1, CT<R> *Uh, cudaStream_t st, const int *gate)
 {
     switch (2 * op->Ny) {
-    case 4: launch_y<R, 4>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 8: launch_y<R, 8>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 16: launch_y<R, 16>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 32: launch_y<R, 32>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 64: launch_y<R, 64>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 128: launch_y<R, 128>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 256: launch_y<R, 256>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 512: launch_y<R, 512>(fwd, op, nv, U1, Uh, st, gate); break;
-    case 1024: launch_y<R, 1024>(fwd, op, nv, U1, Uh, st, gate); break;
+    case 4: launch_y<R, 4>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 8: launch_y<R, 8>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 16: launch_y<R, 16>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 32: launch_y<R, 32>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 64: launch_y<R, 64>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 128: launch_y<R, 128>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 256: launch_y<R, 256>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 512: launch_y<R, 512>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
+    case 1024: launch_y<R, 1024>(fwd, op, nv, pitch, U1, Uh, st, gate); break;
     }
 }
 
@@ -458,10 +472,12 @@ static int ie_apply_core(IeOp *op, const CT<R> *d_in, CT<R> *d_out, cudaStream_t
 {
     const int Nx = op->Nx, Ny = op->Ny, Nz = op->Nz, Z3 = 3 * Nz;
     const size_t es = sizeof(CT<R>);
-    const CT<R> *G = Bufs<R>::G(op);
-    if (!G || !U1 || !Uh) return G2_ERR_STATE;
-    VecSet<CT<R>> vs{{d_in, nullptr}, {d_out, nullptr}, 1};
     const int form = sizeof(R) == 8 ? 0 : 1;
+    const bool mma = ie_uses_mma(op, form);
+    const CT<R> *G = mma ? Bufs<R>::G(op) : Bufs<R>::plain(op);
+    if (!G || !U1 || !Uh) return G2_ERR_STATE;
+    const int pitch = mma ? ie_spectrum_pitch(Nz) : Z3;
+    VecSet<CT<R>> vs{{d_in, nullptr}, {d_out, nullptr}, 1};
     // contraction (bracketed by events when kernel timing is on; never inside a stream capture)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool timed = op->time_contract && op->evc0 &&
@@ -479,10 +495,13 @@ static int ie_apply_core(IeOp *op, const CT<R> *d_in, CT<R> *d_out, cudaStream_t
         G2_CUDA_CHECK(cudaGetLastError());
         return G2_OK;
     }
-    dispatch_y<R>(true, op, 1, U1, Uh, st, gate);
+    dispatch_y<R>(true, op, 1, pitch, U1, Uh, st, gate);
     if (timed) cudaEventRecord(op->evc0, st);
     int rc_fast = G2_ERR_UNSUPPORTED;
-    if (op->use_fast_contract) {
+    if (mma) {
+        rc_fast = ie_contract_mma(form, G, Uh, Nx, Ny, Nz, op->d_err, st, gate);
+        if (rc_fast) return rc_fast;
+    } else if (op->use_fast_contract) {
         if (sizeof(R) == 8)
             rc_fast = ie_contract_fast64(reinterpret_cast<const double2 *>(G), reinterpret_cast<double2 *>(Uh), Nx, Ny,
                                          Nz, op->d_err, st, op->contract_variant[0], gate);
@@ -498,7 +517,7 @@ static int ie_apply_core(IeOp *op, const CT<R> *d_in, CT<R> *d_out, cudaStream_t
         k_contract<R><<<(unsigned)op->units(), threads, sm, st>>>(G, Uh, Nx, Ny, Nz, gate);
     }
     if (timed) cudaEventRecord(op->evc1, st);
-    dispatch_y<R>(false, op, 1, U1, Uh, st, gate);
+    dispatch_y<R>(false, op, 1, pitch, U1, Uh, st, gate);
     dispatch_x<R>(false, op, vs, U1, st, gate);
     g2_count_launches(5);
     G2_CUDA_CHECK(cudaGetLastError());
@@ -670,8 +689,12 @@ size_t ie_pair_scratch_elems(const IeOp *op, size_t *n_u1)
 int ie_apply_pair32(IeOp *op, const float2 *in0, const float2 *in1, float2 *out0, float2 *out1, cudaStream_t st,
                     float2 *U1, float2 *Uh)
 {
-    if (!op->use_fast_contract || !ie_contract_pair32_supported(op->Nx, op->Ny, op->Nz)) return G2_ERR_UNSUPPORTED;
-    if (!op->d_tensor32 || !U1 || !Uh) return G2_ERR_STATE;
+    const bool mma = ie_uses_mma(op, 2);
+    if (!mma && (!op->use_fast_contract || !ie_contract_pair32_supported(op->Nx, op->Ny, op->Nz)))
+        return G2_ERR_UNSUPPORTED;
+    const float2 *G = mma ? op->d_tensor32 : op->d_plain32;
+    if (!G || !U1 || !Uh) return G2_ERR_STATE;
+    const int pitch = mma ? ie_spectrum_pitch(op->Nz) : 3 * op->Nz;
     VecSet<float2> vs{{in0, in1}, {out0, out1}, 2};
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     const bool timed = op->time_contract && op->evc0 &&
@@ -680,7 +703,7 @@ int ie_apply_pair32(IeOp *op, const float2 *in0, const float2 *in1, float2 *out0
     if (uses_ypipe(op, 2)) {
         int *state = reinterpret_cast<int *>(Uh + 2 * spectrum_elems(op));
         if (timed) cudaEventRecord(op->evc0, st);
-        const int rc = ie_ypipe(op, 2, op->d_tensor32, U1, Uh, state, st, nullptr);
+        const int rc = ie_ypipe(op, 2, G, U1, Uh, state, st, nullptr);
         if (rc) return rc;
         if (timed) cudaEventRecord(op->evc1, st);
         dispatch_x<float>(false, op, vs, U1, st, nullptr);
@@ -688,13 +711,14 @@ int ie_apply_pair32(IeOp *op, const float2 *in0, const float2 *in1, float2 *out0
         G2_CUDA_CHECK(cudaGetLastError());
         return G2_OK;
     }
-    dispatch_y<float>(true, op, 2, U1, Uh, st, nullptr);
+    dispatch_y<float>(true, op, 2, pitch, U1, Uh, st, nullptr);
     if (timed) cudaEventRecord(op->evc0, st);
-    const int rc = ie_contract_pair32(op->d_tensor32, Uh, op->Nx, op->Ny, op->Nz, op->d_err, st, nullptr,
-                                      op->contract_variant[2]);
+    const int rc = mma ? ie_contract_mma(2, G, Uh, op->Nx, op->Ny, op->Nz, op->d_err, st, nullptr)
+                       : ie_contract_pair32(G, Uh, op->Nx, op->Ny, op->Nz, op->d_err, st, nullptr,
+                                            op->contract_variant[2]);
     if (rc) return rc;
     if (timed) cudaEventRecord(op->evc1, st);
-    dispatch_y<float>(false, op, 2, U1, Uh, st, nullptr);
+    dispatch_y<float>(false, op, 2, pitch, U1, Uh, st, nullptr);
     dispatch_x<float>(false, op, vs, U1, st, nullptr);
     g2_count_launches(5);
     G2_CUDA_CHECK(cudaGetLastError());

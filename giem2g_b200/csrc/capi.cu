@@ -244,7 +244,8 @@ int giem2g_set_ie_kernel_spatial(void *ie, const void *symm, const void *asym)
     return set_status(0);
 }
 
-static int get_units(IeOp *op, const double2 *d, void *symm, void *asym, int W = 1)
+// the unit tensor d in the reference's arrays; tiled: d is the spectral tensor (unit_pos), else the spatial one
+static int get_units(IeOp *op, const double2 *d, void *symm, void *asym, bool tiled)
 {
     const int P = op->P(), Nz = op->Nz, T = op->Tunit();
     const size_t U = op->units();
@@ -253,12 +254,11 @@ static int get_units(IeOp *op, const double2 *d, void *symm, void *asym, int W =
         cudaStreamSynchronize(op->stream) != cudaSuccess)
         return fail(G2_ERR_CUDA, "tensor download failed");
     double2 *s = reinterpret_cast<double2 *>(symm), *a = reinterpret_cast<double2 *>(asym);
+    std::vector<int> pos(T);
+    for (int e = 0; e < T; e++) pos[e] = tiled ? unit_pos<true>(e, Nz) : e;
     for (size_t u = 0; u < U; u++) {
-        std::memcpy(s + u * 4 * P, &h[u * T], sizeof(double2) * 4 * P);
-        for (int blk = 0; blk < 2; blk++)
-            for (int c = 0; c < Nz; c++)
-                for (int r = 0; r < Nz; r++)
-                    a[u * 2 * Nz * Nz + blk * Nz * Nz + c * Nz + r] = h[u * T + 4 * P + blk * Nz * Nz + asw(r, c, Nz, W)];
+        for (int e = 0; e < 4 * P; e++) s[u * 4 * P + e] = h[u * T + pos[e]];
+        for (int e = 4 * P; e < T; e++) a[u * 2 * Nz * Nz + e - 4 * P] = h[u * T + pos[e]];
     }
     return set_status(0);
 }
@@ -267,14 +267,14 @@ int giem2g_get_ie_kernel_spatial(void *ie, void *symm, void *asym)
 {
     IeOp *op = resolve(ie);
     if (!op || !op->have_spatial) return fail(G2_ERR_STATE, "giem2g_get_ie_kernel_spatial: no spatial tensor");
-    return get_units(op, op->d_spatial, symm, asym);
+    return get_units(op, op->d_spatial, symm, asym, false);
 }
 
 int giem2g_get_ie_kernel_spectral(void *ie, void *symm, void *asym)
 {
     IeOp *op = resolve(ie);
     if (!op || !op->have_spectral) return fail(G2_ERR_STATE, "giem2g_get_ie_kernel_spectral: no spectral tensor");
-    return get_units(op, op->d_tensor64, symm, asym, asw_width64(op->Nz));
+    return get_units(op, op->d_tensor64, symm, asym, true);
 }
 
 void giem2g_calc_fft_of_ie_kernel(void *ie)
@@ -351,7 +351,9 @@ int giem2g_apply_ie_operator_device_static(void *ie, const void *d_in, void *d_o
     const size_t es = precision == 0 ? sizeof(double2) : sizeof(float2);
     const size_t n_all = ie_apply_scratch_elems(op, &n_u1);
     const size_t off_uh = (n_u1 * es + 255) / 256 * 256;
-    const size_t need = off_uh + (n_all - n_u1) * es;
+    // the limit counts the rows of the spectrum without their padding, which the array has room for
+    const size_t pad = op->units() * 4 * (ie_spectrum_pitch(op->Nz) - 3 * op->Nz);
+    const size_t need = off_uh + (n_all - n_u1 - pad) * es;
     if (need > cap)
         return fail(G2_ERR_ARG,
                     "giem2g_apply_ie_operator_device_static: grid %dx%dx%d needs %zu bytes of scratch at precision "
@@ -438,11 +440,13 @@ static GIEM2G_FGMRES_CTL resolve_precision(const IeOp *op, GIEM2G_FGMRES_CTL ctl
     return ctl;
 }
 
-// Variants [0, n) are the separate-pass contraction shapes (k_fy, contraction, k_by); where the fused pass
-// exists, variants [n, n + ie_ypipe_variants) select it with its own shapes instead.
+// Where contract.cu has shapes for Nz, variants [0, n - 1) are those and n - 1 is the tensor-core kernel (the default of
+// a new operator, and the only contraction of other Nz); where the fused pass exists, variants
+// [n, n + ie_ypipe_variants) select it with its own shapes instead of the separate passes.
 static int n_contract(const IeOp *op, int precision)
 {
-    return precision == 2 ? ie_contract_pair_variants(op->Nz) : ie_contract_variants(precision, op->Nz);
+    const int n = precision == 2 ? ie_contract_pair_variants(op->Nz) : ie_contract_variants(precision, op->Nz);
+    return n ? n + 1 : 0;
 }
 static int n_ypipe(const IeOp *op, int precision)
 {
@@ -459,10 +463,12 @@ int giem2g_set_contract_variant(void *ie, int precision, int variant)
     if (variant >= n && ny > 0) {
         op->ypipe_mode[precision] = variant - n;
     } else {
-        op->contract_variant[precision] = variant;
+        op->contract_variant[precision] = variant >= n - 1 ? -1 : variant;
         op->ypipe_mode[precision] = -1;
     }
     op->config_gen++;
+    const int rc = ie_sync_plain(op);
+    if (rc) return fail(rc, "giem2g_set_contract_variant: %s", giem2g_last_error());
     return set_status(0);
 }
 
@@ -921,7 +927,8 @@ void giem2g_delete_ie_operator(void *ie)
     void *ptrs[] = {op->d_spatial, op->d_tensor64, op->d_tensor32, op->d_csiga, op->d_gsig64, op->d_asig64,
                     op->d_gsig32, op->d_asig32, op->d_post64, op->d_post32, op->d_twx64, op->d_twy64,
                     op->d_twx32, op->d_twy32, op->scratch.U1, op->scratch.Uhat, op->pair_scratch.U1,
-                    op->pair_scratch.Uhat, op->d_vin, op->d_vout, op->d_err, op->d_vin32, op->d_vout32};
+                    op->pair_scratch.Uhat, op->d_vin, op->d_vout, op->d_err, op->d_vin32, op->d_vout32, op->d_pos, op->d_plain64,
+                    op->d_plain32};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (op->ev0) cudaEventDestroy(op->ev0);

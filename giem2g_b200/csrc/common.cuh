@@ -97,7 +97,44 @@ G2_D void smem_fft(C *s, int log2L, int nlines, int ls, int es, const C *__restr
     }
 }
 
-// Device layout of the full (xz, yz) Nz x Nz blocks: column-major with the row index XOR-swizzled by
+// Device layout of a spectral tensor unit (the tensor-core contraction's): the six blocks in the packed order of
+// the spatial tensor, each stored as 8 x 8 tiles so that a warp's fragment reads (8 rows x 4 columns, or the
+// transpose) hit distinct shared-memory banks.  Inside a tile element (r, c) sits at c * h + (r ^ f(c)), h the
+// tile's rows (plain c * h + r in a tile of fewer than 8 rows); f spreads 4 x 4 elements over the 16 8-byte banks
+// of complex64, and 2 x 4 and 4 x 2 elements over the 8 16-byte banks of complex128.  Row-major 8 x 8 storage
+// without f cost 4 to 8 wavefronts where 2 (complex64) or 4 (complex128) suffice.
+//   full blocks (xz, yz): tiles by row strips;  symmetric blocks: upper tiles, column of tiles by column of tiles,
+//   the tile on the diagonal packed (lo + hi (hi + 1) / 2).  Every element is stored once: T elements per unit.
+template <bool F64> G2_HD int tile_xor(int c) { return F64 ? ((c & 1) << 2) ^ (c & 2) : (c & 2) << 1; }
+template <bool F64> G2_HD int full_pos(int r, int c, int N)
+{
+    const int I = r >> 3, J = c >> 3, h = N - 8 * I < 8 ? N - 8 * I : 8;
+    return 8 * I * N + h * 8 * J + (c & 7) * h + ((r & 7) ^ (h == 8 ? tile_xor<F64>(c & 7) : 0));
+}
+template <bool F64> G2_HD int sym_pos(int i, int j, int N)
+{
+    const int lo = i < j ? i : j, hi = i < j ? j : i, I = lo >> 3, J = hi >> 3;
+    const int w = N - 8 * J < 8 ? N - 8 * J : 8, base = 36 * J + 32 * J * (J - 1);
+    if (I < J) return base + I * 8 * w + (hi & 7) * 8 + ((lo & 7) ^ tile_xor<F64>(hi & 7));
+    const int a = lo & 7, b = hi & 7;
+    return base + J * 8 * w + a + b * (b + 1) / 2;
+}
+// position of the spatial tensor's element e (packed upper xx, xy, yy, zz; column-major xz, yz) in a unit
+template <bool F64> G2_HD int unit_pos(int e, int Nz)
+{
+    const int P = Nz * (Nz + 1) / 2;
+    if (e < 4 * P) {
+        const int blk = e / P, p = e - blk * P;
+        int j = 0;
+        while ((j + 1) * (j + 2) / 2 <= p) j++;
+        return blk * P + sym_pos<F64>(p - j * (j + 1) / 2, j, Nz);
+    }
+    const int li = e - 4 * P, blk = li / (Nz * Nz), rc = li - blk * Nz * Nz;
+    return 4 * P + blk * Nz * Nz + full_pos<F64>(rc % Nz, rc / Nz, Nz);
+}
+
+// Layout of the copy that the other contraction kernels read: packed upper blocks as they are, and
+// the full (xz, yz) Nz x Nz blocks column-major with the row index XOR-swizzled by
 // the low bits of the column, so lane-parallel reads of a row and of a column both hit distinct
 // shared-memory banks.  W = 1 is plain column-major.
 G2_HD int asw(int r, int c, int N, int W) { return c * N + (r ^ (c & (W - 1))); }

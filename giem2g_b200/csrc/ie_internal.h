@@ -32,6 +32,10 @@ struct IeOp {
     double2 *d_spatial = nullptr;      // [Nx][Ny][Tunit] FP64 spatial tensor
     double2 *d_tensor64 = nullptr;     // [Nx][Ny][Tunit] FP64 spectral tensor
     float2 *d_tensor32 = nullptr;      // same, complex64 copy
+    // copies in the layout of the other contraction kernels, held while a form of that precision selects one
+    ushort2 *d_pos = nullptr;          // a unit element's place in d_tensor64 (x) and d_tensor32 (y)
+    double2 *d_plain64 = nullptr;
+    float2 *d_plain32 = nullptr;
     double2 *d_csiga = nullptr;        // [Nz][Ny][Nx]
     double2 *d_gsig64 = nullptr, *d_asig64 = nullptr;  // per-cell pre/post coefficients
     float2 *d_gsig32 = nullptr, *d_asig32 = nullptr;
@@ -54,7 +58,10 @@ struct IeOp {
     cudaEvent_t evc0 = nullptr, evc1 = nullptr;
     int precision_mode = 0;            // 0 plain FP64, 1 mixed (c64 inner)
     bool use_fast_contract = true;     // GIEM2G_GENERIC_CONTRACT=1 selects the generic contraction kernel
-    int contract_variant[3] = {0, 0, 0};  // tile-shape variant: FP64, complex64, paired complex64
+    // contraction of FP64, complex64 and paired complex64 applies: a tile-shape variant of contract.cu, or -1 for
+    // the tensor-core kernel (contract_mma.cu), the default: it takes every Nz, and at 128x128x32 it beats variant 0
+    // in every form (FP64 215 against 280 us, complex64 151 against 170 us, paired 172 against 291 us)
+    int contract_variant[3] = {-1, -1, -1};
     // fused y-transforms + contraction (ypipe.cu) per form: its variant, or -1 for the separate passes
     // (k_fy, contraction, k_by).  The separate passes are the default (faster at 128x128x32 on a B200);
     // the fused pass is a tile-shape variant the autotuner may pick where ie_ypipe_supported holds.
@@ -138,6 +145,15 @@ int ie_contract_fast64(const double2 *G, double2 *Uhat, int Nx, int Ny, int Nz, 
 int ie_contract_fast32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, int *err, cudaStream_t st, int variant,
                        const int *gate);
 int ie_contract_variants(int precision, int Nz);
+
+// contract_mma.cu: the tensor-core contraction (form 0 FP64, 1 complex64, 2 paired complex64), any Nz.  Its
+// spectrum rows (one point of one vector: 3Nz elements) are ie_spectrum_pitch(Nz) elements apart.
+int ie_spectrum_pitch(int Nz);
+bool ie_uses_mma(const IeOp *op, int form);
+// Makes or frees the plain-layout copies (d_plain64, d_plain32) for the selected contractions; not during a capture.
+int ie_sync_plain(IeOp *op);
+int ie_contract_mma(int form, const void *G, void *Uhat, int Nx, int Ny, int Nz, int *err, cudaStream_t st,
+                    const int *gate);
 
 // tensor_fft.cu
 int ie_tensor_spectrum(IeOp *op, cudaStream_t st);

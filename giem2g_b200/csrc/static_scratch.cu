@@ -14,7 +14,8 @@
 // Limits and rules:
 //   - capacity kStaticScratchBytes (32 MiB).  The apply needs 18*Nx*Ny*Nz complex elements
 //     (U1 6*Nx*Ny*Nz, Uhat 12*Nx*Ny*Nz): 16 B each for precision 0, 8 B for precision 1, so e.g.
-//     64x64x16 fits at both precisions and 128x128x32 fits at neither.  Larger grids are rejected
+//     64x64x16 fits at both precisions and 128x128x32 fits at neither.  (The array itself is 40 MiB:
+//     the tensor-core contraction pads the spectrum's rows of 3Nz elements, at Nz = 1 to 22 for 18.)  Larger grids are rejected
 //     with G2_ERR_ARG and a message; they keep using giem2g_apply_ie_operator_device.
 //   - every call on a device shares the one array.  Nothing in it has to start at zero (every
 //     element is written before it is read within a call), but two calls whose executions overlap
@@ -35,10 +36,11 @@
 
 namespace {
 
-constexpr size_t kStaticScratchBytes = size_t(32) << 20;
+constexpr size_t kStaticScratchBytes = size_t(32) << 20;  // of unpadded intermediates
+constexpr size_t kStaticArrayBytes = size_t(40) << 20;
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) unsigned char g_scratch[kStaticScratchBytes];
+static __device__ __align__(256) unsigned char g_scratch[kStaticArrayBytes];
 
 std::mutex g_scratch_mu;
 void *g_scratch_addr[kMaxDevices] = {};

@@ -12,6 +12,7 @@
 // block-Toeplitz product, for even Nx and Ny.
 // Pass A transforms along x (lines over lx for each (ly, element)), pass B along y with both corrections.
 // Elements of a unit are interleaved in shared memory so global loads/stores are coalesced.
+#include <vector>
 #include "common.cuh"
 #include "ie_internal.h"
 
@@ -30,15 +31,6 @@ G2_D void elem_parity(int e, int P, int Nz, double &sx, double &sy)
         sx = comp == 0 ? -1.0 : 1.0;
         sy = comp == 0 ? 1.0 : -1.0;
     }
-}
-
-// position of unit element e in the device layout (full blocks swizzled, see asw)
-G2_HD int dev_pos(int e, int P, int Nz, int W)
-{
-    if (e < 4 * P) return e;
-    const int li = e - 4 * P, blk = li / (Nz * Nz), rc = li - blk * Nz * Nz;
-    const int r = rc % Nz, c = rc / Nz;
-    return 4 * P + blk * Nz * Nz + asw(r, c, Nz, W);
 }
 
 // pass A: spatial [lx][ly][T] -> S1 [kx 0..Nx][ly][T]
@@ -73,7 +65,8 @@ __global__ void __launch_bounds__(kThreads) k_tensor_x(const double2 *__restrict
 // pass B: S1 [kx][ly][T] -> out [kx][ky][T] (kx < Nx) or nyq [ky][T] (kx == Nx, when corr == nullptr)
 __global__ void __launch_bounds__(kThreads) k_tensor_y(const double2 *__restrict__ S1, double2 *__restrict__ out,
                                                        const double2 *__restrict__ nyq, const double2 *__restrict__ tw,
-                                                       int Nx, int Ny, int Nz, int kx_base)
+                                                       const ushort2 *__restrict__ pos, int Nx, int Ny, int Nz,
+                                                       int kx_base)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *s = reinterpret_cast<double2 *>(smem_raw);
@@ -105,32 +98,93 @@ __global__ void __launch_bounds__(kThreads) k_tensor_y(const double2 *__restrict
         } else {
             const double sx = (kx & 1) ? -1.0 : 1.0;
             const double2 c = nyq[(size_t)ky * T + e0 + t];
-            out[((size_t)kx * Ny + ky) * T + dev_pos(e0 + t, P, Nz, asw_width64(Nz))] =
+            out[((size_t)kx * Ny + ky) * T + pos[e0 + t].x] =
                 make_double2(v.x - sx * c.x, v.y - sx * c.y);
         }
     }
 }
 
-// complex64 copy; the full blocks move from the FP64 swizzle to the FP32 swizzle
-__global__ void k_to_c64(const double2 *__restrict__ a, float2 *__restrict__ b, size_t units, int P, int Nz)
+// complex64 copy: element e of a unit sits at pos[e].x in the FP64 unit and at pos[e].y in the complex64 unit
+__global__ void k_to_c64(const double2 *__restrict__ a, float2 *__restrict__ b, const ushort2 *__restrict__ pos,
+                         size_t units, int T)
 {
-    const int T = 4 * P + 2 * Nz * Nz, W64 = asw_width64(Nz), W32 = asw_width32(Nz);
+    const size_t n = units * T;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t u = i / T;
+        const ushort2 p = pos[i - u * T];
+        const double2 v = a[u * T + p.x];
+        b[u * T + p.y] = make_float2((float)v.x, (float)v.y);
+    }
+}
+// the unit layout of the contraction kernels of contract.cu (packed blocks, full blocks swizzled, see asw)
+template <typename C>
+__global__ void k_to_plain(const C *__restrict__ a, C *__restrict__ b, const ushort2 *__restrict__ pos, size_t units,
+                           int Nz, int W)
+{
+    const int P = Nz * (Nz + 1) / 2, T = 4 * P + 2 * Nz * Nz;
     const size_t n = units * T;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t u = i / T;
         const int e = (int)(i - u * T);
-        const double2 v = a[u * T + dev_pos(e, P, Nz, W64)];
-        b[u * T + dev_pos(e, P, Nz, W32)] = make_float2((float)v.x, (float)v.y);
+        int d = e;
+        if (e >= 4 * P) {
+            const int li = e - 4 * P, blk = li / (Nz * Nz), rc = li - blk * Nz * Nz;
+            d = 4 * P + blk * Nz * Nz + asw(rc % Nz, rc / Nz, Nz, W);
+        }
+        b[u * T + d] = a[u * T + (sizeof(C) == 16 ? pos[e].x : pos[e].y)];
     }
 }
 
 }  // namespace
+
+// positions of a unit's elements in the two tensors (they depend on Nz alone)
+static int make_positions(IeOp *op)
+{
+    if (op->d_pos) return G2_OK;
+    const int T = op->Tunit();
+    std::vector<ushort2> h(T);
+    for (int e = 0; e < T; e++)
+        h[e] = make_ushort2((unsigned short)unit_pos<true>(e, op->Nz), (unsigned short)unit_pos<false>(e, op->Nz));
+    G2_CUDA_CHECK(cudaMalloc(&op->d_pos, T * sizeof(ushort2)));
+    G2_CUDA_CHECK(cudaMemcpyAsync(op->d_pos, h.data(), T * sizeof(ushort2), cudaMemcpyHostToDevice, op->stream));
+    G2_CUDA_CHECK(cudaStreamSynchronize(op->stream));
+    return G2_OK;
+}
+
+int ie_sync_plain(IeOp *op)
+{
+    if (!op->d_tensor64 || !op->d_tensor32) return G2_OK;
+    const bool need64 = !ie_uses_mma(op, 0), need32 = !ie_uses_mma(op, 1) || !ie_uses_mma(op, 2);
+    const size_t n = op->units() * op->Tunit();
+    if (!need64 && op->d_plain64) {
+        cudaFree(op->d_plain64);
+        op->d_plain64 = nullptr;
+    }
+    if (!need32 && op->d_plain32) {
+        cudaFree(op->d_plain32);
+        op->d_plain32 = nullptr;
+    }
+    if (need64 && !op->d_plain64) {
+        G2_CUDA_CHECK(cudaMalloc(&op->d_plain64, n * sizeof(double2)));
+        k_to_plain<<<1184, 256, 0, op->stream>>>(op->d_tensor64, op->d_plain64, op->d_pos, op->units(), op->Nz,
+                                                 asw_width64(op->Nz));
+    }
+    if (need32 && !op->d_plain32) {
+        G2_CUDA_CHECK(cudaMalloc(&op->d_plain32, n * sizeof(float2)));
+        k_to_plain<<<1184, 256, 0, op->stream>>>(op->d_tensor32, op->d_plain32, op->d_pos, op->units(), op->Nz,
+                                                 asw_width32(op->Nz));
+    }
+    G2_CUDA_CHECK(cudaGetLastError());
+    return G2_OK;
+}
 
 int ie_tensor_spectrum(IeOp *op, cudaStream_t st)
 {
     const int Nx = op->Nx, Ny = op->Ny, Nz = op->Nz, T = op->Tunit();
     if (!op->d_spatial) return G2_ERR_STATE;
     const size_t n_out = op->units() * T;
+    const int rcp = make_positions(op);
+    if (rcp) return rcp;
     double2 *S1 = nullptr, *nyq = nullptr;
     G2_CUDA_CHECK(cudaMalloc(&S1, (size_t)(Nx + 1) * Ny * T * sizeof(double2)));
     G2_CUDA_CHECK(cudaMalloc(&nyq, (size_t)Ny * T * sizeof(double2)));
@@ -141,9 +195,9 @@ int ie_tensor_spectrum(IeOp *op, cudaStream_t st)
     G2_CUDA_CHECK(cudaFuncSetAttribute(k_tensor_y, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     const int eb = (T + TE - 1) / TE;
     k_tensor_x<<<dim3(Ny, eb), kThreads, smx, st>>>(op->d_spatial, S1, op->d_twx64, Nx, Ny, Nz);
-    k_tensor_y<<<dim3(1, eb), kThreads, smy, st>>>(S1, nyq, nullptr, op->d_twy64, Nx, Ny, Nz, Nx);
-    k_tensor_y<<<dim3(Nx, eb), kThreads, smy, st>>>(S1, op->d_tensor64, nyq, op->d_twy64, Nx, Ny, Nz, 0);
-    k_to_c64<<<1184, 256, 0, st>>>(op->d_tensor64, op->d_tensor32, op->units(), op->P(), Nz);
+    k_tensor_y<<<dim3(1, eb), kThreads, smy, st>>>(S1, nyq, nullptr, op->d_twy64, op->d_pos, Nx, Ny, Nz, Nx);
+    k_tensor_y<<<dim3(Nx, eb), kThreads, smy, st>>>(S1, op->d_tensor64, nyq, op->d_twy64, op->d_pos, Nx, Ny, Nz, 0);
+    k_to_c64<<<1184, 256, 0, st>>>(op->d_tensor64, op->d_tensor32, op->d_pos, op->units(), T);
     G2_CUDA_CHECK(cudaGetLastError());
     G2_CUDA_CHECK(cudaStreamSynchronize(st));
     cudaFree(S1);
@@ -153,5 +207,13 @@ int ie_tensor_spectrum(IeOp *op, cudaStream_t st)
     cudaFree(op->d_spatial);
     op->d_spatial = nullptr;
     op->have_spatial = false;
-    return G2_OK;
+    // plain-layout copies of an earlier tensor are out of date
+    if (op->d_plain64 || op->d_plain32) {
+        cudaFree(op->d_plain64);
+        cudaFree(op->d_plain32);
+        op->d_plain64 = nullptr;
+        op->d_plain32 = nullptr;
+        op->config_gen++;  // captured graphs hold the copies' addresses
+    }
+    return ie_sync_plain(op);
 }
