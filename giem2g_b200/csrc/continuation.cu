@@ -257,7 +257,7 @@ G2_D void outfunc2(int i, double s_arg, double cphi, double sphi, double alpha, 
 
 // W layout: [6][npts][NLAM], RC_* order, scaled by lambda and masked (calc_rc_tensor_module.F90:182-222)
 __global__ void __launch_bounds__(256, 2) k_rc_weights(const VbtTab *__restrict__ T, int Nx, int Ny, double dx, double dy,
-                                                    double xs, double ys, double *W)
+                                                    double xs, double ys, double *W, int2 *krange)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *g = reinterpret_cast<double2 *>(smem_raw);  // [VN][6]
@@ -266,12 +266,14 @@ __global__ void __launch_bounds__(256, 2) k_rc_weights(const VbtTab *__restrict_
                   "weights would overlap the samples still being read");
     double *wt = reinterpret_cast<double *>(smem_raw + VN * 6 * sizeof(double2) - NLAM * 6 * sizeof(double));
     __shared__ double red[8], w0;
+    __shared__ int kfirst, kend;  // the kept wave numbers lie in [kfirst, kend)
     const int Nx2 = 2 * Nx, Ny2 = 2 * Ny;
     const int pt = blockIdx.x, iy = pt / Nx2, ix = pt - iy * Nx2;
     const size_t npts = (size_t)Nx2 * Ny2;
     if (ix == Nx || iy == Ny) {  // lags Nx and Ny are zero (calc_rc_tensor_module.F90:84-92, :120-123)
         for (int k = threadIdx.x; k < NLAM; k += blockDim.x)
             for (int c = 0; c < 6; c++) W[((size_t)c * npts + pt) * NLAM + k] = 0.0;
+        if (threadIdx.x == 0) krange[pt] = make_int2(0, 0);
         return;
     }
     const int lx = ix < Nx ? ix : ix - Nx2, ly = iy < Ny ? iy : iy - Ny2;
@@ -308,6 +310,8 @@ __global__ void __launch_bounds__(256, 2) k_rc_weights(const VbtTab *__restrict_
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
     if (threadIdx.x == 0) {
+        kfirst = NLAM;
+        kend = 0;
         double m = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) m = fmax(m, red[w]);
         w0 = m;
@@ -327,7 +331,13 @@ __global__ void __launch_bounds__(256, 2) k_rc_weights(const VbtTab *__restrict_
         v[RC_DY] = wt[k * 6 + RC_DY] * lm;
         v[RC_D0] = wt[k * 6 + RC_D0] * lm;
         for (int c = 0; c < 6; c++) W[((size_t)c * npts + pt) * NLAM + k] = keep ? v[c] : 0.0;
+        if (keep) {
+            atomicMin(&kfirst, k);
+            atomicMax(&kend, k + 1);
+        }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) krange[pt] = make_int2(kfirst, kend);
 }
 
 // ---- 2-D FFT passes over [rows][Nx2][E] point-major buffers -----------------------------------------
@@ -646,6 +656,7 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
     RcRecvDev *d_rv = nullptr;
     double2 *d_B = nullptr;
     double *d_W = nullptr;
+    int2 *d_range = nullptr;
     const size_t npts = op->npts();
     int rc = G2_OK;
     auto cleanup = [&]() {
@@ -654,6 +665,7 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
         cudaFree(d_rv);
         cudaFree(d_B);
         cudaFree(d_W);
+        cudaFree(d_range);
         delete tab;
     };
 #define RC_TRY2(expr)                                                     \
@@ -673,6 +685,7 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
     RC_TRY2(cudaMemcpyAsync(d_rv, rv.data(), sizeof(RcRecvDev) * Nr, cudaMemcpyHostToDevice, st));
     RC_TRY2(cudaMalloc(&d_B, sizeof(double2) * (size_t)Nr * RC_NBASIS * NLAM * Nz));
     RC_TRY2(cudaMalloc(&d_W, sizeof(double) * 6 * npts * NLAM));
+    RC_TRY2(cudaMalloc(&d_range, sizeof(int2) * npts));
     double *d_lms = reinterpret_cast<double *>(reinterpret_cast<char *>(d_tab) + offsetof(VbtTab, lms));
     k_rc_basis<<<dim3(NLAM, Nr), 64, 0, st>>>(d_bkg, d_rv, d_lms, d_B);
     RC_TRY2(cudaGetLastError());
@@ -680,18 +693,31 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
     RC_TRY2(cudaFuncSetAttribute(k_rc_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
     const double sc = 1.0 / 4.0 / PI_D;  // s = 1/4/PI (calc_rc_tensor_module.F90:184), G * s (:225-226)
     const int E = (int)op->E();
-    const int gm = (int)((npts + GM - 1) / GM);
-    int launches = 1;
-    for (int r = 0; r < Nr; r++) {
-        k_rc_weights<<<(unsigned)npts, 256, smw, st>>>(d_tab, Nx, Ny, op->dx, op->dy, op->recv[r].x_shift,
-                                                        op->recv[r].y_shift, d_W);
-        RC_TRY2(cudaGetLastError());
+    const int NT = gemm_tile(Nz);
+    int launches = 1, weights_of = -1;
+    // the weights depend on the lag and the lateral shift alone: receivers of one shift (a vertical profile) come one
+    // after the other and share them
+    std::vector<int> order(Nr);
+    for (int r = 0; r < Nr; r++) order[r] = r;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        const RcReceiver &p = op->recv[a], &q = op->recv[b];
+        return p.x_shift != q.x_shift ? p.x_shift < q.x_shift : p.y_shift < q.y_shift;
+    });
+    for (int r : order) {
+        if (weights_of < 0 || op->recv[r].x_shift != op->recv[weights_of].x_shift ||
+            op->recv[r].y_shift != op->recv[weights_of].y_shift) {
+            k_rc_weights<<<(unsigned)npts, 256, smw, st>>>(d_tab, Nx, Ny, op->dx, op->dy, op->recv[r].x_shift,
+                                                            op->recv[r].y_shift, d_W, d_range);
+            RC_TRY2(cudaGetLastError());
+            weights_of = r;
+            launches++;
+        }
         auto Wt = [&](int c) { return d_W + (size_t)c * npts * NLAM; };
         auto Bs = [&](int bsel) { return d_B + ((size_t)r * RC_NBASIS + bsel) * NLAM * Nz; };
+        GemmJobs jobs;
         auto gemm = [&](int comp, int w1, int b1, int w2, int b2) {
-            dim3 grid(gm, (Nz + GN - 1) / GN);
-            k_gemm<<<grid, 256, 0, st>>>(Wt(w1), Bs(b1), w2 >= 0 ? Wt(w2) : nullptr, w2 >= 0 ? Bs(b2) : nullptr,
-                                         (int)npts, Nz, op->d_G, E, (comp * Nr + r) * Nz, sc);
+            add_job(jobs, NT, Wt(w1), Bs(b1), w2 >= 0 ? Wt(w2) : nullptr, w2 >= 0 ? Bs(b2) : nullptr, Nz,
+                    (comp * Nr + r) * Nz);
         };
         // rc_kernel_hankel_module.F90:118-143
         gemm(REXX, RC_D0, B_G11, RC_DXX, B_G3DZ_G11);
@@ -709,8 +735,8 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
         gemm(RHYZ, RC_DX, B_MG2, -1, 0);
         gemm(RHZX, RC_DY, B_MG1, -1, 0);
         gemm(RHZY, RC_DX, B_G1, -1, 0);
-        RC_TRY2(cudaGetLastError());
-        launches += 1 + RC_NCOMP;
+        RC_TRY2(launch_gemm(jobs, NT, d_range, (int)npts, op->d_G, E, sc, st));
+        launches++;
     }
     RC_TRY2(cudaStreamSynchronize(st));
     g2_count_launches(launches);

@@ -243,7 +243,7 @@ G2_D void outfunc(int i, double s_arg, double cphi, double sphi, double alpha, d
 
 // W layout: [6][lags][NLAM] (weight type major), already scaled by lambda and masked
 __global__ void __launch_bounds__(256, 2) k_weights(const VbtTab *__restrict__ T, int Nx, int Ny, double dx, double dy,
-                                                 double *W)
+                                                 double *W, int2 *krange)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *g = reinterpret_cast<double2 *>(smem_raw);  // [VN][6]
@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(256, 2) k_weights(const VbtTab *__restrict__ T
                   "weights would overlap the samples still being read");
     double *wt = reinterpret_cast<double *>(smem_raw + VN * 6 * sizeof(double2) - NLAM * 6 * sizeof(double));
     __shared__ double w0[6], red[8][6];
+    __shared__ int kfirst, kend;  // the kept wave numbers lie in [kfirst, kend)
     const int lag = blockIdx.x, lx = lag / Ny, ly = lag - lx * Ny;
     const size_t nlags = (size_t)Nx * Ny;
     // COMPUTE_WEIGHTS (calc_ie_tensor_module.F90:308-326) + VBTransformWeightsAllDoubleInt (:159-197)
@@ -297,6 +298,8 @@ __global__ void __launch_bounds__(256, 2) k_weights(const VbtTab *__restrict__ T
         for (int c = 0; c < 6; c++) red[threadIdx.x >> 5][c] = mx[c];
     __syncthreads();
     if (threadIdx.x == 0) {
+        kfirst = NLAM;
+        kend = 0;
         double m[6] = {0, 0, 0, 0, 0, 0};
         for (int w = 0; w < (int)(blockDim.x >> 5); w++)
             for (int c = 0; c < 6; c++) m[c] = fmax(m[c], red[w][c]);
@@ -332,7 +335,13 @@ __global__ void __launch_bounds__(256, 2) k_weights(const VbtTab *__restrict__ T
         v[IE_DY] = wt[k * 6 + IE_DY] * lm;
         v[IE_D0] = wt[k * 6 + IE_D0] * lm;
         for (int c = 0; c < 6; c++) W[((size_t)c * nlags + lag) * NLAM + k] = keep ? v[c] : 0.0;
+        if (keep) {
+            atomicMin(&kfirst, k);
+            atomicMax(&kend, k + 1);
+        }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) krange[lag] = make_int2(kfirst, kend);
 }
 
 }  // namespace
@@ -373,12 +382,14 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
     VbtTab *d_tab = nullptr;
     double2 *M[4] = {nullptr, nullptr, nullptr, nullptr};
     double *W = nullptr;
+    int2 *krange = nullptr;
     int rc = G2_OK;
     auto cleanup = [&]() {
         cudaFree(d_bkg);
         cudaFree(d_tab);
         for (auto p : M) cudaFree(p);
         cudaFree(W);
+        cudaFree(krange);
         delete tab;
     };
 #define G2_TRY(expr)                                                      \
@@ -400,26 +411,25 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
     G2_TRY(cudaMalloc(&M[3], sizeof(double2) * NLAM * P));
     G2_TRY(cudaMemsetAsync(M[2], 0, sizeof(double2) * NLAM * Nz * Nz, st));
     G2_TRY(cudaMalloc(&W, sizeof(double) * 6 * lags * NLAM));
+    G2_TRY(cudaMalloc(&krange, sizeof(int2) * lags));
     double *d_lms = reinterpret_cast<double *>(reinterpret_cast<char *>(d_tab) + offsetof(VbtTab, lms));
     k_basis<<<NLAM, 64, 0, st>>>(d_bkg, d_lms, M[0], M[1], M[2], M[3]);
     const size_t smw = sizeof(double2) * VN * 6;  // two blocks per SM
     G2_TRY(cudaFuncSetAttribute(k_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
-    k_weights<<<(unsigned)lags, 256, smw, st>>>(d_tab, Nx, Ny, op->dx, op->dy, W);
+    k_weights<<<(unsigned)lags, 256, smw, st>>>(d_tab, Nx, Ny, op->dx, op->dy, W, krange);
     G2_TRY(cudaGetLastError());
     if (!op->d_spatial) G2_TRY(cudaMalloc(&op->d_spatial, lags * T * sizeof(double2)));
     const double sc = 1.0 / PI_D / 4.0;  // G1/PI/4 (calc_ie_tensor_module.F90:278-286)
     auto Wt = [&](int c) { return W + (size_t)c * lags * NLAM; };
-    const int gm = (int)((lags + GM - 1) / GM);
-    auto gemm = [&](const double *A1, const double2 *B1, const double *A2, const double2 *B2, int ncols, int off) {
-        dim3 grid(gm, (ncols + GN - 1) / GN);
-        k_gemm<<<grid, 256, 0, st>>>(A1, B1, A2, B2, (int)lags, ncols, op->d_spatial, T, off, sc);
-    };
-    gemm(Wt(IE_D0), M[0], Wt(IE_DXX), M[1], P, 0 * P);              // xx
-    gemm(Wt(IE_DXY), M[1], nullptr, nullptr, P, 1 * P);             // xy
-    gemm(Wt(IE_D0), M[0], Wt(IE_DYY), M[1], P, 2 * P);              // yy
-    gemm(Wt(IE_D0), M[3], nullptr, nullptr, P, 3 * P);              // zz
-    gemm(Wt(IE_DX), M[2], nullptr, nullptr, Nz * Nz, 4 * P);        // xz
-    gemm(Wt(IE_DY), M[2], nullptr, nullptr, Nz * Nz, 4 * P + Nz * Nz);  // yz
+    GemmJobs jobs;
+    const int NT = gemm_tile(P);
+    add_job(jobs, NT, Wt(IE_D0), M[0], Wt(IE_DXX), M[1], P, 0 * P);                     // xx
+    add_job(jobs, NT, Wt(IE_DXY), M[1], nullptr, nullptr, P, 1 * P);                    // xy
+    add_job(jobs, NT, Wt(IE_D0), M[0], Wt(IE_DYY), M[1], P, 2 * P);                     // yy
+    add_job(jobs, NT, Wt(IE_D0), M[3], nullptr, nullptr, P, 3 * P);                     // zz
+    add_job(jobs, NT, Wt(IE_DX), M[2], nullptr, nullptr, Nz * Nz, 4 * P);               // xz
+    add_job(jobs, NT, Wt(IE_DY), M[2], nullptr, nullptr, Nz * Nz, 4 * P + Nz * Nz);     // yz
+    G2_TRY(launch_gemm(jobs, NT, krange, (int)lags, op->d_spatial, T, sc, st));
     G2_TRY(cudaGetLastError());
     G2_TRY(cudaStreamSynchronize(st));
     cleanup();
