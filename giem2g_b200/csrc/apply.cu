@@ -663,16 +663,20 @@ int ie_prepare_sigma(IeOp *op, cudaStream_t st)
     G2_CUDA_CHECK(cudaMemcpyAsync(op->d_post32, post32.data(), 2 * Nz * sizeof(float), cudaMemcpyHostToDevice, st));
     double2 *d_csigb = nullptr;
     double *d_sq = nullptr;
-    G2_CUDA_CHECK(cudaMalloc(&d_csigb, Nz * sizeof(double2)));
-    G2_CUDA_CHECK(cudaMalloc(&d_sq, Nz * sizeof(double)));
+    int rc = g2_pool_alloc(&op->pool, (void **)&d_csigb, Nz * sizeof(double2), st);
+    if (!rc) rc = g2_pool_alloc(&op->pool, (void **)&d_sq, Nz * sizeof(double), st);
+    if (rc) {
+        g2_pool_free(d_csigb, st);
+        return rc;
+    }
     G2_CUDA_CHECK(cudaMemcpyAsync(d_csigb, op->csigb.data(), Nz * sizeof(double2), cudaMemcpyHostToDevice, st));
     G2_CUDA_CHECK(cudaMemcpyAsync(d_sq, op->sqsigb.data(), Nz * sizeof(double), cudaMemcpyHostToDevice, st));
     k_sigma<<<592, 256, 0, st>>>(op->d_csiga, d_csigb, d_sq, op->d_gsig64, op->d_asig64, op->d_gsig32, op->d_asig32,
                                  (size_t)op->Nx * op->Ny, Nz);
     G2_CUDA_CHECK(cudaGetLastError());
+    g2_pool_free(d_csigb, st);
+    g2_pool_free(d_sq, st);
     G2_CUDA_CHECK(cudaStreamSynchronize(st));
-    cudaFree(d_csigb);
-    cudaFree(d_sq);
     return G2_OK;
 }
 

@@ -226,8 +226,8 @@ int giem2g_set_ie_kernel_spatial(void *ie, const void *symm, const void *asym)
     if (!op || op->z.empty()) return fail(G2_ERR_STATE, "giem2g_set_ie_kernel_spatial: operator not prepared");
     const int P = op->P(), Nz = op->Nz, T = op->Tunit();
     const size_t U = op->units();
-    if (!op->d_spatial && cudaMalloc(&op->d_spatial, U * T * sizeof(double2)) != cudaSuccess)
-        return fail(G2_ERR_NOMEM, "giem2g_set_ie_kernel_spatial: cudaMalloc failed");
+    if (!op->d_spatial && g2_pool_alloc(&op->pool, (void **)&op->d_spatial, U * T * sizeof(double2), op->stream))
+        return fail(G2_ERR_NOMEM, "giem2g_set_ie_kernel_spatial: device allocation failed");
     std::vector<double2> h(U * T);
     const double2 *s = reinterpret_cast<const double2 *>(symm), *a = reinterpret_cast<const double2 *>(asym);
     for (size_t u = 0; u < U; u++) {
@@ -924,7 +924,10 @@ void giem2g_delete_ie_operator(void *ie)
     if (op->stream) cudaStreamSynchronize(op->stream);
     ie_free_learned(op);
     krylov_free(op);
-    void *ptrs[] = {op->d_spatial, op->d_tensor64, op->d_tensor32, op->d_csiga, op->d_gsig64, op->d_asig64,
+    g2_pool_free(op->d_spatial, op->stream);
+    if (op->stream) cudaStreamSynchronize(op->stream);
+    if (op->pool) cudaMemPoolDestroy(op->pool);
+    void *ptrs[] = {op->d_tensor64, op->d_tensor32, op->d_csiga, op->d_gsig64, op->d_asig64,
                     op->d_gsig32, op->d_asig32, op->d_post64, op->d_post32, op->d_twx64, op->d_twy64,
                     op->d_twx32, op->d_twy32, op->scratch.U1, op->scratch.Uhat, op->pair_scratch.U1,
                     op->pair_scratch.Uhat, op->d_vin, op->d_vout, op->d_err, op->d_vin32, op->d_vout32, op->d_pos, op->d_plain64,

@@ -62,15 +62,17 @@ __global__ void __launch_bounds__(64) k_rc_basis(const Bkg *__restrict__ bk, con
     const int Nl = b.Nl, Nz = b.Nz;
     const RcRecvDev rv = recv[r];
     const int rl = rv.layer;
-    __shared__ cplx s_eta[MAXL + 1], s_p[MAXL + 1][2], s_q[MAXL + 1][2], s_A[MAXL + 1][2];
+    __shared__ cplx s_eta[MAXL + 1], s_el[MAXL + 1], s_p[MAXL + 1][2], s_q[MAXL + 1][2], s_A[MAXL + 1][2];
+    __shared__ cplx s_arr[MAXL + 1][2], w[MAXL + 1][2];
     __shared__ cplx s_expz[MAXZ + 1], s_pez[MAXZ + 1][2], s_qez[MAXZ + 1][2];
+    // one thread for the layers' recursions, then by cell and one thread for each recursion over the cells
     if (threadIdx.x == 0) {
-        cplx eta[MAXL + 1], el[MAXL + 1], p[MAXL + 1][2], q[MAXL + 1][2], Arr[MAXL + 1][2];
+        cplx *eta = s_eta, *el = s_el;
+        cplx (*p)[2] = s_p, (*q)[2] = s_q, (*Arr)[2] = s_arr;
         dev_apq(b, lms, eta, el, p, q, Arr);
         // row rl of the layer-transfer matrix A of Calc_Apq (apq_module.F90:249-264):
         //   A(J,I) = A(J+1,I) w(J) for J < I, A(I,I) = Arr(I), A(I,J,1) = A(J,I,1),
         //   A(I,J,2) = A(J,I,2) csigma(I) / csigma(J)
-        cplx w[MAXL + 1][2];
         for (int i = 1; i <= Nl - 1; i++) {
             cplx tmp = C(b.k2[i]) - C(b.k2[i + 1]);
             tmp = b.depth[i] * tmp;
@@ -96,26 +98,14 @@ __global__ void __launch_bounds__(64) k_rc_basis(const Bkg *__restrict__ bk, con
                 s_A[l][1] = a1 * C(b.csigma[rl]) / C(b.csigma[l]);
             }
         }
-        // expz (rc_kernel_hankel_module.F90:84-87), pexpz / qexpz (apq_module.F90:112-177)
-        cplx expz[MAXZ + 1], pez[MAXZ + 1][2], qez[MAXZ + 1][2];
-        for (int iz = 1; iz <= Nz; iz++) expz[iz] = cuda::std::exp(-eta[b.L[iz]] * (b.z[iz] - b.z[iz - 1]));
-        dev_pexpz(b, eta, p, expz, pez);
-        dev_qexpz(b, eta, q, expz, qez);
-        for (int i = 1; i <= Nl; i++) {
-            s_eta[i] = eta[i];
-            for (int k = 0; k < 2; k++) {
-                s_p[i][k] = p[i][k];
-                s_q[i][k] = q[i][k];
-            }
-        }
-        for (int iz = 1; iz <= Nz; iz++) {
-            s_expz[iz] = expz[iz];
-            for (int k = 0; k < 2; k++) {
-                s_pez[iz][k] = pez[iz][k];
-                s_qez[iz][k] = qez[iz][k];
-            }
-        }
     }
+    __syncthreads();
+    // expz (rc_kernel_hankel_module.F90:84-87), pexpz / qexpz (apq_module.F90:112-177)
+    for (int iz = threadIdx.x + 1; iz <= Nz; iz += blockDim.x)
+        s_expz[iz] = cuda::std::exp(-s_eta[b.L[iz]] * (b.z[iz] - b.z[iz - 1]));
+    __syncthreads();
+    if (threadIdx.x == 0) dev_pexpz(b, s_eta, s_p, s_expz, s_pez);
+    if (threadIdx.x == 32) dev_qexpz(b, s_eta, s_q, s_expz, s_qez);
     __syncthreads();
     const double lm2 = lms * lms;
     const cplx iwm = C(b.iwm), csr = C(b.csigma[rl]);
@@ -478,6 +468,15 @@ __global__ void __launch_bounds__(256) k_rc_contract(const double2 *__restrict__
     }
 }
 
+__global__ void k_dsig(const double2 *__restrict__ csiga, const double2 *__restrict__ csigb, double2 *dsig, size_t plane,
+                       size_t n)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const double2 a = csiga[i], b = csigb[i / plane];
+        dsig[i] = make_double2(a.x - b.x, a.y - b.y);
+    }
+}
+
 void make_twiddles(std::vector<double2> &tw, int L)
 {
     tw.resize(L / 2);
@@ -512,6 +511,7 @@ struct RcOp {
     double2 *d_E = nullptr, *d_Ea = nullptr, *d_Ha = nullptr;  // staging of the host-buffer entry
     std::vector<double2> csigb;  // per cell
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;  // temporaries of the tensor
 
     size_t npts() const { return (size_t)4 * Nx * Ny; }
     size_t E() const { return (size_t)RC_NCOMP * Nr * Nz; }
@@ -575,6 +575,7 @@ void rc_delete(RcOp *op)
                     op->d_E, op->d_Ea, op->d_Ha};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (op->pool) cudaMemPoolDestroy(op->pool);
     if (op->stream) cudaStreamDestroy(op->stream);
     delete op;
 }
@@ -592,17 +593,19 @@ int rc_receivers(const RcOp *op, RcReceiver *out)
 static int rc_update_dsig(RcOp *op)
 {
     if (!op->have_sigma || !op->have_background) return G2_OK;
-    // dsig = csiga - csigb(z) (LoadEint :254), computed on the host once per conductivity / frequency
-    std::vector<double2> h(op->cells());
-    RC_TRY(cudaMemcpyAsync(h.data(), op->d_csiga, h.size() * sizeof(double2), cudaMemcpyDeviceToHost, op->stream));
-    RC_TRY(cudaStreamSynchronize(op->stream));
-    const size_t plane = (size_t)op->Nx * op->Ny;
-    for (int iz = 0; iz < op->Nz; iz++)
-        for (size_t k = 0; k < plane; k++) {
-            double2 &v = h[iz * plane + k];
-            v = make_double2(v.x - op->csigb[iz].x, v.y - op->csigb[iz].y);
-        }
-    RC_TRY(cudaMemcpyAsync(op->d_dsig, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, op->stream));
+    // dsig = csiga - csigb(z) (LoadEint :254)
+    double2 *d_b = nullptr;
+    const int rc = g2_pool_alloc(&op->pool, (void **)&d_b, op->Nz * sizeof(double2), op->stream);
+    if (rc) return rc;
+    cudaError_t e = cudaMemcpyAsync(d_b, op->csigb.data(), op->Nz * sizeof(double2), cudaMemcpyHostToDevice, op->stream);
+    if (e == cudaSuccess) {
+        k_dsig<<<(unsigned)std::min<size_t>((op->cells() + 255) / 256, 1184), 256, 0, op->stream>>>(
+            op->d_csiga, d_b, op->d_dsig, (size_t)op->Nx * op->Ny, op->cells());
+        e = cudaGetLastError();
+        g2_count_launches(1);
+    }
+    g2_pool_free(d_b, op->stream);
+    RC_TRY(e);
     RC_TRY(cudaStreamSynchronize(op->stream));
     return G2_OK;
 }
@@ -660,12 +663,12 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
     const size_t npts = op->npts();
     int rc = G2_OK;
     auto cleanup = [&]() {
-        cudaFree(d_bkg);
-        cudaFree(d_tab);
-        cudaFree(d_rv);
-        cudaFree(d_B);
-        cudaFree(d_W);
-        cudaFree(d_range);
+        g2_pool_free(d_bkg, st);
+        g2_pool_free(d_tab, st);
+        g2_pool_free(d_rv, st);
+        g2_pool_free(d_B, st);
+        g2_pool_free(d_W, st);
+        g2_pool_free(d_range, st);
         delete tab;
     };
 #define RC_TRY2(expr)                                                     \
@@ -677,15 +680,23 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
             return G2_ERR_CUDA;                                           \
         }                                                                 \
     } while (0)
-    RC_TRY2(cudaMalloc(&d_bkg, sizeof(Bkg)));
-    RC_TRY2(cudaMalloc(&d_tab, sizeof(VbtTab)));
-    RC_TRY2(cudaMalloc(&d_rv, sizeof(RcRecvDev) * Nr));
+#define RC_TRY2_RC(expr)       \
+    do {                       \
+        const int r_ = (expr); \
+        if (r_) {              \
+            cleanup();         \
+            return r_;         \
+        }                      \
+    } while (0)
+    RC_TRY2_RC(g2_pool_alloc(&op->pool, (void **)&d_bkg, sizeof(Bkg), st));
+    RC_TRY2_RC(g2_pool_alloc(&op->pool, (void **)&d_tab, sizeof(VbtTab), st));
+    RC_TRY2_RC(g2_pool_alloc(&op->pool, (void **)&d_rv, sizeof(RcRecvDev) * Nr, st));
     RC_TRY2(cudaMemcpyAsync(d_bkg, &h, sizeof(Bkg), cudaMemcpyHostToDevice, st));
     RC_TRY2(cudaMemcpyAsync(d_tab, tab, sizeof(VbtTab), cudaMemcpyHostToDevice, st));
     RC_TRY2(cudaMemcpyAsync(d_rv, rv.data(), sizeof(RcRecvDev) * Nr, cudaMemcpyHostToDevice, st));
-    RC_TRY2(cudaMalloc(&d_B, sizeof(double2) * (size_t)Nr * RC_NBASIS * NLAM * Nz));
-    RC_TRY2(cudaMalloc(&d_W, sizeof(double) * 6 * npts * NLAM));
-    RC_TRY2(cudaMalloc(&d_range, sizeof(int2) * npts));
+    RC_TRY2_RC(g2_pool_alloc(&op->pool, (void **)&d_B, sizeof(double2) * (size_t)Nr * RC_NBASIS * NLAM * Nz, st));
+    RC_TRY2_RC(g2_pool_alloc(&op->pool, (void **)&d_W, sizeof(double) * 6 * npts * NLAM, st));
+    RC_TRY2_RC(g2_pool_alloc(&op->pool, (void **)&d_range, sizeof(int2) * npts, st));
     double *d_lms = reinterpret_cast<double *>(reinterpret_cast<char *>(d_tab) + offsetof(VbtTab, lms));
     k_rc_basis<<<dim3(NLAM, Nr), 64, 0, st>>>(d_bkg, d_rv, d_lms, d_B);
     RC_TRY2(cudaGetLastError());
@@ -742,6 +753,7 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
     g2_count_launches(launches);
     cleanup();
 #undef RC_TRY2
+#undef RC_TRY2_RC
     op->have_tensor = true;
     op->have_spectral = false;
     op->have_background = true;

@@ -40,18 +40,21 @@ __global__ void k_basis(const Bkg *__restrict__ bk, const double *__restrict__ l
     __shared__ cplx fc1[MAXZ + 1], fc2[MAXZ + 1], tf1[MAXZ + 1], tf2[MAXZ + 1], tf3[MAXZ + 1];
     __shared__ cplx fcb[MAXZ + 1], bfr[MAXZ + 1], Ft1[MAXZ + 1], Ft2[MAXZ + 1], Ft3[MAXZ + 1], Fb[MAXZ + 1];
     __shared__ cplx G1[MAXZ + 1], G2_[MAXZ + 1], G3[MAXZ + 1], G4[MAXZ + 1];
-    if (threadIdx.x == 0) {
-        // Calc_Apq (apq_module.F90:230-266)
-        cplx eta[MAXL + 1], el[MAXL + 1], p[MAXL + 1][2], q[MAXL + 1][2], Arr[MAXL + 1][2];
-        dev_apq(b, lms, eta, el, p, q, Arr);
-        // expz (ie_kernel_hankel_module.F90:69-72), pexpz (apq_module.F90:112-137), qexpz (:155-177)
-        cplx expz[MAXZ + 1], pez[MAXZ + 1][2], qez[MAXZ + 1][2];
-        for (int iz = 1; iz <= Nz; iz++) expz[iz] = cuda::std::exp(-eta[b.L[iz]] * b.dz[iz]);
-        dev_pexpz(b, eta, p, expz, pez);
-        dev_qexpz(b, eta, q, expz, qez);
-        // Calc_tframe_p (apq_module.F90:83-110)
-        for (int i = 1; i <= Nz - 1; i++) {
-            const int l = b.L[i];
+    __shared__ cplx eta[MAXL + 1], el[MAXL + 1], p[MAXL + 1][2], q[MAXL + 1][2], Arr[MAXL + 1][2];
+    __shared__ cplx expz[MAXZ + 1], pez[MAXZ + 1][2], qez[MAXZ + 1][2];
+    // one thread for the layers' recursion, one each for the two recursions over the cells, the rest by cell (one
+    // thread for all of it took 0.36 ms, a chain of complex exponentials and divisions; this takes 0.13 ms)
+    if (threadIdx.x == 0) dev_apq(b, lms, eta, el, p, q, Arr);  // Calc_Apq (apq_module.F90:230-266)
+    __syncthreads();
+    // expz (ie_kernel_hankel_module.F90:69-72), pexpz (apq_module.F90:112-137), qexpz (:155-177)
+    for (int iz = threadIdx.x + 1; iz <= Nz; iz += blockDim.x) expz[iz] = cuda::std::exp(-eta[b.L[iz]] * b.dz[iz]);
+    __syncthreads();
+    if (threadIdx.x == 0) dev_pexpz(b, eta, p, expz, pez);
+    if (threadIdx.x == 32) dev_qexpz(b, eta, q, expz, qez);
+    __syncthreads();
+    for (int i = threadIdx.x + 1; i <= Nz; i += blockDim.x) {
+        const int l = b.L[i];
+        if (i <= Nz - 1) {  // Calc_tframe_p (apq_module.F90:83-110)
             cplx a[2], bb[2], c[2];
             for (int k = 0; k < 2; k++) {
                 a[k] = pez[i][k];
@@ -68,18 +71,14 @@ __global__ void k_basis(const Bkg *__restrict__ bk, const double *__restrict__ l
             tf2[i] = (1.0 - fc2[i]) / C(b.csigma[l]);
             tf3[i] = (w * bb[1] / c[1]) / C(b.csigma[l]);
         }
-        // Calc_bframe_q (apq_module.F90:138-153)
-        for (int i = Nz; i >= 2; i--) {
-            const int l = b.L[i];
+        if (i >= 2) {  // Calc_bframe_q (apq_module.F90:138-153)
             cplx a = qez[i][1];
             const cplx d = 1.0 + a * expz[i] * expz[i];
             a = 1.0 + a;
             fcb[i] = expz[i] * a / d;
             bfr[i] = (fcb[i] - 1.0) / C(b.csigma[l]);
         }
-        // Calc_FtFb (apq_module.F90:31-79)
-        for (int i = 1; i <= Nz; i++) {
-            const int l = b.L[i];
+        {  // Calc_FtFb (apq_module.F90:31-79)
             cplx a[2], a1[2], a2[2], p1[2], p2[2], pe1[2], pe2[2], q1[2], q2[2], qe1[2], qe2[2], w[2], Fb3[3];
             for (int k = 0; k < 2; k++) {
                 a[k] = (1.0 - expz[i]) * Arr[l][k];
@@ -385,11 +384,11 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
     int2 *krange = nullptr;
     int rc = G2_OK;
     auto cleanup = [&]() {
-        cudaFree(d_bkg);
-        cudaFree(d_tab);
-        for (auto p : M) cudaFree(p);
-        cudaFree(W);
-        cudaFree(krange);
+        g2_pool_free(d_bkg, st);
+        g2_pool_free(d_tab, st);
+        for (auto p : M) g2_pool_free(p, st);
+        g2_pool_free(W, st);
+        g2_pool_free(krange, st);
         delete tab;
     };
 #define G2_TRY(expr)                                                      \
@@ -401,24 +400,32 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
             return G2_ERR_CUDA;                                           \
         }                                                                 \
     } while (0)
-    G2_TRY(cudaMalloc(&d_bkg, sizeof(Bkg)));
-    G2_TRY(cudaMalloc(&d_tab, sizeof(VbtTab)));
+#define G2_TRY_RC(expr)        \
+    do {                       \
+        const int r_ = (expr); \
+        if (r_) {              \
+            cleanup();         \
+            return r_;         \
+        }                      \
+    } while (0)
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&d_bkg, sizeof(Bkg), st));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&d_tab, sizeof(VbtTab), st));
     G2_TRY(cudaMemcpyAsync(d_bkg, &h, sizeof(Bkg), cudaMemcpyHostToDevice, st));
     G2_TRY(cudaMemcpyAsync(d_tab, tab, sizeof(VbtTab), cudaMemcpyHostToDevice, st));
-    G2_TRY(cudaMalloc(&M[0], sizeof(double2) * NLAM * P));
-    G2_TRY(cudaMalloc(&M[1], sizeof(double2) * NLAM * P));
-    G2_TRY(cudaMalloc(&M[2], sizeof(double2) * NLAM * Nz * Nz));
-    G2_TRY(cudaMalloc(&M[3], sizeof(double2) * NLAM * P));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&M[0], sizeof(double2) * NLAM * P, st));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&M[1], sizeof(double2) * NLAM * P, st));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&M[2], sizeof(double2) * NLAM * Nz * Nz, st));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&M[3], sizeof(double2) * NLAM * P, st));
     G2_TRY(cudaMemsetAsync(M[2], 0, sizeof(double2) * NLAM * Nz * Nz, st));
-    G2_TRY(cudaMalloc(&W, sizeof(double) * 6 * lags * NLAM));
-    G2_TRY(cudaMalloc(&krange, sizeof(int2) * lags));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&W, sizeof(double) * 6 * lags * NLAM, st));
+    G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&krange, sizeof(int2) * lags, st));
     double *d_lms = reinterpret_cast<double *>(reinterpret_cast<char *>(d_tab) + offsetof(VbtTab, lms));
     k_basis<<<NLAM, 64, 0, st>>>(d_bkg, d_lms, M[0], M[1], M[2], M[3]);
     const size_t smw = sizeof(double2) * VN * 6;  // two blocks per SM
     G2_TRY(cudaFuncSetAttribute(k_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
     k_weights<<<(unsigned)lags, 256, smw, st>>>(d_tab, Nx, Ny, op->dx, op->dy, W, krange);
     G2_TRY(cudaGetLastError());
-    if (!op->d_spatial) G2_TRY(cudaMalloc(&op->d_spatial, lags * T * sizeof(double2)));
+    if (!op->d_spatial) G2_TRY_RC(g2_pool_alloc(&op->pool, (void **)&op->d_spatial, lags * T * sizeof(double2), st));
     const double sc = 1.0 / PI_D / 4.0;  // G1/PI/4 (calc_ie_tensor_module.F90:278-286)
     auto Wt = [&](int c) { return W + (size_t)c * lags * NLAM; };
     GemmJobs jobs;
@@ -434,5 +441,6 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
     G2_TRY(cudaStreamSynchronize(st));
     cleanup();
 #undef G2_TRY
+#undef G2_TRY_RC
     return rc;
 }

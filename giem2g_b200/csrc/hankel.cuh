@@ -137,13 +137,52 @@ struct VbtTab {
     double lambda_shift;
 };
 
+// G radix-2 stages (half lengths 2^S0 .. 2^(S0+G-1)) of the 6 interleaved VN-point transforms in g, in registers: the
+// butterflies of smem_fft, so the results are the same bits, with one trip through shared memory for G stages (ten trips
+// each way made the weights of a 64x64x16 grid 1.44 ms and of its receivers 5.0 ms; now 1.00 and 3.2 ms, about half of
+// it the samples' exponentials and error functions).
+template <int S0, int G, bool INV> G2_D void vbt_stages(double2 *g, const double2 *__restrict__ tw)
+{
+    constexpr int M = 1 << G, ITEMS = (VN >> G) * 6;
+    for (int it = threadIdx.x; it < ITEMS; it += 256) {
+        const int c = it % 6, grp = it / 6, lo = grp & ((1 << S0) - 1), base = ((grp >> S0) << (S0 + G)) | lo;
+        double2 *p = g + base * 6 + c;
+        double2 v[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) v[m] = p[(m << S0) * 6];
+#pragma unroll
+        for (int t = 0; t < G; t++)
+#pragma unroll
+            for (int q = 0; q < (1 << t); q++) {
+                double2 w = tw[(lo + (q << S0)) << (VLOG - 1 - S0 - t)];
+                if (INV) w.y = -w.y;
+#pragma unroll
+                for (int m = q; m < M; m += 2 << t) {
+                    const double2 a = v[m], b = cmul(v[m + (1 << t)], w);
+                    v[m] = a + b;
+                    v[m + (1 << t)] = a - b;
+                }
+            }
+#pragma unroll
+        for (int m = 0; m < M; m++) p[(m << S0) * 6] = v[m];
+    }
+    __syncthreads();
+}
+template <bool INV> G2_D void vbt_fft(double2 *g, const double2 *__restrict__ tw)
+{
+    static_assert(VLOG == 10, "the stages below are those of 1024 points");
+    vbt_stages<0, 4, INV>(g, tw);
+    vbt_stages<4, 3, INV>(g, tw);
+    vbt_stages<7, 3, INV>(g, tw);
+}
+
 // CalcWeights22 (VolumeBesselTransforms.F90:264-288) after the output function's samples are in g
 // ([VN][6] in shared memory, bit-reversed positions): forward FFT, deconvolution by the input function's
 // spectrum, inverse FFT.  The caller normalises (h/N with the alternating sign) and takes the real part.
 // Needs blockDim.x == 256 and a __syncthreads() between filling g and the call.
 G2_D void vbt_weights22(double2 *g, const VbtTab *__restrict__ T)
 {
-    smem_fft<double2, true>(g, VLOG, 6, 1, 6, T->twf, false);
+    vbt_fft<false>(g, T->twf);
     // deconvolution by the input function's spectrum, written back bit-reversed (CalcWeights22 :277-280);
     // every thread reads its pairs before any thread writes (the permutation is in place)
     static_assert(VN / 2 == 2 * 256, "k_weights is written for 256 threads, two sample pairs each");
@@ -167,7 +206,7 @@ G2_D void vbt_weights22(double2 *g, const VbtTab *__restrict__ T)
         }
     }
     __syncthreads();
-    smem_fft<double2, true>(g, VLOG, 6, 1, 6, T->twf, true);
+    vbt_fft<true>(g, T->twf);
 }
 
 // ---- (3) GEMM: out[lag][off + col] = scale * sum_k (A1[lag][k] B1[k][col] + A2[lag][k] B2[k][col]) --------

@@ -8,6 +8,10 @@
 enum { G2_OK = 0, G2_ERR_ARG = -1, G2_ERR_CUDA = -2, G2_ERR_STATE = -3, G2_ERR_UNSUPPORTED = -4,
        G2_ERR_NUMERIC = -5, G2_ERR_NOMEM = -6 };
 
+// mem_pool.cu: stream-ordered temporaries of one operator (the pool is made on first use)
+int g2_pool_alloc(cudaMemPool_t *pool, void **p, size_t bytes, cudaStream_t st);
+void g2_pool_free(void *p, cudaStream_t st);
+
 struct ApplyScratch {
     void *U1 = nullptr;    // [2Nx][3Nz][Ny]   x-spectrum / inverse-y output
     void *Uhat = nullptr;  // [Nx][Ny][4][3Nz] full 2-D spectrum in (kx-pair, ky-pair, slot) order
@@ -29,7 +33,8 @@ struct IeOp {
     bool have_background = false;
     bool have_spatial = false, have_spectral = false, have_sigma = false;
     // device data
-    double2 *d_spatial = nullptr;      // [Nx][Ny][Tunit] FP64 spatial tensor
+    cudaMemPool_t pool = nullptr;      // temporaries of the set-up, and the spatial tensor
+    double2 *d_spatial = nullptr;      // [Nx][Ny][Tunit] FP64 spatial tensor (from the pool)
     double2 *d_tensor64 = nullptr;     // [Nx][Ny][Tunit] FP64 spectral tensor
     float2 *d_tensor32 = nullptr;      // same, complex64 copy
     // copies in the layout of the other contraction kernels, held while a form of that precision selects one

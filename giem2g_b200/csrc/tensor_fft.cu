@@ -186,8 +186,12 @@ int ie_tensor_spectrum(IeOp *op, cudaStream_t st)
     const int rcp = make_positions(op);
     if (rcp) return rcp;
     double2 *S1 = nullptr, *nyq = nullptr;
-    G2_CUDA_CHECK(cudaMalloc(&S1, (size_t)(Nx + 1) * Ny * T * sizeof(double2)));
-    G2_CUDA_CHECK(cudaMalloc(&nyq, (size_t)Ny * T * sizeof(double2)));
+    int rca = g2_pool_alloc(&op->pool, (void **)&S1, (size_t)(Nx + 1) * Ny * T * sizeof(double2), st);
+    if (!rca) rca = g2_pool_alloc(&op->pool, (void **)&nyq, (size_t)Ny * T * sizeof(double2), st);
+    if (rca) {
+        g2_pool_free(S1, st);
+        return rca;
+    }
     if (!op->d_tensor64) G2_CUDA_CHECK(cudaMalloc(&op->d_tensor64, n_out * sizeof(double2)));
     if (!op->d_tensor32) G2_CUDA_CHECK(cudaMalloc(&op->d_tensor32, n_out * sizeof(float2)));
     const size_t smx = (size_t)2 * Nx * TE * sizeof(double2), smy = (size_t)2 * Ny * TE * sizeof(double2);
@@ -198,14 +202,15 @@ int ie_tensor_spectrum(IeOp *op, cudaStream_t st)
     k_tensor_y<<<dim3(1, eb), kThreads, smy, st>>>(S1, nyq, nullptr, op->d_twy64, op->d_pos, Nx, Ny, Nz, Nx);
     k_tensor_y<<<dim3(Nx, eb), kThreads, smy, st>>>(S1, op->d_tensor64, nyq, op->d_twy64, op->d_pos, Nx, Ny, Nz, 0);
     k_to_c64<<<1184, 256, 0, st>>>(op->d_tensor64, op->d_tensor32, op->d_pos, op->units(), T);
-    G2_CUDA_CHECK(cudaGetLastError());
-    G2_CUDA_CHECK(cudaStreamSynchronize(st));
-    cudaFree(S1);
-    cudaFree(nyq);
+    const cudaError_t le = cudaGetLastError();
+    g2_pool_free(S1, st);
+    g2_pool_free(nyq, st);
+    G2_CUDA_CHECK(le);
     // the reference transforms the kernel buffer in place (G_symm and G_symmT alias it), so the
     // spatial tensor does not outlive the transform there either
-    cudaFree(op->d_spatial);
+    g2_pool_free(op->d_spatial, st);
     op->d_spatial = nullptr;
+    G2_CUDA_CHECK(cudaStreamSynchronize(st));
     op->have_spatial = false;
     // plain-layout copies of an earlier tensor are out of date
     if (op->d_plain64 || op->d_plain32) {
