@@ -74,17 +74,18 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fx(con
                                                  CT<R> *__restrict__ U1, const CT<R> *__restrict__ twg, int Nx,
                                                  int Ny, int Nz, int NL, const int *gate)
 {
-    if (gate && *gate == 0) return;
     using C = CT<R>;
     constexpr int N1 = Fact<L>::N1, N2 = Fact<L>::N2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
     C *sm = tw + L;
+    load_tw(tw, twg, L);  // the table is older than the kernels before this one
+    pdl_wait();
+    if (gate && *gate == 0) return;
     // indices fit 32 bits: every buffer holds fewer than 2^31 elements for 2Nx, 2Ny <= 1024
     const int Z3 = 3 * Nz, ZL = vs.nv * Z3, zc0 = blockIdx.x * NL, y = blockIdx.y;
     const int nl = min(NL, ZL - zc0);
     const int plane = Nx * Ny, row = y * Nx;
-    load_tw(tw, twg, L);
     __syncthreads();
     auto load = [&](int t, int x) -> C {
         const int zc = zc0 + t, v = zc >= Z3 ? 1 : 0, lzc = zc - v * Z3, z = lzc % Nz;
@@ -103,12 +104,14 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(con
                                                  const CT<R> *__restrict__ twg, int Nx, int Ny, int Nz, int NL,
                                                  int nv, int pitch, const int *gate)
 {
-    if (gate && *gate == 0) return;
     using C = CT<R>;
     constexpr int N1 = Fact<L>::N1, N2 = Fact<L>::N2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
     C *sm = tw + L;
+    load_tw(tw, twg, L);  // the table is older than the kernels before this one
+    pdl_wait();
+    if (gate && *gate == 0) return;
     const int Z3 = nv * 3 * Nz, zc0 = blockIdx.x * NL, kx = blockIdx.y;  // Z3: lines of all vectors
     // in the spectrum a vector's 3Nz lines are `pitch` elements apart from the next vector's
     const int ZP = nv * pitch, gap = pitch - 3 * Nz;
@@ -125,7 +128,6 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(con
         }
         return;
     }
-    load_tw(tw, twg, L);
     __syncthreads();
     const C *col = U1 + kx * Ny * Z3 + zc0;
     C *dst = Uh + q * Ny * 4 * ZP + sx * 2 * ZP;
@@ -145,12 +147,14 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_by(con
                                                  const CT<R> *__restrict__ twg, int Nx, int Ny, int Nz, int NL,
                                                  int nv, int pitch, const int *gate)
 {
-    if (gate && *gate == 0) return;
     using C = CT<R>;
     constexpr int N1 = Fact<L>::N1, N2 = Fact<L>::N2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
     C *sm = tw + L;
+    load_tw(tw, twg, L);  // the table is older than the kernels before this one
+    pdl_wait();
+    if (gate && *gate == 0) return;
     const int Z3 = nv * 3 * Nz, zc0 = blockIdx.x * NL, kx = blockIdx.y;  // Z3: lines of all vectors
     // in the spectrum a vector's 3Nz lines are `pitch` elements apart from the next vector's
     const int ZP = nv * pitch, gap = pitch - 3 * Nz;
@@ -159,7 +163,6 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_by(con
     const int nl = min(NL, Z3 - zc0);
     int q, sx;
     kx_to_slot(kx, Nx, q, sx);
-    load_tw(tw, twg, L);
     __syncthreads();
     const C *src = Uh + q * Ny * 4 * ZP + sx * 2 * ZP;
     C *col = U1 + kx * Ny * Z3 + zc0;
@@ -181,16 +184,17 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_bx(con
                                                  const CT<R> *__restrict__ twg, int Nx, int Ny, int Nz, int NL,
                                                  const int *gate)
 {
-    if (gate && *gate == 0) return;
     using C = CT<R>;
     constexpr int N1 = Fact<L>::N1, N2 = Fact<L>::N2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *tw = reinterpret_cast<C *>(smem_raw);
     C *sm = tw + L;
+    load_tw(tw, twg, L);  // the table is older than the kernels before this one
+    pdl_wait();
+    if (gate && *gate == 0) return;
     const int Z3 = 3 * Nz, ZL = vs.nv * Z3, zc0 = blockIdx.x * NL, y = blockIdx.y;
     const int nl = min(NL, ZL - zc0);
     const int plane = Nx * Ny, row = y * Nx;
-    load_tw(tw, twg, L);
     __syncthreads();
     auto load = [&](int t, int kx) -> C {
         return kx == L / 2 ? czero<C>() : U1[(kx * Ny + y) * ZL + zc0 + t];  // L = 2Nx
@@ -224,6 +228,7 @@ template <typename R>
 __global__ void k_contract(const CT<R> *__restrict__ G, CT<R> *__restrict__ Uhat, int Nx, int Ny, int Nz,
                            const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     const int AW = sizeof(R) == 8 ? asw_width64(Nz) : asw_width32(Nz);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -392,9 +397,9 @@ static void launch_x_k(bool fwd, IeOp *op, const VecSet<CT<R>> &vs, CT<R> *U1, c
     static bool attr = false;
     if (!attr) { big_smem(k_fx<R, L, CAP>); big_smem(k_bx<R, L, CAP>); attr = true; }
     if (fwd)
-        k_fx<R, L, CAP><<<grid, nt, sm, st>>>(vs, Bufs<R>::gsig(op), U1, Bufs<R>::twx(op), Nx, Ny, Nz, NL, gate);
+        g2_launch(k_fx<R, L, CAP>, grid, nt, sm, st, vs, Bufs<R>::gsig(op), U1, Bufs<R>::twx(op), Nx, Ny, Nz, NL, gate);
     else
-        k_bx<R, L, CAP><<<grid, nt, sm, st>>>(U1, vs, Bufs<R>::asig(op), Bufs<R>::post(op), Bufs<R>::twx(op), Nx,
+        g2_launch(k_bx<R, L, CAP>, grid, nt, sm, st, U1, vs, Bufs<R>::asig(op), Bufs<R>::post(op), Bufs<R>::twx(op), Nx,
                                               Ny, Nz, NL, gate);
 }
 
@@ -417,8 +422,8 @@ static void launch_y_k(bool fwd, IeOp *op, int nv, int pitch, CT<R> *U1, CT<R> *
     const int Nx = op->Nx, Ny = op->Ny, Nz = op->Nz;
     static bool attr = false;
     if (!attr) { big_smem(k_fy<R, L, CAP>); big_smem(k_by<R, L, CAP>); attr = true; }
-    if (fwd) k_fy<R, L, CAP><<<grid, nt, sm, st>>>(U1, Uh, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, pitch, gate);
-    else k_by<R, L, CAP><<<grid, nt, sm, st>>>(Uh, U1, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, pitch, gate);
+    if (fwd) g2_launch(k_fy<R, L, CAP>, grid, nt, sm, st, U1, Uh, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, pitch, gate);
+    else g2_launch(k_by<R, L, CAP>, grid, nt, sm, st, Uh, U1, Bufs<R>::twy(op), Nx, Ny, Nz, NL, nv, pitch, gate);
 }
 
 template <typename R, int L>
@@ -514,7 +519,7 @@ static int ie_apply_core(IeOp *op, const CT<R> *d_in, CT<R> *d_out, cudaStream_t
         const int T = op->Tunit();
         const size_t sm = ((size_t)T + 4 * Z3) * es;
         const int threads = ((Z3 + 31) / 32) * 32;
-        k_contract<R><<<(unsigned)op->units(), threads, sm, st>>>(G, Uh, Nx, Ny, Nz, gate);
+        g2_launch(k_contract<R>, (unsigned)op->units(), threads, sm, st, G, Uh, Nx, Ny, Nz, gate);
     }
     if (timed) cudaEventRecord(op->evc1, st);
     dispatch_y<R>(false, op, 1, pitch, U1, Uh, st, gate);
@@ -538,11 +543,13 @@ int ie_apply_device64(IeOp *op, const double2 *d_in, double2 *d_out, cudaStream_
 namespace {
 __global__ void k_c128_to_c64(const double2 *__restrict__ a, float2 *__restrict__ b, long long n)
 {
+    pdl_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         b[i] = make_float2((float)a[i].x, (float)a[i].y);
 }
 __global__ void k_c64_to_c128(const float2 *__restrict__ a, double2 *__restrict__ b, long long n)
 {
+    pdl_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         b[i] = make_double2((double)a[i].x, (double)a[i].y);
 }
@@ -557,11 +564,11 @@ int ie_apply_host_mixed(IeOp *op, const double2 *d_in, double2 *d_out, cudaStrea
         G2_CUDA_CHECK(cudaMalloc(&op->d_vout32, n * sizeof(float2)));
     }
     const int blocks = (int)std::min<long long>((n + 255) / 256, 148LL * 16);
-    k_c128_to_c64<<<blocks, 256, 0, st>>>(d_in, op->d_vin32, n);
+    g2_launch(k_c128_to_c64, blocks, 256, 0, st, d_in, op->d_vin32, n);
     G2_CUDA_CHECK(cudaGetLastError());
     int rc = ie_apply_device32(op, op->d_vin32, op->d_vout32, st);
     if (rc) return rc;
-    k_c64_to_c128<<<blocks, 256, 0, st>>>(op->d_vout32, d_out, n);
+    g2_launch(k_c64_to_c128, blocks, 256, 0, st, op->d_vout32, d_out, n);
     G2_CUDA_CHECK(cudaGetLastError());
     g2_count_launches(2);
     return G2_OK;

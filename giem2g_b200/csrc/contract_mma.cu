@@ -262,7 +262,6 @@ template <int KT1, int KT2, int NG_>
 __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
     k_contract_mma64(const double2 *__restrict__ G, double2 *__restrict__ Uhat, MmaArgs a, int *err, const int *gate)
 {
-    if (gate && *gate == 0) return;  // uniform across the CTA: nothing has been issued yet
     using Cfg = MmaCfg64<KT1, KT2, NG_>;
     constexpr int KT = Cfg::KT, W = Cfg::W;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -275,6 +274,8 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
     for (int kt = 0; kt < KT; kt++)
         off[kt] = (uint32_t)mma_offset<KT1>(rt, nl, kt, kl, Nz, P, T + u_elems) |
                   (uint32_t)mma_offset<KT1>(rt, nl, kt, kl + 4, Nz, P, T + u_elems) << 16;
+    pdl_wait();  // the offsets above need nothing of the kernels before this one
+    if (gate && *gate == 0) return;
     mma_ring<double2, W, NG_, true>(smem, G, Uhat, a, u_elems, T, err,
                               [&](const unsigned char *g, const unsigned char *us, long long unit, auto release) {
         const double *u = reinterpret_cast<const double *>(us) + 2 * pt * a.pitch + comp;
@@ -474,7 +475,6 @@ template <int NP, int KZ, bool HALF, int NG_>
 __global__ void __launch_bounds__(MmaCfg32<KZ, NG_>::NTHREADS, 1)
     k_contract_mma32(const float2 *__restrict__ G, float2 *__restrict__ Uhat, MmaArgs a, int *err, const int *gate)
 {
-    if (gate && *gate == 0) return;
     extern __shared__ __align__(128) unsigned char smem[];
     const int Nz = a.Nz, P = Nz * (Nz + 1) / 2, T = 4 * P + 2 * Nz * Nz, u_elems = 4 * NP * a.pitch;
     const int lane = threadIdx.x & 31, rt = (threadIdx.x >> 5) % KZ;
@@ -496,6 +496,8 @@ __global__ void __launch_bounds__(MmaCfg32<KZ, NG_>::NTHREADS, 1)
                         k1 < Nz ? 4 * P + full_pos<false>(k1, z, Nz) : zero);
         }
     }
+    pdl_wait();
+    if (gate && *gate == 0) return;
     mma_ring<float2, KZ, NG_, false>(smem, G, Uhat, a, u_elems, T, err,
                               [&](const unsigned char *g, const unsigned char *us, long long unit, auto release) {
         const float2 *u = reinterpret_cast<const float2 *>(us) + pt * a.pitch;
@@ -569,7 +571,7 @@ int launch_mma(K kern, int nthreads, int multiple, int pts, const void *G, void 
     if (a.nstage < 1) return G2_ERR_UNSUPPORTED;
     const int sm = a.nstage * (a.stage_bytes + 16);
     const int grid = (int)(a.nunits < mma_sms() ? a.nunits : mma_sms());
-    kern<<<grid, nthreads, sm, st>>>(reinterpret_cast<const C *>(G), reinterpret_cast<C *>(Uhat), a, err, gate);
+    g2_launch(kern, grid, nthreads, sm, st, reinterpret_cast<const C *>(G), reinterpret_cast<C *>(Uhat), a, err, gate);
     G2_CUDA_CHECK(cudaGetLastError());
     return G2_OK;
 }

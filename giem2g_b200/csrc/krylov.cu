@@ -350,6 +350,7 @@ template <typename C, int K>
 __global__ void __launch_bounds__(kVT) k_dots_first_t(const C *__restrict__ V, size_t ld, const C *__restrict__ w,
                                                       size_t N, double2 *part, Level L, const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     dots_first_body<C, K>(V, ld, w, N, part, L);
 }
@@ -369,6 +370,7 @@ struct Multi {
 template <typename C, int K>
 __global__ void __launch_bounds__(kVT) k_dots_first_m(Multi<C> mm, size_t ld, size_t N)
 {
+    pdl_wait();
     const int y = blockIdx.y;
     if (mm.gate[y] && *mm.gate[y] == 0) return;
     Level L = mm.L[y];
@@ -500,12 +502,14 @@ template <typename C, int K>
 __global__ void __launch_bounds__(kVT) k_cgs_pass_fused_t(const C *__restrict__ V, size_t ld, C *__restrict__ w,
                                                           size_t N, double2 *part, Level L, int p, const int *gate)
 {
+    pdl_wait();
     if ((gate && *gate == 0) || L.flags[F_PASS] == 0) return;
     cgs_pass_body<C, K>(V, ld, w, N, part, L, p);
 }
 template <typename C, int K>
 __global__ void __launch_bounds__(kVT) k_cgs_pass_fused_m(Multi<C> mm, size_t ld, size_t N, int p)
 {
+    pdl_wait();
     const int y = blockIdx.y;
     if ((mm.gate[y] && *mm.gate[y] == 0) || mm.L[y].flags[F_PASS] == 0) return;
     Level L = mm.L[y];
@@ -517,6 +521,7 @@ template <typename C>
 __global__ void __launch_bounds__(kVT) k_norm2_fused(const C *__restrict__ w, size_t N, double2 *part, double *nrm2,
                                                      unsigned *counter, const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     using R = typename RealOf<C>::T;
     using W = typename Wide<C>::T;
@@ -600,6 +605,7 @@ template <typename C>
 __global__ void __launch_bounds__(kVT) k_scale_finish(C *v, const C *w, size_t N, Level L, int j, double tol,
                                                       const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     scale_finish_body<C>(v, w, N, L, j, tol);
 }
@@ -607,6 +613,7 @@ __global__ void __launch_bounds__(kVT) k_scale_finish(C *v, const C *w, size_t N
 template <typename C>
 __global__ void __launch_bounds__(kVT) k_scale_finish_m(Multi<C> mm, size_t N, int j, double tol)
 {
+    pdl_wait();
     const int y = blockIdx.y;
     if (mm.gate[y] && *mm.gate[y] == 0) return;
     Level L = mm.L[y];
@@ -620,6 +627,7 @@ __global__ void __launch_bounds__(kVT) k_scale_finish_m(Multi<C> mm, size_t N, i
 constexpr int kTriThreads = 128;
 __global__ void __launch_bounds__(kTriThreads) k_trisolve(Level L, const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     __shared__ double2 Hs[KMAX * (KMAX + 1)];  // column j < n of the triangle at j * KMAX, then g at n * KMAX
     __shared__ double2 ys[KMAX];
@@ -650,6 +658,7 @@ __global__ void __launch_bounds__(kTriThreads) k_trisolve(Level L, const int *ga
 // start of a cycle: H(0,m) = beta, H(1..m, m) = 0, krylov active (gmres.F90:172-185)
 __global__ void k_cycle_start(Level L, const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     const int m = L.m;
     L.H[hix(0, m, m)] = make_double2(L.scal[S_BETA], 0.0);
@@ -661,6 +670,7 @@ __global__ void k_cycle_start(Level L, const int *gate)
 // inner solve start: bn from nrm2; beta from the residual; exit when beta/bn < tol (gmres.F90:139-168)
 __global__ void k_set_bn(Level L)
 {
+    pdl_wait();
     L.scal[S_BN] = sqrt(L.scal[S_NRM2]);
     L.flags[F_SOLVER] = L.scal[S_BN] < ZERO_THRESHOLD ? 0 : 1;
     L.flags[F_ITER] = 0;
@@ -670,6 +680,7 @@ __global__ void k_set_bn(Level L)
 }
 __global__ void k_set_beta(Level L, double tol)
 {
+    pdl_wait();
     if (L.flags[F_SOLVER] == 0) return;
     const double beta = sqrt(L.scal[S_NRM2]);
     L.scal[S_BETA] = beta;
@@ -680,6 +691,7 @@ __global__ void k_set_beta(Level L, double tol)
 }
 __global__ void k_zero_level(Level L)
 {
+    pdl_wait();
     const int n = (L.m + 1) * (L.m + 1);
     for (int i = threadIdx.x; i < n; i += blockDim.x) L.H[i] = make_double2(0.0, 0.0);
 }
@@ -687,6 +699,7 @@ __global__ void k_zero_level(Level L)
 // restart (gmres.F90:369-376): beta = |g_m|, g <- inverse rotations of (0..0, g_m)
 __global__ void k_restart_g(Level L)
 {
+    pdl_wait();
     const int m = L.m;
     L.scal[S_BETA] = cabs_(L.H[hix(m, m, m)]);
     for (int J = m - 1; J >= 0; J--) {
@@ -702,6 +715,7 @@ template <typename CO, typename CX, typename CY>
 __global__ void __launch_bounds__(kVT) k_axpby(CO *out, double a, const CX *x, double b, const CY *y, size_t N,
                                                const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     auto elem = [&](double2 xv, double2 yv) {
         double2 r = make_double2(a * xv.x, a * xv.y);
@@ -731,6 +745,7 @@ __global__ void __launch_bounds__(kVT) k_axpby(CO *out, double a, const CX *x, d
 template <typename C>
 __global__ void __launch_bounds__(kVT) k_copy_or_zero(C *x, const C *v, const double *scal, size_t N)
 {
+    pdl_wait();
     const bool zero = scal[S_BN] < ZERO_THRESHOLD;
     for (size_t i = blockIdx.x * (size_t)kVT + threadIdx.x; i < N; i += (size_t)gridDim.x * kVT)
         st2(x, i, zero ? make_double2(0.0, 0.0) : ld2(v, i));
@@ -740,6 +755,7 @@ template <typename C>
 __global__ void __launch_bounds__(kVT) k_scale_by(C *v, const C *w, const double *scal, int idx, size_t N,
                                                   const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     const double inv = 1.0 / scal[idx];
     for (size_t i = blockIdx.x * (size_t)kVT + threadIdx.x; i < N; i += (size_t)gridDim.x * kVT) {
@@ -753,6 +769,7 @@ __global__ void __launch_bounds__(kVT) k_lincomb(CO *out, double a0, const CO *i
                                                  size_t ld, const double2 *__restrict__ coef, const int *nflag,
                                                  size_t N, const int *gate)
 {
+    pdl_wait();
     if (gate && *gate == 0) return;
     __shared__ double2 cs[KMAX + 1];
     const int n = *nflag;
@@ -818,6 +835,7 @@ __global__ void __launch_bounds__(kVT) k_lincomb(CO *out, double a0, const CO *i
 // copy the g column into a coefficient vector (restart residual w = V g)
 __global__ void k_copy_g(Level L)
 {
+    pdl_wait();
     const int m = L.m;
     for (int i = threadIdx.x; i <= m; i += blockDim.x) L.y[i] = L.H[hix(i, m, m)];
 }
@@ -825,6 +843,7 @@ __global__ void k_copy_g(Level L)
 // SolveEquation helpers (ie_solver_module.F90:64-97); vectors are [c][cell], cell = z*NxNy + y*Nx + x
 __global__ void k_rhs(double2 *rhs, const double2 *Ebkg, const double *post, size_t plane, int Nz)
 {
+    pdl_wait();
     const size_t n = 3 * plane * Nz;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int z = (int)((i / plane) % Nz);
@@ -833,6 +852,7 @@ __global__ void k_rhs(double2 *rhs, const double2 *Ebkg, const double *post, siz
 }
 __global__ void k_scale_asig(double2 *out, const double2 *in, const double2 *asig, size_t cells, bool divide)
 {
+    pdl_wait();
     const size_t n = 3 * cells;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double2 a = asig[i % cells];
@@ -1010,12 +1030,12 @@ template <typename C, int K>
 static void launch_dots_first_k(KrylovWork *k, const C *V, const C *w, Level &L, const int *g, cudaStream_t st)
 {
     static const int per_sm = resident_blocks(k_dots_first_t<C, K>);
-    k_dots_first_t<C, K><<<wave_grid(per_sm, k->nparts, 1), kVT, 0, st>>>(V, k->N, w, k->N, k->part, L, g);
+    g2_launch(k_dots_first_t<C, K>, wave_grid(per_sm, k->nparts, 1), kVT, 0, st, V, k->N, w, k->N, k->part, L, g);
 }
 template <typename C, int K>
 static void launch_pass_fused_k(KrylovWork *k, const C *V, C *w, Level &L, int p, const int *g, cudaStream_t st)
 {
-    k_cgs_pass_fused_t<C, K><<<k->nparts, kVT, 0, st>>>(V, k->N, w, k->N, k->part, L, p, g);
+    g2_launch(k_cgs_pass_fused_t<C, K>, k->nparts, kVT, 0, st, V, k->N, w, k->N, k->part, L, p, g);
 }
 #define G2_KCASES(F, ...)                                                                                     \
     switch (K) {                                                                                          \
@@ -1042,7 +1062,7 @@ template <typename C>
 static void norm2(KrylovWork *k, const C *w, double *nrm2, const int *g, cudaStream_t st)
 {
     // kernels on one stream run one after another, so any level's counter serves
-    k_norm2_fused<C><<<k->nparts, kVT, 0, st>>>(w, k->N, k->part, nrm2, k->Lo.counter, g); g2_count_launches(1);
+    g2_launch(k_norm2_fused<C>, k->nparts, kVT, 0, st, w, k->N, k->part, nrm2, k->Lo.counter, g); g2_count_launches(1);
 }
 
 // CGS for Arnoldi step j on level L with basis V (j+1 columns) and vector w: the first pass's dots and
@@ -1062,7 +1082,7 @@ static void cgs(KrylovWork *k, Level &L, const C *V, int j, C *w, const int *gat
 template <typename C>
 static void arnoldi_tail(KrylovWork *k, Level &L, C *V, int j, const C *w, double tol, const int *gate, cudaStream_t st)
 {
-    k_scale_finish<C><<<sweep_grid(k->N), kVT, 0, st>>>(V + (size_t)(j + 1) * k->N, w, k->N, L, j, tol, gate);
+    g2_launch(k_scale_finish<C>, sweep_grid(k->N), kVT, 0, st, V + (size_t)(j + 1) * k->N, w, k->N, L, j, tol, gate);
     g2_count_launches(1);
 }
 
@@ -1072,12 +1092,12 @@ template <typename C, int K>
 static void launch_dots_first_km(const Multi<C> &mm, int n, size_t N, int nparts, cudaStream_t st)
 {
     static const int per_sm = resident_blocks(k_dots_first_m<C, K>);
-    k_dots_first_m<C, K><<<dim3(wave_grid(per_sm, nparts, n), n), kVT, 0, st>>>(mm, N, N);
+    g2_launch(k_dots_first_m<C, K>, dim3(wave_grid(per_sm, nparts, n), n), kVT, 0, st, mm, N, N);
 }
 template <typename C, int K>
 static void launch_pass_fused_km(const Multi<C> &mm, int n, size_t N, int nparts, int p, cudaStream_t st)
 {
-    k_cgs_pass_fused_m<C, K><<<dim3(nparts, n), kVT, 0, st>>>(mm, N, N, p);
+    g2_launch(k_cgs_pass_fused_m<C, K>, dim3(nparts, n), kVT, 0, st, mm, N, N, p);
 }
 template <typename C>
 static void cgs_multi(const Multi<C> &mm, int n, size_t N, int nparts, int j, cudaStream_t st)
@@ -1093,7 +1113,7 @@ static void cgs_multi(const Multi<C> &mm, int n, size_t N, int nparts, int j, cu
 template <typename C>
 static void arnoldi_tail_multi(const Multi<C> &mm, int n, size_t N, int j, double tol, cudaStream_t st)
 {
-    k_scale_finish_m<C><<<dim3(sweep_grid(N), n), kVT, 0, st>>>(mm, N, j, tol);
+    g2_launch(k_scale_finish_m<C>, dim3(sweep_grid(N), n), kVT, 0, st, mm, N, j, tol);
     g2_count_launches(1);
 }
 
@@ -1117,19 +1137,19 @@ static int inner_solve(IeOp *op, KrylovWork *k, const CI *v, const CI *x0, CI *x
     const int g = vec_grid(N);
     CI *Vi = reinterpret_cast<CI *>(k->Vi), *ri = reinterpret_cast<CI *>(k->ri), *wi = reinterpret_cast<CI *>(k->wi);
     const int *solver = L.flags + F_SOLVER, *krylov = L.flags + F_KRYLOV;
-    k_zero_level<<<1, 256, 0, st>>>(L); g2_count_launches(1);
+    g2_launch(k_zero_level, 1, 256, 0, st, L); g2_count_launches(1);
     norm2<CI>(k, v, L.scal + S_NRM2, nullptr, st);
-    k_set_bn<<<1, 1, 0, st>>>(L); g2_count_launches(1);
-    k_copy_or_zero<CI><<<g, kVT, 0, st>>>(x, x0, L.scal, N);  // x = x0, or 0 when ||b|| < 1e-14
+    g2_launch(k_set_bn, 1, 1, 0, st, L); g2_count_launches(1);
+    g2_launch(k_copy_or_zero<CI>, g, kVT, 0, st, x, x0, L.scal, N);  // x = x0, or 0 when ||b|| < 1e-14
     int rc = apply_prec<CI>(op, x0, ri, st, solver);
     if (rc) return rc;
     k->applies32 += sizeof(CI) == 8 ? 1 : 0;
     k->applies64 += sizeof(CI) == 16 ? 1 : 0;
-    k_axpby<CI, CI, CI><<<g, kVT, 0, st>>>(ri, 1.0, v, -1.0, ri, N, solver);  // r0 = b - A x0
+    g2_launch(k_axpby<CI, CI, CI>, g, kVT, 0, st, ri, 1.0, v, -1.0, ri, N, solver);  // r0 = b - A x0
     norm2<CI>(k, ri, L.scal + S_NRM2, solver, st);
-    k_set_beta<<<1, 1, 0, st>>>(L, tol); g2_count_launches(1);
-    k_cycle_start<<<1, 1, 0, st>>>(L, solver); g2_count_launches(1);
-    k_scale_by<CI><<<g, kVT, 0, st>>>(Vi, ri, L.scal, S_BETA, N, solver); g2_count_launches(1);
+    g2_launch(k_set_beta, 1, 1, 0, st, L, tol); g2_count_launches(1);
+    g2_launch(k_cycle_start, 1, 1, 0, st, L, solver); g2_count_launches(1);
+    g2_launch(k_scale_by<CI>, g, kVT, 0, st, Vi, ri, L.scal, S_BETA, N, solver); g2_count_launches(1);
     for (int j = 0; j < k->mi; j++) {
         CI *Vj = Vi + (size_t)j * N;
         rc = apply_prec<CI>(op, Vj, wi, st, krylov);
@@ -1140,8 +1160,8 @@ static int inner_solve(IeOp *op, KrylovWork *k, const CI *v, const CI *x0, CI *x
         arnoldi_tail<CI>(k, L, Vi, j, wi, tol, krylov, st);
     }
     // FinalActions -> ConstructCurrentSolution (gmres.F90:423-458): x = x0 + V y
-    k_trisolve<<<1, kTriThreads, 0, st>>>(L, solver); g2_count_launches(1);
-    k_lincomb<CI, CI><<<g, kVT, 0, st>>>(x, 1.0, x, Vi, N, L.y, L.flags + F_L, N, solver); g2_count_launches(1);
+    g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, solver); g2_count_launches(1);
+    g2_launch(k_lincomb<CI, CI>, g, kVT, 0, st, x, 1.0, x, Vi, N, L.y, L.flags + F_L, N, solver); g2_count_launches(1);
     if (true_residual) {  // gmres.F90:402-419, result unused by the outer solver
         rc = apply_prec<CI>(op, x, ri, st, solver);
         if (rc) return rc;
@@ -1233,9 +1253,9 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
     info->bea = -1.0;
     info->be = -1.0;
     // gmres.F90:129-168
-    k_zero_level<<<1, 256, 0, st>>>(L); g2_count_launches(1);
+    g2_launch(k_zero_level, 1, 256, 0, st, L); g2_count_launches(1);
     norm2<double2>(k, k->b, L.scal + S_NRM2, nullptr, st);
-    k_set_bn<<<1, 1, 0, st>>>(L); g2_count_launches(1);
+    g2_launch(k_set_bn, 1, 1, 0, st, L); g2_count_launches(1);
     int rc = pull();
     if (rc) return rc;
     if (h_scal[S_BN] < ZERO_THRESHOLD) {
@@ -1247,10 +1267,10 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
     rc = ie_apply_device64(op, k->x, k->r0, st);  // x holds x0
     if (rc) return rc;
     k->applies64++;
-    k_axpby<double2, double2, double2><<<g, kVT, 0, st>>>(k->r0, 1.0, k->b, -1.0, k->r0, N, nullptr); g2_count_launches(1);
-    k_axpby<double2, double2, double2><<<g, kVT, 0, st>>>(k->w, 1.0, k->r0, 0.0, (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
+    g2_launch(k_axpby<double2, double2, double2>, g, kVT, 0, st, k->r0, 1.0, k->b, -1.0, k->r0, N, nullptr); g2_count_launches(1);
+    g2_launch(k_axpby<double2, double2, double2>, g, kVT, 0, st, k->w, 1.0, k->r0, 0.0, (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
     norm2<double2>(k, k->w, L.scal + S_NRM2, nullptr, st);
-    k_set_beta<<<1, 1, 0, st>>>(L, tol); g2_count_launches(1);
+    g2_launch(k_set_beta, 1, 1, 0, st, L, tol); g2_count_launches(1);
     if ((rc = pull())) return rc;
     if (h_scal[S_BETA] / bn < tol) {
         info->stat = 1;
@@ -1263,8 +1283,8 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
     double bea = -1.0;
     char msg[256];
     for (;;) {
-        k_cycle_start<<<1, 1, 0, st>>>(L, nullptr); g2_count_launches(1);
-        k_scale_by<double2><<<g, kVT, 0, st>>>(k->Vo, k->w, L.scal, S_BETA, N, nullptr); g2_count_launches(1);
+        g2_launch(k_cycle_start, 1, 1, 0, st, L, nullptr); g2_count_launches(1);
+        g2_launch(k_scale_by<double2>, g, kVT, 0, st, k->Vo, k->w, L.scal, S_BETA, N, nullptr); g2_count_launches(1);
         for (int j = 0; j < M; j++) {
             const double2 *Vj = k->Vo + (size_t)j * N;
             CI *Zj = Z + (size_t)j * N;
@@ -1278,20 +1298,20 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
                 else hook_off = true;
             }
             if (hooked && op->precond_mode == 2) {
-                k_axpby<CI, double2, double2><<<g, kVT, 0, st>>>(Zj, 1.0, k->tmp, 0.0, (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
+                g2_launch(k_axpby<CI, double2, double2>, g, kVT, 0, st, Zj, 1.0, k->tmp, 0.0, (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
             } else {
-                k_axpby<CI, double2, double2><<<g, kVT, 0, st>>>(vin, 1.0, Vj, 0.0, (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
+                g2_launch(k_axpby<CI, double2, double2>, g, kVT, 0, st, vin, 1.0, Vj, 0.0, (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
                 if (hooked) {
-                    k_axpby<CI, double2, double2><<<g, kVT, 0, st>>>(reinterpret_cast<CI *>(k->x0in), 1.0, k->tmp, 0.0,
+                    g2_launch(k_axpby<CI, double2, double2>, g, kVT, 0, st, reinterpret_cast<CI *>(k->x0in), 1.0, k->tmp, 0.0,
                                                                      (const double2 *)nullptr, N, nullptr); g2_count_launches(1);
                 }
                 if ((rc = inner_solve_fixed<CI>(op, k, tol, true_res, hooked, st))) return rc;
-                k_axpby<CI, CI, CI><<<g, kVT, 0, st>>>(Zj, 1.0, reinterpret_cast<const CI *>(k->xin), 0.0, (const CI *)nullptr, N, nullptr); g2_count_launches(1);
+                g2_launch(k_axpby<CI, CI, CI>, g, kVT, 0, st, Zj, 1.0, reinterpret_cast<const CI *>(k->xin), 0.0, (const CI *)nullptr, N, nullptr); g2_count_launches(1);
             }
             if (sizeof(CI) == sizeof(double2)) {
                 if ((rc = ie_apply_device64(op, reinterpret_cast<const double2 *>(Zj), k->w, st))) return rc;
             } else {
-                k_axpby<double2, CI, CI><<<g, kVT, 0, st>>>(k->tmp, 1.0, Zj, 0.0, (const CI *)nullptr, N, nullptr); g2_count_launches(1);
+                g2_launch(k_axpby<double2, CI, CI>, g, kVT, 0, st, k->tmp, 1.0, Zj, 0.0, (const CI *)nullptr, N, nullptr); g2_count_launches(1);
                 if ((rc = ie_apply_device64(op, k->tmp, k->w, st))) return rc;
             }
             k->applies64++;
@@ -1318,20 +1338,20 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
         iter++;
         if (iter >= ctl.fgmres_maxit) break;
         // PrepareRestart: x += Z y; w = V g' (gmres.F90:333-379)
-        k_trisolve<<<1, kTriThreads, 0, st>>>(L, nullptr); g2_count_launches(1);
-        k_lincomb<double2, CI><<<g, kVT, 0, st>>>(k->x, 1.0, k->x, Z, N, L.y, L.flags + F_L, N, nullptr); g2_count_launches(1);
-        k_restart_g<<<1, 1, 0, st>>>(L); g2_count_launches(1);
-        k_copy_g<<<1, 64, 0, st>>>(L); g2_count_launches(1);
-        k_lincomb<double2, double2><<<g, kVT, 0, st>>>(k->w, 0.0, (const double2 *)nullptr, k->Vo, N, L.y,
+        g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, nullptr); g2_count_launches(1);
+        g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, Z, N, L.y, L.flags + F_L, N, nullptr); g2_count_launches(1);
+        g2_launch(k_restart_g, 1, 1, 0, st, L); g2_count_launches(1);
+        g2_launch(k_copy_g, 1, 64, 0, st, L); g2_count_launches(1);
+        g2_launch(k_lincomb<double2, double2>, g, kVT, 0, st, k->w, 0.0, (const double2 *)nullptr, k->Vo, N, L.y,
                                                        L.flags + F_L, N, nullptr);
     }
     (void)L_used;
     // FinalActions (gmres.F90:382-421)
-    k_trisolve<<<1, kTriThreads, 0, st>>>(L, nullptr); g2_count_launches(1);
-    k_lincomb<double2, CI><<<g, kVT, 0, st>>>(k->x, 1.0, k->x, Z, N, L.y, L.flags + F_L, N, nullptr); g2_count_launches(1);
+    g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, nullptr); g2_count_launches(1);
+    g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, Z, N, L.y, L.flags + F_L, N, nullptr); g2_count_launches(1);
     if ((rc = ie_apply_device64(op, k->x, k->r0, st))) return rc;
     k->applies64++;
-    k_axpby<double2, double2, double2><<<g, kVT, 0, st>>>(k->r0, 1.0, k->b, -1.0, k->r0, N, nullptr); g2_count_launches(1);
+    g2_launch(k_axpby<double2, double2, double2>, g, kVT, 0, st, k->r0, 1.0, k->b, -1.0, k->r0, N, nullptr); g2_count_launches(1);
     norm2<double2>(k, k->r0, L.scal + S_NRM2, nullptr, st);
     if ((rc = pull())) return rc;
     const double be = std::sqrt(h_scal[S_NRM2]) / bn;
@@ -1363,9 +1383,9 @@ int krylov_solve_device(IeOp *op, const double2 *d_Ebkg, double2 *d_Esol, const 
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
     // SolveEquation (ie_solver_module.F90:62-80): rhs = sqrt(Re sb) E_bkg; guess = E0/a or rhs
-    k_rhs<<<g, 256, 0, st>>>(k->b, d_Ebkg, op->d_post64, (size_t)op->Nx * op->Ny, op->Nz); g2_count_launches(1);
+    g2_launch(k_rhs, g, 256, 0, st, k->b, d_Ebkg, op->d_post64, (size_t)op->Nx * op->Ny, op->Nz); g2_count_launches(1);
     if (d_E0) {
-        k_scale_asig<<<g, 256, 0, st>>>(k->x, d_E0, op->d_asig64, cells, true);
+        g2_launch(k_scale_asig, g, 256, 0, st, k->x, d_E0, op->d_asig64, cells, true);
         g2_count_launches(1);
     } else {
         cudaMemcpyAsync(k->x, k->b, sizeof(double2) * k->N, cudaMemcpyDeviceToDevice, st);
@@ -1374,7 +1394,7 @@ int krylov_solve_device(IeOp *op, const double2 *d_Ebkg, double2 *d_Esol, const 
     else rc = outer_solve<float2>(op, k, ctl, info, st);
     if (rc) return rc;
     // Esol = a * chi (ie_solver_module.F90:85-97)
-    k_scale_asig<<<g, 256, 0, st>>>(d_Esol, k->x, op->d_asig64, cells, false); g2_count_launches(1);
+    g2_launch(k_scale_asig, g, 256, 0, st, d_Esol, k->x, op->d_asig64, cells, false); g2_count_launches(1);
     cudaEventRecord(e1, st);
     G2_CUDA_CHECK(cudaStreamSynchronize(st));
     float ms = 0;
@@ -1415,6 +1435,7 @@ namespace {
 // launch nothing: each mask has its own captured cycle.)
 __global__ void k_set_bn_masked(Level L, const int *outer_go)
 {
+    pdl_wait();
     L.scal[S_BN] = sqrt(L.scal[S_NRM2]);
     L.flags[F_SOLVER] = (L.scal[S_BN] < ZERO_THRESHOLD || *outer_go == 0) ? 0 : 1;
     L.flags[F_ITER] = 0;
@@ -1562,10 +1583,10 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
         KrylovWork *k = b->k[i];
         Level &L = k->Li;
         const int g = vec_grid(k->N);
-        k_zero_level<<<1, 256, 0, st>>>(L); g2_count_launches(1);
+        g2_launch(k_zero_level, 1, 256, 0, st, L); g2_count_launches(1);
         norm2<CI>(k, reinterpret_cast<const CI *>(k->vin), L.scal + S_NRM2, nullptr, st);
-        k_set_bn_masked<<<1, 1, 0, st>>>(L, k->Lo.flags + F_KRYLOV); g2_count_launches(1);
-        k_copy_or_zero<CI><<<g, kVT, 0, st>>>(reinterpret_cast<CI *>(k->xin), reinterpret_cast<const CI *>(k->vin),
+        g2_launch(k_set_bn_masked, 1, 1, 0, st, L, k->Lo.flags + F_KRYLOV); g2_count_launches(1);
+        g2_launch(k_copy_or_zero<CI>, g, kVT, 0, st, reinterpret_cast<CI *>(k->xin), reinterpret_cast<const CI *>(k->vin),
                                              L.scal, k->N); g2_count_launches(1);
     }
     auto vin = [&](int i) { return reinterpret_cast<const CI *>(b->k[i]->vin); };
@@ -1579,11 +1600,11 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
         const int g = vec_grid(k->N);
         const int *solver = L.flags + F_SOLVER;
         CI *r = reinterpret_cast<CI *>(k->ri);
-        k_axpby<CI, CI, CI><<<g, kVT, 0, st>>>(r, 1.0, reinterpret_cast<const CI *>(k->vin), -1.0, r, k->N, solver); g2_count_launches(1);
+        g2_launch(k_axpby<CI, CI, CI>, g, kVT, 0, st, r, 1.0, reinterpret_cast<const CI *>(k->vin), -1.0, r, k->N, solver); g2_count_launches(1);
         norm2<CI>(k, r, L.scal + S_NRM2, solver, st);
-        k_set_beta<<<1, 1, 0, st>>>(L, tol); g2_count_launches(1);
-        k_cycle_start<<<1, 1, 0, st>>>(L, solver); g2_count_launches(1);
-        k_scale_by<CI><<<g, kVT, 0, st>>>(reinterpret_cast<CI *>(k->Vi), r, L.scal, S_BETA, k->N, solver); g2_count_launches(1);
+        g2_launch(k_set_beta, 1, 1, 0, st, L, tol); g2_count_launches(1);
+        g2_launch(k_cycle_start, 1, 1, 0, st, L, solver); g2_count_launches(1);
+        g2_launch(k_scale_by<CI>, g, kVT, 0, st, reinterpret_cast<CI *>(k->Vi), r, L.scal, S_BETA, k->N, solver); g2_count_launches(1);
     }
     // Arnoldi step j of the active instances in `act`: runs of up to KMI instances with the same vector length
     // share each launch (each instance keeps its own blocks, partials and gates)
@@ -1637,8 +1658,8 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
         const int g = vec_grid(k->N);
         const int *solver = L.flags + F_SOLVER;
         CI *x = reinterpret_cast<CI *>(k->xin);
-        k_trisolve<<<1, kTriThreads, 0, st>>>(L, solver); g2_count_launches(1);
-        k_lincomb<CI, CI><<<g, kVT, 0, st>>>(x, 1.0, x, reinterpret_cast<const CI *>(k->Vi), k->N, L.y, L.flags + F_L,
+        g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, solver); g2_count_launches(1);
+        g2_launch(k_lincomb<CI, CI>, g, kVT, 0, st, x, 1.0, x, reinterpret_cast<const CI *>(k->Vi), k->N, L.y, L.flags + F_L,
                                              k->N, solver); g2_count_launches(1);
     }
     return G2_OK;
@@ -1786,11 +1807,11 @@ static void batch_final_launch(BatchWork *b, int i, cudaStream_t st, int &rc)
     Level &L = k->Lo;
     const int g = vec_grid(k->N);
     CI *Z = reinterpret_cast<CI *>(k->Zo);
-    k_trisolve<<<1, kTriThreads, 0, st>>>(L, nullptr); g2_count_launches(1);
-    k_lincomb<double2, CI><<<g, kVT, 0, st>>>(k->x, 1.0, k->x, Z, k->N, L.y, L.flags + F_L, k->N, nullptr); g2_count_launches(1);
+    g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, nullptr); g2_count_launches(1);
+    g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, Z, k->N, L.y, L.flags + F_L, k->N, nullptr); g2_count_launches(1);
     if ((rc = ie_apply_device64(b->ops[i], k->x, k->r0, st))) return;
     k->applies64++;
-    k_axpby<double2, double2, double2><<<g, kVT, 0, st>>>(k->r0, 1.0, k->b, -1.0, k->r0, k->N, nullptr); g2_count_launches(1);
+    g2_launch(k_axpby<double2, double2, double2>, g, kVT, 0, st, k->r0, 1.0, k->b, -1.0, k->r0, k->N, nullptr); g2_count_launches(1);
     norm2<double2>(k, k->r0, L.scal + S_NRM2, nullptr, st);
 }
 
@@ -1818,14 +1839,14 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
         KrylovWork *k = b->k[i];
         const int g = vec_grid(k->N);
         const int *solver = k->Lo.flags + F_SOLVER;
-        k_zero_level<<<1, 256, 0, st>>>(k->Lo); g2_count_launches(1);
+        g2_launch(k_zero_level, 1, 256, 0, st, k->Lo); g2_count_launches(1);
         norm2<double2>(k, k->b, k->Lo.scal + S_NRM2, nullptr, st);
-        k_set_bn<<<1, 1, 0, st>>>(k->Lo); g2_count_launches(1);
+        g2_launch(k_set_bn, 1, 1, 0, st, k->Lo); g2_count_launches(1);
         if ((rc = ie_apply_device64(b->ops[i], k->x, k->r0, st, solver))) return rc;
-        k_axpby<double2, double2, double2><<<g, kVT, 0, st>>>(k->r0, 1.0, k->b, -1.0, k->r0, k->N, solver); g2_count_launches(1);
-        k_axpby<double2, double2, double2><<<g, kVT, 0, st>>>(k->w, 1.0, k->r0, 0.0, (const double2 *)nullptr, k->N, solver); g2_count_launches(1);
+        g2_launch(k_axpby<double2, double2, double2>, g, kVT, 0, st, k->r0, 1.0, k->b, -1.0, k->r0, k->N, solver); g2_count_launches(1);
+        g2_launch(k_axpby<double2, double2, double2>, g, kVT, 0, st, k->w, 1.0, k->r0, 0.0, (const double2 *)nullptr, k->N, solver); g2_count_launches(1);
         norm2<double2>(k, k->w, k->Lo.scal + S_NRM2, solver, st);
-        k_set_beta<<<1, 1, 0, st>>>(k->Lo, tol); g2_count_launches(1);
+        g2_launch(k_set_beta, 1, 1, 0, st, k->Lo, tol); g2_count_launches(1);
     }
     if ((rc = batch_pull(b, h, st))) return rc;
     for (int i = 0; i < n; i++) {
@@ -1856,8 +1877,8 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
         for (int i = 0; i < n; i++) {
             if (!b->h_active[i]) continue;
             KrylovWork *k = b->k[i];
-            k_cycle_start<<<1, 1, 0, st>>>(k->Lo, nullptr); g2_count_launches(1);
-            k_scale_by<double2><<<vec_grid(k->N), kVT, 0, st>>>(k->Vo, k->w, k->Lo.scal, S_BETA, k->N, nullptr); g2_count_launches(1);
+            g2_launch(k_cycle_start, 1, 1, 0, st, k->Lo, nullptr); g2_count_launches(1);
+            g2_launch(k_scale_by<double2>, vec_grid(k->N), kVT, 0, st, k->Vo, k->w, k->Lo.scal, S_BETA, k->N, nullptr); g2_count_launches(1);
         }
         bool cycle_done = false;
         // Outer step j of every active instance.  Its kernels are gated by the instance's outer Krylov flag,
@@ -1870,7 +1891,7 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                 if (!b->h_active[i]) continue;
                 KrylovWork *k = b->k[i];
                 const int *go = k->Lo.flags + F_KRYLOV;
-                k_axpby<CI, double2, double2><<<vec_grid(k->N), kVT, 0, st>>>(
+                g2_launch(k_axpby<CI, double2, double2>, vec_grid(k->N), kVT, 0, st, 
                     reinterpret_cast<CI *>(k->vin), 1.0, k->Vo + (size_t)j * k->N, 0.0, (const double2 *)nullptr, k->N,
                     go); g2_count_launches(1);
             }
@@ -1887,11 +1908,11 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                     const int g = vec_grid(k->N);
                     const int *go = k->Lo.flags + F_KRYLOV;
                     CI *Zj = reinterpret_cast<CI *>(k->Zo) + (size_t)j * k->N;
-                    k_axpby<CI, CI, CI><<<g, kVT, 0, st>>>(Zj, 1.0, reinterpret_cast<const CI *>(k->xin), 0.0, (const CI *)nullptr, k->N, go); g2_count_launches(1);
+                    g2_launch(k_axpby<CI, CI, CI>, g, kVT, 0, st, Zj, 1.0, reinterpret_cast<const CI *>(k->xin), 0.0, (const CI *)nullptr, k->N, go); g2_count_launches(1);
                     if (sizeof(CI) == sizeof(double2)) {
                         if ((r = ie_apply_device64(b->ops[i], reinterpret_cast<const double2 *>(Zj), k->w, st, go))) return r;
                     } else {
-                        k_axpby<double2, CI, CI><<<g, kVT, 0, st>>>(k->tmp, 1.0, Zj, 0.0, (const CI *)nullptr, k->N, go); g2_count_launches(1);
+                        g2_launch(k_axpby<double2, CI, CI>, g, kVT, 0, st, k->tmp, 1.0, Zj, 0.0, (const CI *)nullptr, k->N, go); g2_count_launches(1);
                         if ((r = ie_apply_device64(b->ops[i], k->tmp, k->w, st, go))) return r;
                     }
                 }
@@ -1978,12 +1999,12 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                 b->h_active[i] = 0;
                 continue;
             }
-            k_trisolve<<<1, kTriThreads, 0, st>>>(k->Lo, nullptr); g2_count_launches(1);
-            k_lincomb<double2, CI><<<g, kVT, 0, st>>>(k->x, 1.0, k->x, reinterpret_cast<const CI *>(k->Zo), k->N,
+            g2_launch(k_trisolve, 1, kTriThreads, 0, st, k->Lo, nullptr); g2_count_launches(1);
+            g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, reinterpret_cast<const CI *>(k->Zo), k->N,
                                                       k->Lo.y, k->Lo.flags + F_L, k->N, nullptr); g2_count_launches(1);
-            k_restart_g<<<1, 1, 0, st>>>(k->Lo); g2_count_launches(1);
-            k_copy_g<<<1, 64, 0, st>>>(k->Lo); g2_count_launches(1);
-            k_lincomb<double2, double2><<<g, kVT, 0, st>>>(k->w, 0.0, (const double2 *)nullptr, k->Vo, k->N, k->Lo.y,
+            g2_launch(k_restart_g, 1, 1, 0, st, k->Lo); g2_count_launches(1);
+            g2_launch(k_copy_g, 1, 64, 0, st, k->Lo); g2_count_launches(1);
+            g2_launch(k_lincomb<double2, double2>, g, kVT, 0, st, k->w, 0.0, (const double2 *)nullptr, k->Vo, k->N, k->Lo.y,
                                                            k->Lo.flags + F_L, k->N, nullptr); g2_count_launches(1);
         }
         // instances that stopped in this cycle: final actions now (their own kernels only)
@@ -2036,9 +2057,9 @@ int batch_solve_device(void *h, const double2 *const *d_Ebkg, double2 *const *d_
         k->applies32 = k->applies64 = 0;
         const int g = vec_grid(k->N);
         // SolveEquation (ie_solver_module.F90:62-80): rhs = sqrt(Re sb) E_bkg; guess = E0/a or rhs
-        k_rhs<<<g, 256, 0, st>>>(k->b, d_Ebkg[i], op->d_post64, (size_t)op->Nx * op->Ny, op->Nz); g2_count_launches(1);
+        g2_launch(k_rhs, g, 256, 0, st, k->b, d_Ebkg[i], op->d_post64, (size_t)op->Nx * op->Ny, op->Nz); g2_count_launches(1);
         if (d_E0 && d_E0[i]) {
-            k_scale_asig<<<g, 256, 0, st>>>(k->x, d_E0[i], op->d_asig64, op->cells(), true); g2_count_launches(1);
+            g2_launch(k_scale_asig, g, 256, 0, st, k->x, d_E0[i], op->d_asig64, op->cells(), true); g2_count_launches(1);
         } else {
             G2_CUDA_CHECK(cudaMemcpyAsync(k->x, k->b, sizeof(double2) * k->N, cudaMemcpyDeviceToDevice, st));
         }
@@ -2048,7 +2069,7 @@ int batch_solve_device(void *h, const double2 *const *d_Ebkg, double2 *const *d_
     for (int i = 0; i < b->n; i++) {
         IeOp *op = b->ops[i];
         KrylovWork *k = b->k[i];
-        k_scale_asig<<<vec_grid(k->N), 256, 0, st>>>(d_Esol[i], k->x, op->d_asig64, op->cells(), false); g2_count_launches(1);
+        g2_launch(k_scale_asig, vec_grid(k->N), 256, 0, st, d_Esol[i], k->x, op->d_asig64, op->cells(), false); g2_count_launches(1);
     }
     cudaEventRecord(e1, st);
     G2_CUDA_CHECK(cudaStreamSynchronize(st));
