@@ -355,9 +355,14 @@ bool ie_uses_mma(const IeOp *op, int form)
 static size_t spectrum_elems(const IeOp *op) { return (size_t)op->Nx * op->Ny * 4 * ie_spectrum_pitch(op->Nz); }
 static size_t ystate_elems(const IeOp *op) { return (ie_ypipe_state_bytes(op->Nx) + 7) / 8; }
 
-// lines per CTA: tile of at most ~100 KB of shared memory, power of two, <= 32
+// Lines per CTA: tile of at most ~100 KB of shared memory, power of two, <= 32.  cap 0 is the default rule: 16
+// complex64 lines and 8 complex128 lines fit the register-capped kernels (PassLB) at every length they take.  Whole
+// applies with 32 / 16 / 8 / 4 lines: 128x128x32 complex128 390 / 391 / 348 / 358 us, paired complex64 313 / 299 / 301 /
+// 340; 64x128x27 178 / 180 / 158 / 162 and 161 / 155 / 157 / 173; 32x32x27 50 / 49 / 48 / 49 and 47 / 45 / 45 / 46.  Longer
+// lines take what the tile allows (256x256x48 complex64 1754 / 1754 / 1855 / 1864 us).
 static int lines_for(int L, size_t es, int cap)
 {
+    if (cap == 0 && L <= 256) cap = es == sizeof(double2) ? 8 : 16;
     int n = cap >= 1 && cap <= 32 ? cap : 32;
     while (n > 1 && (size_t)(n * (L + 1) + L) * es > 100 * 1024) n >>= 1;
     return n;

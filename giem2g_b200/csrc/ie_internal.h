@@ -71,7 +71,7 @@ struct IeOp {
     // (k_fy, contraction, k_by).  The separate passes are the default (faster at 128x128x32 on a B200);
     // the fused pass is a tile-shape variant the autotuner may pick where ie_ypipe_supported holds.
     int ypipe_mode[3] = {-1, -1, -1};
-    int fft_lines[2] = {32, 32};          // lines per CTA of the FFT passes, complex128 / complex64 (autotuned)
+    int fft_lines[2] = {0, 0};            // lines per CTA of the FFT passes, complex128 / complex64; 0: by rule
     long long config_gen = 0;             // bumped on every launch-shape change; captured graphs compare it
     // outer right-preconditioner hook (learned preconditioner): 0 off, 1 warm-starts the inner GMRES,
     // 2 replaces it
