@@ -1,0 +1,295 @@
+// One Arnoldi step of up to KMI lockstep instances in one cooperative launch: the dots of the first Gram-Schmidt pass, the
+// correction passes, V_{j+1} = w / ||w|| and the Givens update (gmres.F90:263-326), with a grid barrier per pass.
+//
+// As a launch per sweep (dots, four passes of which usually one or two do anything, scaling) a step of a small grid took
+// about 25 us, nearly all of it ramps, tails and last-block reductions.  Here every block keeps its part of the vectors
+// for the whole step, reduces all partial sums of a pass itself (a fixed order, so the result does not depend on the
+// schedule) and takes the pass decision with the others.  blockIdx.y is the instance; the barrier joins the blocks of one
+// instance.  The launch is cooperative, so all blocks are resident; the waits are bounded (2 s, error code 51).
+// Whole solves, launches per sweep -> one launch: FP64 32x32x8 3.00 -> 2.66 ms, mixed pairs 64x64x16 9.75 -> 8.80 ms,
+// 128x128x32 75.3 -> 74.3 ms (bound by the sweeps' HBM and L2 traffic).
+#include <type_traits>
+#include "krylov_dev.cuh"
+
+namespace {
+
+// all blocks of an instance; bar[0] arrivals, bar[1] generation
+G2_D bool grid_barrier(unsigned *bar, unsigned n, int *err)
+{
+    __shared__ bool ok;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ok = true;
+        const unsigned gen = atomicAdd(bar + 1, 0u);  // cannot advance before this block arrives
+        __threadfence();
+        if (atomicAdd(bar, 1u) == n - 1) {
+            atomicExch(bar, 0u);
+            __threadfence();
+            atomicAdd(bar + 1, 1u);
+        } else {
+            volatile const unsigned *g = bar + 1;
+            unsigned long long t0 = 0, t1;
+            for (int spin = 0; *g == gen; spin++) {
+                if ((spin & 255) != 255) continue;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+                if (t0 == 0) t0 = t1;
+                if (t1 - t0 > 2000000000ull) {
+                    atomicCAS(err, 0, 51);
+                    ok = false;
+                    break;
+                }
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok;
+}
+
+template <typename C, int K>
+__global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double tol, int *err)
+{
+    pdl_wait();
+    const int y = blockIdx.y;
+    if (mm.gate[y] && *mm.gate[y] == 0) return;
+    using R = typename RealOf<C>::T;
+    using W = typename Wide<C>::T;
+    constexpr int E = Wide<C>::E, j = K - 1;
+    __shared__ double2 hs[KMAX + 1], hn[KMAX + 1], hsum[KMAX + 1];
+    __shared__ double nrm;
+    Level L = mm.L[y];
+    C *V = mm.V[y], *w = mm.w[y];
+    const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x;
+    const size_t Nw = wide_words<C>(N, N), ldw = N / E;
+    const W *Vw = reinterpret_cast<const W *>(V);
+    W *ww = reinterpret_cast<W *>(w);
+    const size_t set = (size_t)gridDim.x * (KMAX + 1);
+    R ax[K + 1], ay[K + 1];
+    auto clear = [&] {
+#pragma unroll
+        for (int k = 0; k <= K; k++) ax[k] = ay[k] = R(0);
+    };
+    auto dots = [&](const C &a, const C *b) {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            ax[k] += b[k].x * a.x + b[k].y * a.y;
+            ay[k] += b[k].x * a.y - b[k].y * a.x;
+        }
+    };
+    auto dots_of = [&](const C &a, size_t i) {  // the basis values of element i from memory
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const C b = V[(size_t)k * N + i];
+            ax[k] += b.x * a.x + b.y * a.y;
+            ay[k] += b.x * a.y - b.y * a.x;
+        }
+    };
+    // U words per thread and round, every load of the round first; HOLD: the K basis values fit the registers
+    constexpr bool HOLD = SweepU<K, W>::v > 0;
+    constexpr int U = HOLD ? SweepU<K, W>::v : 1, KH = HOLD ? K : 1;
+    clear();
+    size_t i = t0;
+    if constexpr (HOLD) {
+        auto round = [&](auto nu) {
+            constexpr int NU = decltype(nu)::value;
+            W wv[NU], v[KH][NU];
+#pragma unroll
+            for (int u = 0; u < NU; u++) wv[u] = ww[i + u * S];
+#pragma unroll
+            for (int k = 0; k < KH; k++)
+#pragma unroll
+                for (int u = 0; u < NU; u++) v[k][u] = Vw[(size_t)k * ldw + i + u * S];
+#pragma unroll
+            for (int u = 0; u < NU; u++)
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    C b[KH];
+#pragma unroll
+                    for (int k = 0; k < KH; k++) b[k] = part_of(v[k][u], e);
+                    dots(part_of(wv[u], e), b);
+                }
+        };
+        for (; i + (U - 1) * S < Nw; i += U * S) round(std::integral_constant<int, U>());
+        for (; i < Nw; i += S) round(std::integral_constant<int, 1>());
+    }
+    for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) dots_of(w[i], i);
+    block_reduce_store_r<K, R>(ax, ay, mm.part[y]);
+    if (!grid_barrier(L.counter + 1, gridDim.x, err)) return;
+    reduce_partials(mm.part[y], gridDim.x, K, hs, nullptr);
+    if (threadIdx.x < K) hsum[threadIdx.x] = hs[threadIdx.x];
+    __syncthreads();
+    double dloo;
+    for (int p = 1;; p++) {
+        // w -= V hs; dots and norm of the new w
+        clear();
+        auto take = [&](C &a, const C &b, int k) {
+            const R hx = (R)hs[k].x, hy = (R)hs[k].y;
+            a.x -= b.x * hx - b.y * hy;
+            a.y -= b.x * hy + b.y * hx;
+        };
+        i = t0;
+        if constexpr (HOLD) {
+            auto round = [&](auto nu) {
+                constexpr int NU = decltype(nu)::value;
+                W wv[NU], v[KH][NU];
+#pragma unroll
+                for (int u = 0; u < NU; u++) wv[u] = ww[i + u * S];
+#pragma unroll
+                for (int k = 0; k < KH; k++)
+#pragma unroll
+                    for (int u = 0; u < NU; u++) v[k][u] = Vw[(size_t)k * ldw + i + u * S];
+#pragma unroll
+                for (int u = 0; u < NU; u++) {
+#pragma unroll
+                    for (int e = 0; e < E; e++) {
+                        C a = part_of(wv[u], e), b[KH];
+#pragma unroll
+                        for (int k = 0; k < KH; k++) {
+                            b[k] = part_of(v[k][u], e);
+                            take(a, b[k], k);
+                        }
+                        ax[K] += a.x * a.x + a.y * a.y;
+                        dots(a, b);
+                        set_part(wv[u], e, a);
+                    }
+                    ww[i + u * S] = wv[u];
+                }
+            };
+            for (; i + (U - 1) * S < Nw; i += U * S) round(std::integral_constant<int, U>());
+            for (; i < Nw; i += S) round(std::integral_constant<int, 1>());
+        }
+        for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) {
+            C a = w[i];
+#pragma unroll
+            for (int k = 0; k < K; k++) take(a, V[(size_t)k * N + i], k);
+            w[i] = a;
+            ax[K] += a.x * a.x + a.y * a.y;
+            dots_of(a, i);
+        }
+        double2 *part = mm.part[y] + (p & 1) * set;  // the other set may still be read by a slower block
+        block_reduce_store_r<K, R>(ax, ay, part);
+        if (!grid_barrier(L.counter + 1, gridDim.x, err)) return;
+        reduce_partials(part, gridDim.x, K, hn, &nrm);
+        // gmres.F90:277-280
+        double dl = 0.0;
+        for (int k = 0; k < K; k++) dl += hs[k].x * hs[k].x + hs[k].y * hs[k].y;
+        dloo = sqrt(dl);
+        if (2.0 * sqrt(nrm) > dloo || p > N_IGS) break;
+        __syncthreads();
+        if (threadIdx.x < K) {
+            hsum[threadIdx.x].x += hn[threadIdx.x].x;
+            hsum[threadIdx.x].y += hn[threadIdx.x].y;
+            hs[threadIdx.x] = hn[threadIdx.x];
+        }
+        __syncthreads();
+    }
+    const double dnormw = sqrt(nrm), inv = 1.0 / dnormw;
+    // in the scaling every thread takes the words that it wrote
+    for (i = t0; HOLD && i < Nw; i += S) {
+        W x = ww[i];
+#pragma unroll
+        for (int e = 0; e < E; e++) set_part(x, e, scaled(part_of(x, e), inv));
+        reinterpret_cast<W *>(V)[(size_t)K * ldw + i] = x;
+    }
+    for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) V[(size_t)K * N + i] = scaled(w[i], inv);
+    if (blockIdx.x != 0) return;
+    // every block has read its gate, a flag that the step below may clear: all of them passed the barriers above
+    if (threadIdx.x < K) L.H[hix(threadIdx.x, j, L.m)] = hsum[threadIdx.x];
+    if (threadIdx.x == 0) {
+        L.scal[S_NRM2] = nrm;
+        L.scal[S_DLOO] = dloo;
+        L.scal[S_DNORMW] = dnormw;
+        L.flags[F_PASS] = 0;
+    }
+    __threadfence_block();
+    __syncthreads();
+    arnoldi_finish_body(L, j, tol);
+}
+
+int sms()
+{
+    static const int n = [] {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v > 0 ? v : 1;
+    }();
+    return n;
+}
+
+template <typename C, int K>
+int launch(const Multi<C> &mm, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st)
+{
+    static const int per_sm = [] {
+        int b = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_arnoldi<C, K>, kVT, 0) == cudaSuccess && b > 0 ? b : 1;
+    }();
+    const size_t words = N / Wide<C>::E + 1, need = (words + kVT - 1) / kVT;
+    int g = per_sm * sms() / n;
+    g = g < nparts ? g : nparts;
+    g = (size_t)g < need ? g : (int)need;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(g < 1 ? 1 : g, n);
+    cfg.blockDim = dim3(kVT);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    G2_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_arnoldi<C, K>, mm, N, tol, err));
+    return G2_OK;
+}
+template <typename C>
+int dispatch(const Multi<C> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
+{
+    switch (j + 1) {
+#define G2_K(k) \
+    case k: return launch<C, k>(mm, n, N, nparts, tol, err, st)
+        G2_K(1);
+        G2_K(2);
+        G2_K(3);
+        G2_K(4);
+        G2_K(5);
+        G2_K(6);
+        G2_K(7);
+        G2_K(8);
+        G2_K(9);
+        G2_K(10);
+        G2_K(11);
+        G2_K(12);
+        G2_K(13);
+        G2_K(14);
+        G2_K(15);
+        G2_K(16);
+        G2_K(17);
+        G2_K(18);
+        G2_K(19);
+        G2_K(20);
+        G2_K(21);
+        G2_K(22);
+        G2_K(23);
+        G2_K(24);
+        G2_K(25);
+        G2_K(26);
+        G2_K(27);
+        G2_K(28);
+        G2_K(29);
+        G2_K(30);
+        G2_K(31);
+#undef G2_K
+    }
+    return G2_ERR_UNSUPPORTED;
+}
+
+}  // namespace
+
+int arnoldi_step(const Multi<float2> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
+{
+    return dispatch(mm, n, N, nparts, j, tol, err, st);
+}
+int arnoldi_step(const Multi<double2> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
+{
+    return dispatch(mm, n, N, nparts, j, tol, err, st);
+}

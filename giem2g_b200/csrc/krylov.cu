@@ -21,500 +21,9 @@
 #include <cstdlib>
 #include <vector>
 #include "common.cuh"
-#include "krylov.h"
+#include "krylov_dev.cuh"
 
 namespace {
-
-constexpr int kVT = 256;   // threads of the vector kernels
-constexpr int kILP = 4;    // elements per thread and iteration of the element-wise vector kernels
-constexpr int KMAX = 32;   // largest basis handled in one sweep
-constexpr double ZERO_THRESHOLD = 1e-14;  // gmres.F90:21
-constexpr int N_IGS = 3;                  // gmres.F90:22
-constexpr double kHookGain = 0.5;         // an outer step through the hook must halve the misfit
-
-enum { F_KRYLOV = 0, F_PASS = 1, F_L = 2, F_ITER = 3, F_SOLVER = 4, F_NFLAGS = 8 };
-enum { S_BN = 0, S_BETA = 1, S_DNORMW = 2, S_DLOO = 3, S_BEA = 4, S_NRM2 = 5, S_NSCAL = 8 };
-
-struct Level {
-    int m = 0;
-    double2 *H = nullptr;   // (m+1) x (m+1) column-major, column m holds g
-    double *cs = nullptr;
-    double2 *sn = nullptr;
-    double2 *hpass = nullptr, *hnext = nullptr, *y = nullptr;
-    double *scal = nullptr;
-    int *flags = nullptr;
-    unsigned *counter = nullptr;  // blocks done, for the last-block reductions (back to 0 after each use)
-};
-
-G2_HD int hix(int i, int j, int m) { return i + j * (m + 1); }
-
-template <typename C> G2_D double2 ld2(const C *p, size_t i);
-template <> G2_D double2 ld2<double2>(const double2 *p, size_t i) { return p[i]; }
-template <> G2_D double2 ld2<float2>(const float2 *p, size_t i)
-{
-    const float2 v = p[i];
-    return make_double2(v.x, v.y);
-}
-template <typename C> G2_D void st2(C *p, size_t i, double2 v);
-template <> G2_D void st2<double2>(double2 *p, size_t i, double2 v) { p[i] = v; }
-template <> G2_D void st2<float2>(float2 *p, size_t i, double2 v) { p[i] = make_float2((float)v.x, (float)v.y); }
-
-// The basis sweeps move 16-byte words: two complex64 values per load (complex128 values are 16 bytes
-// already).  On a B200 a two-instance sweep of 11 complex64 vectors of 1.57 M elements took 84 us with
-// 8-byte loads and 52 us with 16-byte loads.  Vectors whose length (and column stride) is odd keep
-// element-wise loads, since their odd columns are not 16-byte aligned.
-template <typename C> struct Wide;
-template <> struct Wide<float2> {
-    using T = float4;
-    static constexpr int E = 2;
-};
-template <> struct Wide<double2> {
-    using T = double2;
-    static constexpr int E = 1;
-};
-G2_D float2 part_of(const float4 &p, int e) { return e ? make_float2(p.z, p.w) : make_float2(p.x, p.y); }
-G2_D double2 part_of(const double2 &p, int) { return p; }
-G2_D void set_part(float4 &p, int e, float2 v)
-{
-    if (e) {
-        p.z = v.x;
-        p.w = v.y;
-    } else {
-        p.x = v.x;
-        p.y = v.y;
-    }
-}
-G2_D void set_part(double2 &p, int, double2 v) { p = v; }
-// words of E elements over the whole vector, or 0 when the lengths do not allow them
-template <typename C> G2_D size_t wide_words(size_t N, size_t ld)
-{
-    constexpr int E = Wide<C>::E;
-    return (N % E == 0 && ld % E == 0) ? N / E : 0;
-}
-
-template <typename C> struct RealOf;
-template <> struct RealOf<double2> { using T = double; };
-template <> struct RealOf<float2> { using T = float; };
-
-// per-thread partial sums in the vector's precision (a handful of elements each), block and grid
-// reductions in FP64
-template <int KM, typename R>
-G2_D void block_reduce_store_r(R (&ax)[KM + 1], R (&ay)[KM + 1], double2 *part)
-{
-    __shared__ double2 red[kVT / 32][KM + 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k <= KM; k++) {
-        double vx = ax[k], vy = ay[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            vx += __shfl_xor_sync(0xffffffffu, vx, o);
-            vy += __shfl_xor_sync(0xffffffffu, vy, o);
-        }
-        if (lane == 0) red[warp][k] = make_double2(vx, vy);
-    }
-    __syncthreads();
-    if (threadIdx.x <= KM) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int w = 0; w < kVT / 32; w++) {
-            s.x += red[w][threadIdx.x].x;
-            s.y += red[w][threadIdx.x].y;
-        }
-        part[(size_t)blockIdx.x * (KMAX + 1) + (threadIdx.x == KM ? KMAX : threadIdx.x)] = s;
-    }
-}
-
-// ---- scalar control kernels (one thread) -------------------------------------------------------
-// first CGS pass of step j: H(0..j, j) = h, hpass = h, pass active
-G2_D void cgs_first_body(Level &L, int j, const double2 *h)
-{
-    for (int i = 0; i <= j; i++) {
-        L.H[hix(i, j, L.m)] = h[i];
-        L.hpass[i] = h[i];
-    }
-    L.flags[F_PASS] = 1;
-}
-// after pass p (1-based) subtracted hpass: decide on another pass (gmres.F90:277-280)
-G2_D void cgs_next_body(Level &L, int j, int p)
-{
-    double dl = 0.0;
-    for (int i = 0; i <= j; i++) dl += L.hpass[i].x * L.hpass[i].x + L.hpass[i].y * L.hpass[i].y;
-    const double dloo = sqrt(dl), dnormw = sqrt(L.scal[S_NRM2]);
-    L.scal[S_DLOO] = dloo;
-    L.scal[S_DNORMW] = dnormw;
-    if (2.0 * dnormw > dloo || p > N_IGS) {
-        L.flags[F_PASS] = 0;
-    } else {
-        for (int i = 0; i <= j; i++) {
-            L.H[hix(i, j, L.m)].x += L.hnext[i].x;
-            L.H[hix(i, j, L.m)].y += L.hnext[i].y;
-            L.hpass[i] = L.hnext[i];
-        }
-    }
-}
-
-G2_D double cabs_(double2 a) { return hypot(a.x, a.y); }
-G2_D double2 cmul_(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
-G2_D double2 cdivr(double2 a, double r) { return make_double2(a.x / r, a.y / r); }
-// netlib ZROT on one pair
-G2_D void zrot1(double2 &cx, double2 &cy, double c, double2 s)
-{
-    const double2 t = make_double2(c * cx.x + (s.x * cy.x - s.y * cy.y), c * cx.y + (s.x * cy.y + s.y * cy.x));
-    const double2 sc = make_double2(s.x, -s.y);
-    cy = make_double2(c * cy.x - (sc.x * cx.x - sc.y * cx.y), c * cy.y - (sc.x * cx.y + sc.y * cx.x));
-    cx = t;
-}
-// netlib ZROTG
-G2_D void zrotg(double2 &ca, double2 cb, double &c, double2 &s)
-{
-    const double aca = cabs_(ca);
-    if (aca == 0.0) {
-        c = 0.0;
-        s = make_double2(1.0, 0.0);
-        ca = cb;
-    } else {
-        const double scale = aca + cabs_(cb);
-        const double a1 = cabs_(cdivr(ca, scale)), b1 = cabs_(cdivr(cb, scale));
-        const double norm = scale * sqrt(a1 * a1 + b1 * b1);
-        const double2 alpha = cdivr(ca, aca);
-        c = aca / norm;
-        s = cdivr(cmul_(alpha, make_double2(cb.x, -cb.y)), norm);
-        ca = make_double2(alpha.x * norm, alpha.y * norm);
-    }
-}
-
-// end of Arnoldi step j (gmres.F90:283-326): H(j+1,j), rotations, Arnoldi misfit, exit test
-G2_D void arnoldi_finish_body(Level &L, int j, double tol)
-{
-    // run by every thread of one block: column j of H, the rotations so far and g(j), g(j+1) are staged in
-    // shared memory with one round of loads; thread 0 then applies the same operations in the same order
-    // as a single thread on global memory would (a chain of dependent L2 loads otherwise)
-    __shared__ double2 hc[KMAX + 1], sn_s[KMAX], gs[2];
-    __shared__ double cs_s[KMAX];
-    const int m = L.m;
-    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) hc[i] = L.H[hix(i, j, m)];
-    for (int i = threadIdx.x; i < j; i += blockDim.x) {
-        cs_s[i] = L.cs[i];
-        sn_s[i] = L.sn[i];
-    }
-    if (threadIdx.x < 2) gs[threadIdx.x] = L.H[hix(j + threadIdx.x, m, m)];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double dnormw = L.scal[S_DNORMW], bn = L.scal[S_BN];
-        hc[j + 1] = make_double2(dnormw, 0.0);
-        for (int i = 0; i < j; i++) zrot1(hc[i], hc[i + 1], cs_s[i], sn_s[i]);
-        double2 h1 = hc[j], sn;
-        double c;
-        zrotg(h1, hc[j + 1], c, sn);
-        zrot1(gs[0], gs[1], c, sn);
-        zrot1(hc[j], hc[j + 1], c, sn);
-        hc[j + 1] = make_double2(0.0, 0.0);
-        L.cs[j] = c;
-        L.sn[j] = sn;
-        L.H[hix(j, m, m)] = gs[0];
-        L.H[hix(j + 1, m, m)] = gs[1];
-        const double bea = cabs_(gs[1]) / bn;
-        L.scal[S_BEA] = bea;
-        L.flags[F_ITER] += 1;
-        L.flags[F_L] = j + 1;
-        if (bea < tol || j + 1 >= m) L.flags[F_KRYLOV] = 0;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) L.H[hix(i, j, m)] = hc[i];
-}
-
-// ---- fused reductions: the last block to finish sums every block's partials ----------------------
-// Each block stores its partials, then counts itself done; the block that counts last reduces all
-// partials in a fixed order (lane-strided sums, shuffle tree: the result does not depend on which block
-// is last) and runs the scalar step that used to be a separate one-thread launch.  It resets the counter
-// for the next use.  Blocks test their gates before any of them can reach the last block, so a flag the
-// last block changes cannot be seen half-way through the grid.
-G2_D bool last_block(unsigned *counter)
-{
-    __shared__ bool am_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) am_last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (am_last && threadIdx.x == 0) *counter = 0u;
-    return am_last;
-}
-// sums of part[b][col] over blocks for columns 0..K-1 into h[], and of column KMAX into *nrm (one block)
-G2_D void reduce_partials(const double2 *part, int nb, int K, double2 *h, double *nrm)
-{
-    __threadfence();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = warp; k <= K; k += nw) {
-        const int col = (k == K) ? KMAX : k;
-        double sx = 0.0, sy = 0.0;
-        // eight independent loads per lane and round (rows past nb predicated off): the partials come from
-        // L2, and each round is one L2 round trip, so 256 rows cost one
-        for (int b0 = 0; b0 < nb; b0 += 256) {
-            double2 v[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const int b = b0 + lane + 32 * q;
-                v[q] = b < nb ? __ldcg(part + (size_t)b * (KMAX + 1) + col) : make_double2(0.0, 0.0);
-            }
-            sx += ((v[0].x + v[1].x) + (v[2].x + v[3].x)) + ((v[4].x + v[5].x) + (v[6].x + v[7].x));
-            sy += ((v[0].y + v[1].y) + (v[2].y + v[3].y)) + ((v[4].y + v[5].y) + (v[6].y + v[7].y));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sx += __shfl_xor_sync(0xffffffffu, sx, o);
-            sy += __shfl_xor_sync(0xffffffffu, sy, o);
-        }
-        if (lane == 0) {
-            if (k < K) h[k] = make_double2(sx, sy);
-            else if (nrm) *nrm = sx;
-        }
-    }
-    __syncthreads();
-}
-
-// first CGS pass of Arnoldi step j = K-1: h = V^H w, then H(0..j, j) = h, hpass = h
-// elements per thread and round of the basis sweeps: all (K + 1) * U loads of a round are issued before the
-// first product, so a round costs one memory round trip; the values held stay within 256 bytes per thread
-// (32 complex64 or 16 complex128).  0: the basis is too wide to hold, the sweep loads one element at a time.
-template <int K, typename C> struct SweepU {
-    static constexpr int B = (K + 1) * (int)sizeof(C);
-    static constexpr int v = B * 4 <= 256 ? 4 : (B * 2 <= 256 ? 2 : (B <= 256 ? 1 : 0));
-};
-
-template <typename C, int K>
-G2_D void dots_first_body(const C *__restrict__ V, size_t ld, const C *__restrict__ w, size_t N, double2 *part,
-                          Level &L)
-{
-    using R = typename RealOf<C>::T;
-    using W = typename Wide<C>::T;
-    constexpr int E = Wide<C>::E;
-    constexpr int U = SweepU<K, W>::v > 0 ? SweepU<K, W>::v : 1;
-    R ax[K + 1], ay[K + 1];
-#pragma unroll
-    for (int k = 0; k <= K; k++) ax[k] = ay[k] = R(0);
-    const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x;
-    const size_t Nw = wide_words<C>(N, ld), ldw = ld / E;
-    const W *__restrict__ Vw = reinterpret_cast<const W *>(V);
-    const W *__restrict__ ww = reinterpret_cast<const W *>(w);
-    size_t i = t0;
-    for (; SweepU<K, W>::v > 0 && i + (U - 1) * S < Nw; i += U * S) {
-        W wv[U], v[K > 0 ? K : 1][U];
-#pragma unroll
-        for (int u = 0; u < U; u++) wv[u] = ww[i + u * S];
-#pragma unroll
-        for (int k = 0; k < K; k++)
-#pragma unroll
-            for (int u = 0; u < U; u++) v[k][u] = Vw[(size_t)k * ldw + i + u * S];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                const C a = part_of(wv[u], e);
-#pragma unroll
-                for (int k = 0; k < K; k++) {
-                    const C b = part_of(v[k][u], e);
-                    ax[k] += b.x * a.x + b.y * a.y;
-                    ay[k] += b.x * a.y - b.y * a.x;
-                }
-            }
-    }
-    for (; i < Nw; i += S) {
-        const W wv = ww[i];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const W v = Vw[(size_t)k * ldw + i];
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                const C a = part_of(wv, e), b = part_of(v, e);
-                ax[k] += b.x * a.x + b.y * a.y;
-                ay[k] += b.x * a.y - b.y * a.x;
-            }
-        }
-    }
-    for (i = Nw * E + t0; i < N; i += S) {
-        const C wv = w[i];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const C v = V[(size_t)k * ld + i];
-            ax[k] += v.x * wv.x + v.y * wv.y;
-            ay[k] += v.x * wv.y - v.y * wv.x;
-        }
-    }
-    block_reduce_store_r<K, R>(ax, ay, part);
-    if (!last_block(L.counter)) return;
-    __shared__ double2 hs[KMAX + 1];
-    reduce_partials(part, gridDim.x, K, hs, nullptr);
-    if (threadIdx.x == 0) cgs_first_body(L, K - 1, hs);
-}
-template <typename C, int K>
-__global__ void __launch_bounds__(kVT) k_dots_first_t(const C *__restrict__ V, size_t ld, const C *__restrict__ w,
-                                                      size_t N, double2 *part, Level L, const int *gate)
-{
-    pdl_wait();
-    if (gate && *gate == 0) return;
-    dots_first_body<C, K>(V, ld, w, N, part, L);
-}
-
-// Several instances of one batch in one launch (blockIdx.y = instance): the same blocks, partials,
-// counters and last-block steps per instance as separate launches, so the results are the same; what
-// goes is the launch per instance and its ramp and tail.
-constexpr int KMI = 4;
-template <typename C>
-struct Multi {
-    C *V[KMI];
-    C *w[KMI];
-    double2 *part[KMI];
-    Level L[KMI];
-    const int *gate[KMI];
-};
-template <typename C, int K>
-__global__ void __launch_bounds__(kVT) k_dots_first_m(Multi<C> mm, size_t ld, size_t N)
-{
-    pdl_wait();
-    const int y = blockIdx.y;
-    if (mm.gate[y] && *mm.gate[y] == 0) return;
-    Level L = mm.L[y];
-    dots_first_body<C, K>(mm.V[y], ld, mm.w[y], N, mm.part[y], L);
-}
-
-// CGS pass p of step j = K-1: w -= V hpass; dots of the new w; then the pass decision (gmres.F90:277-280)
-template <typename C, int K>
-G2_D void cgs_pass_body(const C *__restrict__ V, size_t ld, C *__restrict__ w, size_t N, double2 *part, Level &L,
-                        int p)
-{
-    using R = typename RealOf<C>::T;
-    using W = typename Wide<C>::T;
-    constexpr int E = Wide<C>::E;
-    constexpr int KA = K > 0 ? K : 1;
-    __shared__ double2 hsh[KA];
-    if (threadIdx.x < K) hsh[threadIdx.x] = L.hpass[threadIdx.x];
-    __syncthreads();
-    R ax[K + 1], ay[K + 1];
-#pragma unroll
-    for (int k = 0; k <= K; k++) ax[k] = ay[k] = R(0);
-    constexpr int U = SweepU<K, W>::v > 0 ? SweepU<K, W>::v : 1;
-    const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x;
-    const size_t Nw = wide_words<C>(N, ld), ldw = ld / E;
-    const W *__restrict__ Vw = reinterpret_cast<const W *>(V);
-    W *__restrict__ ww = reinterpret_cast<W *>(w);
-    // one element: w -= V hpass, then |w|^2 and the dots of the new w (the basis values stay in registers)
-    auto element = [&](C &a, const C *b) {
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const R hx = (R)hsh[k].x, hy = (R)hsh[k].y;
-            a.x -= b[k].x * hx - b[k].y * hy;
-            a.y -= b[k].x * hy + b[k].y * hx;
-        }
-        ax[K] += a.x * a.x + a.y * a.y;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            ax[k] += b[k].x * a.x + b[k].y * a.y;
-            ay[k] += b[k].x * a.y - b[k].y * a.x;
-        }
-    };
-    size_t i = t0;
-    // U words per round, every load of the round first
-    for (; SweepU<K, W>::v > 0 && i + (U - 1) * S < Nw; i += U * S) {
-        W wv[U], v[K > 0 ? K : 1][U];
-#pragma unroll
-        for (int u = 0; u < U; u++) wv[u] = ww[i + u * S];
-#pragma unroll
-        for (int k = 0; k < K; k++)
-#pragma unroll
-            for (int u = 0; u < U; u++) v[k][u] = Vw[(size_t)k * ldw + i + u * S];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                C a = part_of(wv[u], e), b[K > 0 ? K : 1];
-#pragma unroll
-                for (int k = 0; k < K; k++) b[k] = part_of(v[k][u], e);
-                element(a, b);
-                set_part(wv[u], e, a);
-            }
-            ww[i + u * S] = wv[u];
-        }
-    }
-    // the rest (all of it when the basis is too wide to hold): one word at a time, the basis read twice
-    for (; i < Nw; i += S) {
-        W wv = ww[i];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const W v = Vw[(size_t)k * ldw + i];
-            const R hx = (R)hsh[k].x, hy = (R)hsh[k].y;
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                C a = part_of(wv, e);
-                const C b = part_of(v, e);
-                a.x -= b.x * hx - b.y * hy;
-                a.y -= b.x * hy + b.y * hx;
-                set_part(wv, e, a);
-            }
-        }
-        ww[i] = wv;
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const C a = part_of(wv, e);
-            ax[K] += a.x * a.x + a.y * a.y;
-        }
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const W v = Vw[(size_t)k * ldw + i];
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                const C a = part_of(wv, e), b = part_of(v, e);
-                ax[k] += b.x * a.x + b.y * a.y;
-                ay[k] += b.x * a.y - b.y * a.x;
-            }
-        }
-    }
-    for (i = Nw * E + t0; i < N; i += S) {
-        C wv = w[i];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const C v = V[(size_t)k * ld + i];
-            const R hx = (R)hsh[k].x, hy = (R)hsh[k].y;
-            wv.x -= v.x * hx - v.y * hy;
-            wv.y -= v.x * hy + v.y * hx;
-        }
-        w[i] = wv;
-        ax[K] += wv.x * wv.x + wv.y * wv.y;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const C v = V[(size_t)k * ld + i];
-            ax[k] += v.x * wv.x + v.y * wv.y;
-            ay[k] += v.x * wv.y - v.y * wv.x;
-        }
-    }
-    block_reduce_store_r<K, R>(ax, ay, part);
-    if (!last_block(L.counter)) return;
-    __shared__ double2 hs[KMAX + 1];
-    __shared__ double nrm;
-    reduce_partials(part, gridDim.x, K, hs, &nrm);
-    if (threadIdx.x < K) L.hnext[threadIdx.x] = hs[threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        L.scal[S_NRM2] = nrm;
-        cgs_next_body(L, K - 1, p);
-    }
-}
-template <typename C, int K>
-__global__ void __launch_bounds__(kVT) k_cgs_pass_fused_t(const C *__restrict__ V, size_t ld, C *__restrict__ w,
-                                                          size_t N, double2 *part, Level L, int p, const int *gate)
-{
-    pdl_wait();
-    if ((gate && *gate == 0) || L.flags[F_PASS] == 0) return;
-    cgs_pass_body<C, K>(V, ld, w, N, part, L, p);
-}
-template <typename C, int K>
-__global__ void __launch_bounds__(kVT) k_cgs_pass_fused_m(Multi<C> mm, size_t ld, size_t N, int p)
-{
-    pdl_wait();
-    const int y = blockIdx.y;
-    if ((mm.gate[y] && *mm.gate[y] == 0) || mm.L[y].flags[F_PASS] == 0) return;
-    Level L = mm.L[y];
-    cgs_pass_body<C, K>(mm.V[y], ld, mm.w[y], N, mm.part[y], L, p);
-}
 
 // ||w||^2 into *nrm2
 template <typename C>
@@ -562,63 +71,8 @@ __global__ void __launch_bounds__(kVT) k_norm2_fused(const C *__restrict__ w, si
     if (threadIdx.x == 0) *nrm2 = nrm;
 }
 
-// end of Arnoldi step j: V_{j+1} = w / ||w||, then the last block runs the Givens/misfit step
-G2_D float2 scaled(float2 a, double s) { return make_float2((float)(a.x * s), (float)(a.y * s)); }
-G2_D double2 scaled(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 G2_D double2 widen(float2 a) { return make_double2(a.x, a.y); }
 G2_D double2 widen(double2 a) { return a; }
-
-template <typename C>
-G2_D void scale_finish_body(C *v, const C *w, size_t N, Level &L, int j, double tol)
-{
-    using W = typename Wide<C>::T;
-    constexpr int E = Wide<C>::E;
-    const double inv = 1.0 / L.scal[S_DNORMW];
-    // kILP independent words per thread and iteration, loads first: more bytes in flight per SM
-    const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x;
-    const size_t Nw = wide_words<C>(N, N);
-    const W *__restrict__ ww = reinterpret_cast<const W *>(w);
-    W *__restrict__ vw = reinterpret_cast<W *>(v);
-    size_t i = t0;
-    for (; i + (kILP - 1) * S < Nw; i += kILP * S) {
-        W x[kILP];
-#pragma unroll
-        for (int u = 0; u < kILP; u++) x[u] = ww[i + u * S];
-#pragma unroll
-        for (int u = 0; u < kILP; u++) {
-#pragma unroll
-            for (int e = 0; e < E; e++) set_part(x[u], e, scaled(part_of(x[u], e), inv));
-            vw[i + u * S] = x[u];
-        }
-    }
-    for (; i < Nw; i += S) {
-        W x = ww[i];
-#pragma unroll
-        for (int e = 0; e < E; e++) set_part(x, e, scaled(part_of(x, e), inv));
-        vw[i] = x;
-    }
-    for (i = Nw * E + t0; i < N; i += S) v[i] = scaled(w[i], inv);
-    if (!last_block(L.counter)) return;
-    arnoldi_finish_body(L, j, tol);
-}
-template <typename C>
-__global__ void __launch_bounds__(kVT) k_scale_finish(C *v, const C *w, size_t N, Level L, int j, double tol,
-                                                      const int *gate)
-{
-    pdl_wait();
-    if (gate && *gate == 0) return;
-    scale_finish_body<C>(v, w, N, L, j, tol);
-}
-// Multi: V[y] is the instance's basis, column j+1 is written
-template <typename C>
-__global__ void __launch_bounds__(kVT) k_scale_finish_m(Multi<C> mm, size_t N, int j, double tol)
-{
-    pdl_wait();
-    const int y = blockIdx.y;
-    if (mm.gate[y] && *mm.gate[y] == 0) return;
-    Level L = mm.L[y];
-    scale_finish_body<C>(mm.V[y] + (size_t)(j + 1) * N, mm.w[y], N, L, j, tol);
-}
 
 // ConstructCurrentSolution's triangular solve (gmres.F90:441-445): y = H(0:L,0:L)^-1 g.  The block stages the
 // L x L triangle and g in shared memory with one coalesced load; thread 0 then substitutes in the same order
@@ -694,6 +148,7 @@ __global__ void k_zero_level(Level L)
     pdl_wait();
     const int n = (L.m + 1) * (L.m + 1);
     for (int i = threadIdx.x; i < n; i += blockDim.x) L.H[i] = make_double2(0.0, 0.0);
+    if (threadIdx.x == 0) L.counter[1] = 0u;  // a step that gave up at its barrier may have left arrivals
 }
 
 // restart (gmres.F90:369-376): beta = |g_m|, g <- inverse rotations of (0..0, g_m)
@@ -906,8 +361,9 @@ struct KrylovWork {
     bool inner_true_res[2] = {false, false};
     long long inner_gen[2] = {-1, -1};          // operator launch configuration baked into the graphs
     void *x0in = nullptr;                       // warm start of the inner cycle (inner precision)
-    double2 *part = nullptr;
+    double2 *part = nullptr;  // partial sums of a sweep, two sets
     int nparts = 0;
+    int *err = nullptr;       // the operator's device error word
     std::vector<double> history;
     int applies64 = 0, applies32 = 0;
     int hook_steps = 0;  // outer steps preconditioned through the hook in the last solve
@@ -924,8 +380,8 @@ static int alloc_level(Level &L, int m)
     G2_CUDA_CHECK(cudaMalloc(&L.y, sizeof(double2) * (KMAX + 1)));
     G2_CUDA_CHECK(cudaMalloc(&L.scal, sizeof(double) * S_NSCAL));
     G2_CUDA_CHECK(cudaMalloc(&L.flags, sizeof(int) * F_NFLAGS));
-    G2_CUDA_CHECK(cudaMalloc(&L.counter, sizeof(unsigned)));
-    G2_CUDA_CHECK(cudaMemset(L.counter, 0, sizeof(unsigned)));
+    G2_CUDA_CHECK(cudaMalloc(&L.counter, 3 * sizeof(unsigned)));
+    G2_CUDA_CHECK(cudaMemset(L.counter, 0, 3 * sizeof(unsigned)));
     G2_CUDA_CHECK(cudaMemset(L.flags, 0, sizeof(int) * F_NFLAGS));
     G2_CUDA_CHECK(cudaMemset(L.scal, 0, sizeof(double) * S_NSCAL));
     // the solver's kernels run on non-blocking streams, which are not ordered after the legacy stream
@@ -981,7 +437,7 @@ static int kw_alloc(KrylovWork *k, size_t N, int mo, int mi, int precision)
     G2_CUDA_CHECK(cudaMalloc(&k->xin, ei * N));
     G2_CUDA_CHECK(cudaMalloc(&k->x0in, ei * N));
     k->nparts = sweep_grid(N);
-    G2_CUDA_CHECK(cudaMalloc(&k->part, sizeof(double2) * (size_t)k->nparts * (KMAX + 1)));
+    G2_CUDA_CHECK(cudaMalloc(&k->part, 2 * sizeof(double2) * (size_t)k->nparts * (KMAX + 1)));
     int rc = alloc_level(k->Lo, mo);
     if (!rc) rc = alloc_level(k->Li, mi);
     return rc;
@@ -993,71 +449,12 @@ static int krylov_alloc(IeOp *op, int mo, int mi, int precision)
     if (k && k->mo == mo && k->mi == mi && k->precision == precision) return G2_OK;
     krylov_free(op);
     k = new KrylovWork();
+    k->err = op->d_err;
     op->krylov = k;
     return kw_alloc(k, op->nvec(), mo, mi, precision);
 }
 
 // ---- launch helpers ------------------------------------------------------------------------------
-// Blocks per instance of a sweep: whole waves of the instantiation's resident blocks, as near as possible to
-// `want` (the instance's partial-sum slots, never more).  A grid that asks for 4 blocks per SM of a kernel
-// that fits 3 runs a last wave at a third of the bytes in flight: the FP64 first-dots sweep (80 registers)
-// streamed at 2.6 TB/s that way against 5 TB/s for the same data in the correction pass.
-static int sm_count()
-{
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n > 0 ? n : 1;
-    }();
-    return sms;
-}
-template <class F> static int resident_blocks(F fn)
-{
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, kVT, 0) != cudaSuccess || b < 1) b = 1;
-    return b;
-}
-static int wave_grid(int per_sm, int want, int ninst)
-{
-    const int wave = per_sm * sm_count(), total = want * ninst;
-    int waves = (total + wave / 2) / wave;
-    if (waves < 1) waves = 1;
-    const int g = waves * wave / ninst;
-    return g < 1 ? 1 : (g < want ? g : want);
-}
-template <typename C, int K>
-static void launch_dots_first_k(KrylovWork *k, const C *V, const C *w, Level &L, const int *g, cudaStream_t st)
-{
-    static const int per_sm = resident_blocks(k_dots_first_t<C, K>);
-    g2_launch(k_dots_first_t<C, K>, wave_grid(per_sm, k->nparts, 1), kVT, 0, st, V, k->N, w, k->N, k->part, L, g);
-}
-template <typename C, int K>
-static void launch_pass_fused_k(KrylovWork *k, const C *V, C *w, Level &L, int p, const int *g, cudaStream_t st)
-{
-    g2_launch(k_cgs_pass_fused_t<C, K>, k->nparts, kVT, 0, st, V, k->N, w, k->N, k->part, L, p, g);
-}
-#define G2_KCASES(F, ...)                                                                                     \
-    switch (K) {                                                                                          \
-    case 0: F<C, 0>(__VA_ARGS__); break; case 1: F<C, 1>(__VA_ARGS__); break;                             \
-    case 2: F<C, 2>(__VA_ARGS__); break; case 3: F<C, 3>(__VA_ARGS__); break;                             \
-    case 4: F<C, 4>(__VA_ARGS__); break; case 5: F<C, 5>(__VA_ARGS__); break;                             \
-    case 6: F<C, 6>(__VA_ARGS__); break; case 7: F<C, 7>(__VA_ARGS__); break;                             \
-    case 8: F<C, 8>(__VA_ARGS__); break; case 9: F<C, 9>(__VA_ARGS__); break;                             \
-    case 10: F<C, 10>(__VA_ARGS__); break; case 11: F<C, 11>(__VA_ARGS__); break;                         \
-    case 12: F<C, 12>(__VA_ARGS__); break; case 13: F<C, 13>(__VA_ARGS__); break;                         \
-    case 14: F<C, 14>(__VA_ARGS__); break; case 15: F<C, 15>(__VA_ARGS__); break;                         \
-    case 16: F<C, 16>(__VA_ARGS__); break; case 17: F<C, 17>(__VA_ARGS__); break;                         \
-    case 18: F<C, 18>(__VA_ARGS__); break; case 19: F<C, 19>(__VA_ARGS__); break;                         \
-    case 20: F<C, 20>(__VA_ARGS__); break; case 21: F<C, 21>(__VA_ARGS__); break;                         \
-    case 22: F<C, 22>(__VA_ARGS__); break; case 23: F<C, 23>(__VA_ARGS__); break;                         \
-    case 24: F<C, 24>(__VA_ARGS__); break; case 25: F<C, 25>(__VA_ARGS__); break;                         \
-    case 26: F<C, 26>(__VA_ARGS__); break; case 27: F<C, 27>(__VA_ARGS__); break;                         \
-    case 28: F<C, 28>(__VA_ARGS__); break; case 29: F<C, 29>(__VA_ARGS__); break;                         \
-    case 30: F<C, 30>(__VA_ARGS__); break; case 31: F<C, 31>(__VA_ARGS__); break;                         \
-    default: F<C, 32>(__VA_ARGS__); break;                                                                \
-    }
-
 template <typename C>
 static void norm2(KrylovWork *k, const C *w, double *nrm2, const int *g, cudaStream_t st)
 {
@@ -1065,56 +462,25 @@ static void norm2(KrylovWork *k, const C *w, double *nrm2, const int *g, cudaStr
     g2_launch(k_norm2_fused<C>, k->nparts, kVT, 0, st, w, k->N, k->part, nrm2, k->Lo.counter, g); g2_count_launches(1);
 }
 
-// CGS for Arnoldi step j on level L with basis V (j+1 columns) and vector w: the first pass's dots and
-// up to N_IGS+1 correction passes, each one launch (passes after the decision to stop exit at once)
+// Arnoldi step j on level L with basis V (j + 1 columns) and vector w
 template <typename C>
-static void cgs(KrylovWork *k, Level &L, const C *V, int j, C *w, const int *gate, cudaStream_t st)
+static int arnoldi_step1(KrylovWork *k, Level &L, C *V, int j, C *w, double tol, const int *gate, cudaStream_t st)
 {
-    const int K = j + 1;
-    G2_KCASES(launch_dots_first_k, k, V, w, L, gate, st)
+    Multi<C> mm{};
+    mm.V[0] = V;
+    mm.w[0] = w;
+    mm.part[0] = k->part;
+    mm.L[0] = L;
+    mm.gate[0] = gate;
     g2_count_launches(1);
-    for (int p = 1; p <= N_IGS + 1; p++) {
-        G2_KCASES(launch_pass_fused_k, k, V, w, L, p, gate, st)
-        g2_count_launches(1);
-    }
+    return arnoldi_step(mm, 1, k->N, k->nparts, j, tol, k->err, st);
 }
-// end of Arnoldi step j: V_{j+1} = w / ||w|| and the Givens / misfit update, one launch
+// the same for n lockstep instances (vector length N, nparts partial-sum slots each) in one launch
 template <typename C>
-static void arnoldi_tail(KrylovWork *k, Level &L, C *V, int j, const C *w, double tol, const int *gate, cudaStream_t st)
+static int arnoldi_step_multi(const Multi<C> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
 {
-    g2_launch(k_scale_finish<C>, sweep_grid(k->N), kVT, 0, st, V + (size_t)(j + 1) * k->N, w, k->N, L, j, tol, gate);
     g2_count_launches(1);
-}
-
-// the same CGS and Arnoldi tail for n lockstep instances (vector length N, nparts blocks each) in one
-// launch per kernel
-template <typename C, int K>
-static void launch_dots_first_km(const Multi<C> &mm, int n, size_t N, int nparts, cudaStream_t st)
-{
-    static const int per_sm = resident_blocks(k_dots_first_m<C, K>);
-    g2_launch(k_dots_first_m<C, K>, dim3(wave_grid(per_sm, nparts, n), n), kVT, 0, st, mm, N, N);
-}
-template <typename C, int K>
-static void launch_pass_fused_km(const Multi<C> &mm, int n, size_t N, int nparts, int p, cudaStream_t st)
-{
-    g2_launch(k_cgs_pass_fused_m<C, K>, dim3(nparts, n), kVT, 0, st, mm, N, N, p);
-}
-template <typename C>
-static void cgs_multi(const Multi<C> &mm, int n, size_t N, int nparts, int j, cudaStream_t st)
-{
-    const int K = j + 1;
-    G2_KCASES(launch_dots_first_km, mm, n, N, nparts, st)
-    g2_count_launches(1);
-    for (int p = 1; p <= N_IGS + 1; p++) {
-        G2_KCASES(launch_pass_fused_km, mm, n, N, nparts, p, st)
-        g2_count_launches(1);
-    }
-}
-template <typename C>
-static void arnoldi_tail_multi(const Multi<C> &mm, int n, size_t N, int j, double tol, cudaStream_t st)
-{
-    g2_launch(k_scale_finish_m<C>, dim3(sweep_grid(N), n), kVT, 0, st, mm, N, j, tol);
-    g2_count_launches(1);
+    return arnoldi_step(mm, n, N, nparts, j, tol, err, st);
 }
 
 template <typename C> static int apply_prec(IeOp *op, const C *in, C *out, cudaStream_t st, const int *gate);
@@ -1156,8 +522,7 @@ static int inner_solve(IeOp *op, KrylovWork *k, const CI *v, const CI *x0, CI *x
         if (rc) return rc;
         k->applies32 += sizeof(CI) == 8 ? 1 : 0;
         k->applies64 += sizeof(CI) == 16 ? 1 : 0;
-        cgs<CI>(k, L, Vi, j, wi, krylov, st);
-        arnoldi_tail<CI>(k, L, Vi, j, wi, tol, krylov, st);
+        if ((rc = arnoldi_step1<CI>(k, L, Vi, j, wi, tol, krylov, st))) return rc;
     }
     // FinalActions -> ConstructCurrentSolution (gmres.F90:423-458): x = x0 + V y
     g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, solver); g2_count_launches(1);
@@ -1315,8 +680,7 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
                 if ((rc = ie_apply_device64(op, k->tmp, k->w, st))) return rc;
             }
             k->applies64++;
-            cgs<double2>(k, L, k->Vo, j, k->w, nullptr, st);
-            arnoldi_tail<double2>(k, L, k->Vo, j, k->w, tol, nullptr, st);
+            if ((rc = arnoldi_step1<double2>(k, L, k->Vo, j, k->w, tol, nullptr, st))) return rc;
             if ((rc = pull())) return rc;
             bea = h_scal[S_BEA];
             if (!std::isfinite(bea)) {
@@ -1510,6 +874,7 @@ int batch_create(IeOp *const *ops, int n, int mo, int mi, int precision, void **
         if (!ops[i]) { batch_destroy(b); return G2_ERR_ARG; }
         b->ops.push_back(ops[i]);
         KrylovWork *k = new KrylovWork();
+        k->err = ops[i]->d_err;
         b->k.push_back(k);
         const int rc = kw_alloc(k, ops[i]->nvec(), mo, mi, precision);
         if (rc) { batch_destroy(b); return rc; }
@@ -1608,7 +973,7 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
     }
     // Arnoldi step j of the active instances in `act`: runs of up to KMI instances with the same vector length
     // share each launch (each instance keeps its own blocks, partials and gates)
-    auto arnoldi_step = [&](const std::vector<int> &act, int j) {
+    auto arnoldi_of = [&](const std::vector<int> &act, int j) -> int {
         for (size_t c = 0; c < act.size();) {
             KrylovWork *k0 = b->k[act[c]];
             size_t e = c + 1;
@@ -1617,8 +982,8 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
             if (e - c == 1) {
                 Level &L = k0->Li;
                 CI *Vi = reinterpret_cast<CI *>(k0->Vi);
-                cgs<CI>(k0, L, Vi, j, reinterpret_cast<CI *>(k0->wi), L.flags + F_KRYLOV, st);
-                arnoldi_tail<CI>(k0, L, Vi, j, reinterpret_cast<const CI *>(k0->wi), tol, L.flags + F_KRYLOV, st);
+                const int r = arnoldi_step1<CI>(k0, L, Vi, j, reinterpret_cast<CI *>(k0->wi), tol, L.flags + F_KRYLOV, st);
+                if (r) return r;
             } else {
                 Multi<CI> mm{};
                 for (size_t q = 0; q < e - c; q++) {
@@ -1629,11 +994,12 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
                     mm.L[q] = k->Li;
                     mm.gate[q] = k->Li.flags + F_KRYLOV;
                 }
-                cgs_multi<CI>(mm, (int)(e - c), k0->N, k0->nparts, j, st);
-                arnoldi_tail_multi<CI>(mm, (int)(e - c), k0->N, j, tol, st);
+                const int r = arnoldi_step_multi<CI>(mm, (int)(e - c), k0->N, k0->nparts, j, tol, k0->err, st);
+                if (r) return r;
             }
             c = e;
         }
+        return G2_OK;
     };
     // Each operator group (one frequency's polarisations) runs its apply and then its Arnoldi step before the
     // next group's apply, so the group's fresh w is still in L2 when its Gram-Schmidt reads it (with all
@@ -1648,7 +1014,7 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
                 if (b->h_active[i]) act.push_back(i);
             if (act.empty()) continue;
             if ((rc = batch_apply<CI>(b, vj, wi, F_KRYLOV, st, &g))) return rc;
-            arnoldi_step(act, j);
+            if ((rc = arnoldi_of(act, j))) return rc;
         }
     }
     for (int i = 0; i < n; i++) {
@@ -1919,8 +1285,7 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                 if (act.size() == 1) {
                     KrylovWork *k0 = b->k[act[0]];
                     const int *go = k0->Lo.flags + F_KRYLOV;
-                    cgs<double2>(k0, k0->Lo, k0->Vo, j, k0->w, go, st);
-                    arnoldi_tail<double2>(k0, k0->Lo, k0->Vo, j, k0->w, tol, go, st);
+                    if ((r = arnoldi_step1<double2>(k0, k0->Lo, k0->Vo, j, k0->w, tol, go, st))) return r;
                 } else if (act.size() == 2 && b->k[act[0]]->N == b->k[act[1]]->N &&
                            b->k[act[0]]->nparts == b->k[act[1]]->nparts) {
                     Multi<double2> mm{};
@@ -1932,14 +1297,13 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                         mm.L[q] = k->Lo;
                         mm.gate[q] = k->Lo.flags + F_KRYLOV;
                     }
-                    cgs_multi<double2>(mm, 2, b->k[act[0]]->N, b->k[act[0]]->nparts, j, st);
-                    arnoldi_tail_multi<double2>(mm, 2, b->k[act[0]]->N, j, tol, st);
+                    KrylovWork *k0 = b->k[act[0]];
+                    if ((r = arnoldi_step_multi<double2>(mm, 2, k0->N, k0->nparts, j, tol, k0->err, st))) return r;
                 } else {
                     for (int i : act) {
                         KrylovWork *k = b->k[i];
                         const int *go = k->Lo.flags + F_KRYLOV;
-                        cgs<double2>(k, k->Lo, k->Vo, j, k->w, go, st);
-                        arnoldi_tail<double2>(k, k->Lo, k->Vo, j, k->w, tol, go, st);
+                        if ((r = arnoldi_step1<double2>(k, k->Lo, k->Vo, j, k->w, tol, go, st))) return r;
                     }
                 }
             }

@@ -1,0 +1,257 @@
+// Device pieces of the Krylov solver shared by its kernels (arnoldi.cu: a whole Arnoldi step in one launch;
+// krylov.cu: everything else): the state of one GMRES level, the reductions and the scalar steps.
+#pragma once
+#include "common.cuh"
+#include "krylov.h"
+
+struct Level {
+    int m = 0;
+    double2 *H = nullptr;   // (m+1) x (m+1) column-major, column m holds g
+    double *cs = nullptr;
+    double2 *sn = nullptr;
+    double2 *hpass = nullptr, *hnext = nullptr, *y = nullptr;
+    double *scal = nullptr;
+    int *flags = nullptr;
+    // [0] blocks done, for the last-block reductions (back to 0 after each use); [1], [2] arrivals and generation of
+    // the grid barrier of arnoldi.cu
+    unsigned *counter = nullptr;
+};
+
+// Several instances of one batch in one launch (blockIdx.y = instance): vectors of one length, and per instance its
+// partials, barrier and gate.
+constexpr int KMI = 4;
+template <typename C>
+struct Multi {
+    C *V[KMI];
+    C *w[KMI];
+    double2 *part[KMI];
+    Level L[KMI];
+    const int *gate[KMI];
+};
+
+// arnoldi.cu: Arnoldi step j (dots, correction passes, scaling, Givens) of n instances in one cooperative launch
+int arnoldi_step(const Multi<float2> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st);
+int arnoldi_step(const Multi<double2> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st);
+
+namespace {
+
+constexpr int kVT = 256;   // threads of the vector kernels
+constexpr int kILP = 4;    // elements per thread and iteration of the element-wise vector kernels
+constexpr int KMAX = 32;   // largest basis handled in one sweep
+constexpr double ZERO_THRESHOLD = 1e-14;  // gmres.F90:21
+constexpr int N_IGS = 3;                  // gmres.F90:22
+constexpr double kHookGain = 0.5;         // an outer step through the hook must halve the misfit
+
+enum { F_KRYLOV = 0, F_PASS = 1, F_L = 2, F_ITER = 3, F_SOLVER = 4, F_NFLAGS = 8 };
+enum { S_BN = 0, S_BETA = 1, S_DNORMW = 2, S_DLOO = 3, S_BEA = 4, S_NRM2 = 5, S_NSCAL = 8 };
+
+G2_HD int hix(int i, int j, int m) { return i + j * (m + 1); }
+
+template <typename C> G2_D double2 ld2(const C *p, size_t i);
+template <> G2_D double2 ld2<double2>(const double2 *p, size_t i) { return p[i]; }
+template <> G2_D double2 ld2<float2>(const float2 *p, size_t i)
+{
+    const float2 v = p[i];
+    return make_double2(v.x, v.y);
+}
+template <typename C> G2_D void st2(C *p, size_t i, double2 v);
+template <> G2_D void st2<double2>(double2 *p, size_t i, double2 v) { p[i] = v; }
+template <> G2_D void st2<float2>(float2 *p, size_t i, double2 v) { p[i] = make_float2((float)v.x, (float)v.y); }
+
+// The basis sweeps move 16-byte words: two complex64 values per load (complex128 values are 16 bytes
+// already).  On a B200 a two-instance sweep of 11 complex64 vectors of 1.57 M elements took 84 us with
+// 8-byte loads and 52 us with 16-byte loads.  Vectors whose length (and column stride) is odd keep
+// element-wise loads, since their odd columns are not 16-byte aligned.
+template <typename C> struct Wide;
+template <> struct Wide<float2> {
+    using T = float4;
+    static constexpr int E = 2;
+};
+template <> struct Wide<double2> {
+    using T = double2;
+    static constexpr int E = 1;
+};
+G2_D float2 part_of(const float4 &p, int e) { return e ? make_float2(p.z, p.w) : make_float2(p.x, p.y); }
+G2_D double2 part_of(const double2 &p, int) { return p; }
+G2_D void set_part(float4 &p, int e, float2 v)
+{
+    if (e) {
+        p.z = v.x;
+        p.w = v.y;
+    } else {
+        p.x = v.x;
+        p.y = v.y;
+    }
+}
+G2_D void set_part(double2 &p, int, double2 v) { p = v; }
+// words of E elements over the whole vector, or 0 when the lengths do not allow them
+template <typename C> G2_D size_t wide_words(size_t N, size_t ld)
+{
+    constexpr int E = Wide<C>::E;
+    return (N % E == 0 && ld % E == 0) ? N / E : 0;
+}
+
+template <typename C> struct RealOf;
+template <> struct RealOf<double2> { using T = double; };
+template <> struct RealOf<float2> { using T = float; };
+
+// per-thread partial sums in the vector's precision (a handful of elements each), block and grid
+// reductions in FP64
+template <int KM, typename R>
+G2_D void block_reduce_store_r(R (&ax)[KM + 1], R (&ay)[KM + 1], double2 *part)
+{
+    __shared__ double2 red[kVT / 32][KM + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k <= KM; k++) {
+        double vx = ax[k], vy = ay[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            vx += __shfl_xor_sync(0xffffffffu, vx, o);
+            vy += __shfl_xor_sync(0xffffffffu, vy, o);
+        }
+        if (lane == 0) red[warp][k] = make_double2(vx, vy);
+    }
+    __syncthreads();
+    if (threadIdx.x <= KM) {
+        double2 s = make_double2(0.0, 0.0);
+        for (int w = 0; w < kVT / 32; w++) {
+            s.x += red[w][threadIdx.x].x;
+            s.y += red[w][threadIdx.x].y;
+        }
+        part[(size_t)blockIdx.x * (KMAX + 1) + (threadIdx.x == KM ? KMAX : threadIdx.x)] = s;
+    }
+}
+
+// ---- scalar steps -------------------------------------------------------------------------------
+G2_D double cabs_(double2 a) { return hypot(a.x, a.y); }
+G2_D double2 cmul_(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+G2_D double2 cdivr(double2 a, double r) { return make_double2(a.x / r, a.y / r); }
+// netlib ZROT on one pair
+G2_D void zrot1(double2 &cx, double2 &cy, double c, double2 s)
+{
+    const double2 t = make_double2(c * cx.x + (s.x * cy.x - s.y * cy.y), c * cx.y + (s.x * cy.y + s.y * cy.x));
+    const double2 sc = make_double2(s.x, -s.y);
+    cy = make_double2(c * cy.x - (sc.x * cx.x - sc.y * cx.y), c * cy.y - (sc.x * cx.y + sc.y * cx.x));
+    cx = t;
+}
+// netlib ZROTG
+G2_D void zrotg(double2 &ca, double2 cb, double &c, double2 &s)
+{
+    const double aca = cabs_(ca);
+    if (aca == 0.0) {
+        c = 0.0;
+        s = make_double2(1.0, 0.0);
+        ca = cb;
+    } else {
+        const double scale = aca + cabs_(cb);
+        const double a1 = cabs_(cdivr(ca, scale)), b1 = cabs_(cdivr(cb, scale));
+        const double norm = scale * sqrt(a1 * a1 + b1 * b1);
+        const double2 alpha = cdivr(ca, aca);
+        c = aca / norm;
+        s = cdivr(cmul_(alpha, make_double2(cb.x, -cb.y)), norm);
+        ca = make_double2(alpha.x * norm, alpha.y * norm);
+    }
+}
+
+// end of Arnoldi step j (gmres.F90:283-326): H(j+1,j), rotations, Arnoldi misfit, exit test
+G2_D void arnoldi_finish_body(Level &L, int j, double tol)
+{
+    // run by every thread of one block: column j of H, the rotations so far and g(j), g(j+1) are staged in
+    // shared memory with one round of loads; thread 0 then applies the same operations in the same order
+    // as a single thread on global memory would (a chain of dependent L2 loads otherwise)
+    __shared__ double2 hc[KMAX + 1], sn_s[KMAX], gs[2];
+    __shared__ double cs_s[KMAX];
+    const int m = L.m;
+    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) hc[i] = L.H[hix(i, j, m)];
+    for (int i = threadIdx.x; i < j; i += blockDim.x) {
+        cs_s[i] = L.cs[i];
+        sn_s[i] = L.sn[i];
+    }
+    if (threadIdx.x < 2) gs[threadIdx.x] = L.H[hix(j + threadIdx.x, m, m)];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double dnormw = L.scal[S_DNORMW], bn = L.scal[S_BN];
+        hc[j + 1] = make_double2(dnormw, 0.0);
+        for (int i = 0; i < j; i++) zrot1(hc[i], hc[i + 1], cs_s[i], sn_s[i]);
+        double2 h1 = hc[j], sn;
+        double c;
+        zrotg(h1, hc[j + 1], c, sn);
+        zrot1(gs[0], gs[1], c, sn);
+        zrot1(hc[j], hc[j + 1], c, sn);
+        hc[j + 1] = make_double2(0.0, 0.0);
+        L.cs[j] = c;
+        L.sn[j] = sn;
+        L.H[hix(j, m, m)] = gs[0];
+        L.H[hix(j + 1, m, m)] = gs[1];
+        const double bea = cabs_(gs[1]) / bn;
+        L.scal[S_BEA] = bea;
+        L.flags[F_ITER] += 1;
+        L.flags[F_L] = j + 1;
+        if (bea < tol || j + 1 >= m) L.flags[F_KRYLOV] = 0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) L.H[hix(i, j, m)] = hc[i];
+}
+
+// ---- fused reductions: the last block to finish sums every block's partials ----------------------
+// Each block stores its partials, then counts itself done; the block that counts last reduces all
+// partials in a fixed order (lane-strided sums, shuffle tree: the result does not depend on which block
+// is last) and runs the scalar step that used to be a separate one-thread launch.  It resets the counter
+// for the next use.  Blocks test their gates before any of them can reach the last block, so a flag the
+// last block changes cannot be seen half-way through the grid.
+G2_D bool last_block(unsigned *counter)
+{
+    __shared__ bool am_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) am_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (am_last && threadIdx.x == 0) *counter = 0u;
+    return am_last;
+}
+// sums of part[b][col] over blocks for columns 0..K-1 into h[], and of column KMAX into *nrm (one block)
+G2_D void reduce_partials(const double2 *part, int nb, int K, double2 *h, double *nrm)
+{
+    __threadfence();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int k = warp; k <= K; k += nw) {
+        const int col = (k == K) ? KMAX : k;
+        double sx = 0.0, sy = 0.0;
+        // eight independent loads per lane and round (rows past nb predicated off): the partials come from
+        // L2, and each round is one L2 round trip, so 256 rows cost one
+        for (int b0 = 0; b0 < nb; b0 += 256) {
+            double2 v[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int b = b0 + lane + 32 * q;
+                v[q] = b < nb ? __ldcg(part + (size_t)b * (KMAX + 1) + col) : make_double2(0.0, 0.0);
+            }
+            sx += ((v[0].x + v[1].x) + (v[2].x + v[3].x)) + ((v[4].x + v[5].x) + (v[6].x + v[7].x));
+            sy += ((v[0].y + v[1].y) + (v[2].y + v[3].y)) + ((v[4].y + v[5].y) + (v[6].y + v[7].y));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        }
+        if (lane == 0) {
+            if (k < K) h[k] = make_double2(sx, sy);
+            else if (nrm) *nrm = sx;
+        }
+    }
+    __syncthreads();
+}
+
+// elements per thread and round of the basis sweeps: all (K + 1) * U loads of a round are issued before the
+// first product, so a round costs one memory round trip; the values held stay within 256 bytes per thread
+// (32 complex64 or 16 complex128).  0: the basis is too wide to hold, the sweep loads one element at a time.
+template <int K, typename C> struct SweepU {
+    static constexpr int B = (K + 1) * (int)sizeof(C);
+    static constexpr int v = B * 4 <= 256 ? 4 : (B * 2 <= 256 ? 2 : (B <= 256 ? 1 : 0));
+};
+
+G2_D float2 scaled(float2 a, double s) { return make_float2((float)(a.x * s), (float)(a.y * s)); }
+G2_D double2 scaled(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
+
+}  // namespace
