@@ -37,6 +37,8 @@ constexpr int kThreads = 256;
 template <typename R, int CAP> struct PassLB { static constexpr int T = kThreads, B = 1; };
 template <> struct PassLB<float, 1> { static constexpr int T = 256, B = 4; };
 template <> struct PassLB<double, 1> { static constexpr int T = 128, B = 4; };
+// CAP = 2: the three-step transform of 512-point lines, two blocks of 512 threads
+template <typename R> struct PassLB<R, 2> { static constexpr int T = 512, B = 2; };
 
 // The vectors of one apply: nv = 1, or nv = 2 right-hand sides of the same operator that share every
 // tensor read.  Line zc of a pass runs over [0, nv*3Nz): vector zc / 3Nz, row zc % 3Nz.
@@ -93,8 +95,14 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fx(con
         return cmul(in[lzc * plane + row + x], gsig[z * plane + row + x]);
     };
     auto store = [&](int t, int kx, C v) { U1[(kx * Ny + y) * ZL + zc0 + t] = v; };
-    auto off = [&](int t, int n1, int k2) { return n1 + N1 * k2 + (L + 1) * t; };
-    fft4step<C, N1, N2, false, true, false, false, true>(sm, nl, ilog2(NL), tw, load, store, off);
+    if constexpr (CAP == 2) {
+        fft512<C, false, true, false, false, true>(
+            sm, nl, ilog2(NL), tw, load, [](int, int) { return 0; }, [&](int t, int kx, C v, int) { store(t, kx, v); },
+            [&](int t, int n0, int k2) { return n0 + 64 * k2 + (L + 1) * t; });
+    } else {
+        auto off = [&](int t, int n1, int k2) { return n1 + N1 * k2 + (L + 1) * t; };
+        fft4step<C, N1, N2, false, true, false, false, true>(sm, nl, ilog2(NL), tw, load, store, off);
+    }
 }
 
 // k_fy: zero-pad to 2Ny, forward y-FFT of one kx column, scatter to (q, r, slot).
@@ -137,8 +145,14 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_fy(con
         ky_to_slot(ky, L / 2, r, sy);  // L = 2Ny: with the output index's range known, this folds per output
         dst[(r * 4 + sy) * ZP + zpos(t)] = v;
     };
-    auto off = [&](int t, int n1, int k2) { return t + NL * (n1 + N1 * k2); };
-    fft4step<C, N1, N2, false, true, false, true, true>(sm, nl, ilog2(NL), tw, load, store, off);
+    if constexpr (CAP == 2) {
+        fft512<C, false, true, false, true, true>(
+            sm, nl, ilog2(NL), tw, load, [](int, int) { return 0; }, [&](int t, int ky, C v, int) { store(t, ky, v); },
+            [&](int t, int n0, int k2) { return t + NL * (n0 + 64 * k2); });
+    } else {
+        auto off = [&](int t, int n1, int k2) { return t + NL * (n1 + N1 * k2); };
+        fft4step<C, N1, N2, false, true, false, true, true>(sm, nl, ilog2(NL), tw, load, store, off);
+    }
 }
 
 // k_by: inverse y-FFT of one kx column, crop y < Ny.  Distributed_FFT.F90:455-476, 696-788
@@ -172,8 +186,14 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_by(con
         return src[(r * 4 + sy) * ZP + zpos(t)];
     };
     auto store = [&](int t, int yy, C v) { col[yy * Z3 + t] = v; };
-    auto off = [&](int t, int n1, int k2) { return t + NL * (n1 + N1 * k2); };
-    fft4step<C, N1, N2, true, false, true, true, true>(sm, nl, ilog2(NL), tw, load, store, off);
+    if constexpr (CAP == 2) {
+        fft512<C, true, false, true, true, true>(
+            sm, nl, ilog2(NL), tw, load, [](int, int) { return 0; }, [&](int t, int yy, C v, int) { store(t, yy, v); },
+            [&](int t, int n0, int k2) { return t + NL * (n0 + 64 * k2); });
+    } else {
+        auto off = [&](int t, int n1, int k2) { return t + NL * (n1 + N1 * k2); };
+        fft4step<C, N1, N2, true, false, true, true, true>(sm, nl, ilog2(NL), tw, load, store, off);
+    }
 }
 
 // k_bx: inverse x-FFT, crop x < Nx, post-combine y = s*(a*x - w/(dz*4NxNy)).
@@ -214,8 +234,13 @@ __global__ void __launch_bounds__(PassLB<R, CAP>::T, PassLB<R, CAP>::B) k_bx(con
         o.y = (d1.y - w.y * inv) * sq;
         out[lzc * plane + row + x] = o;
     };
-    auto off = [&](int t, int n1, int k2) { return t * (L + 1) + k2 + N2 * n1; };
-    fft4step_pre<C, N1, N2, true, false, true, true, false>(sm, nl, ilog2(NL), tw, load, pre, store, off);
+    if constexpr (CAP == 2) {
+        fft512<C, true, false, true, true, false>(sm, nl, ilog2(NL), tw, load, pre, store,
+                                                  [&](int t, int n0, int k2) { return t * (L + 1) + k2 + 8 * n0; });
+    } else {
+        auto off = [&](int t, int n1, int k2) { return t * (L + 1) + k2 + N2 * n1; };
+        fft4step_pre<C, N1, N2, true, false, true, true, false>(sm, nl, ilog2(NL), tw, load, pre, store, off);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -362,7 +387,7 @@ static size_t ystate_elems(const IeOp *op) { return (ie_ypipe_state_bytes(op->Nx
 // lines take what the tile allows (256x256x48 complex64 1754 / 1754 / 1855 / 1864 us).
 static int lines_for(int L, size_t es, int cap)
 {
-    if (cap == 0 && L <= 256) cap = es == sizeof(double2) ? 8 : 16;
+    if (cap == 0 && L <= 512) cap = es == sizeof(double2) ? 8 : 16;
     int n = cap >= 1 && cap <= 32 ? cap : 32;
     while (n > 1 && (size_t)(n * (L + 1) + L) * es > 100 * 1024) n >>= 1;
     return n;
@@ -391,9 +416,6 @@ template <typename K> static void big_smem(K k)
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
-// the register-capped pass kernels apply when the block fits their bounds (PassLB)
-template <typename R, int L> static bool use_cap(int nt) { return L <= 256 && nt <= PassLB<R, 1>::T; }
-
 template <typename R, int L, int CAP>
 static void launch_x_k(bool fwd, IeOp *op, const VecSet<CT<R>> &vs, CT<R> *U1, cudaStream_t st, const int *gate,
                        dim3 grid, int nt, size_t sm, int NL)
@@ -416,8 +438,13 @@ static void launch_x(bool fwd, IeOp *op, const VecSet<CT<R>> &vs, CT<R> *U1, cud
     const int NL = lines_for(L, es, op->fft_lines[es == sizeof(double2) ? 0 : 1]), nt = threads_for(L, NL);
     const size_t sm = (size_t)(NL * (L + 1) + L) * es;
     dim3 grid((ZL + NL - 1) / NL, op->Ny);
-    if (use_cap<R, L>(nt)) launch_x_k<R, L, 1>(fwd, op, vs, U1, st, gate, grid, nt, sm, NL);
-    else launch_x_k<R, L, 0>(fwd, op, vs, U1, st, gate, grid, nt, sm, NL);
+    if constexpr (L == 512) {
+        launch_x_k<R, L, 2>(fwd, op, vs, U1, st, gate, grid, 512, sm, NL);
+    } else {
+        if constexpr (L <= 256)
+            if (nt <= PassLB<R, 1>::T) return launch_x_k<R, L, 1>(fwd, op, vs, U1, st, gate, grid, nt, sm, NL);
+        launch_x_k<R, L, 0>(fwd, op, vs, U1, st, gate, grid, nt, sm, NL);
+    }
 }
 
 template <typename R, int L, int CAP>
@@ -439,8 +466,14 @@ static void launch_y(bool fwd, IeOp *op, int nv, int pitch, CT<R> *U1, CT<R> *Uh
     const int NL = lines_for(L, es, op->fft_lines[es == sizeof(double2) ? 0 : 1]), nt = threads_for(L, NL);
     const size_t sm = (size_t)(NL * (L + 1) + L) * es;
     dim3 grid((ZL + NL - 1) / NL, 2 * op->Nx);
-    if (use_cap<R, L>(nt)) launch_y_k<R, L, 1>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, nt, sm, NL);
-    else launch_y_k<R, L, 0>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, nt, sm, NL);
+    if constexpr (L == 512) {
+        launch_y_k<R, L, 2>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, 512, sm, NL);
+    } else {
+        if constexpr (L <= 256)
+            if (nt <= PassLB<R, 1>::T)
+                return launch_y_k<R, L, 1>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, nt, sm, NL);
+        launch_y_k<R, L, 0>(fwd, op, nv, pitch, U1, Uh, st, gate, grid, nt, sm, NL);
+    }
 }
 
 template <typename R>

@@ -33,7 +33,7 @@ G2_D C twid(const C *tw, int idx)
 }
 
 // d * W_N^e for the register DFTs: e = 0 is 1 and e = N/4 is -i (forward) or +i (inverse), exactly (a
-// swap and a sign); other exponents read the table.
+// swap and a sign); multiples of N/16 are constants; the rest (32-point DFTs) reads the table.
 template <typename C, int N, bool INV>
 G2_D C twiddle_mul(C d, int e, const C *tw, int Lstride)
 {
@@ -43,6 +43,17 @@ G2_D C twiddle_mul(C d, int e, const C *tw, int Lstride)
         if (INV) { r.x = -d.y; r.y = d.x; }
         else { r.x = d.y; r.y = -d.x; }
         return r;
+    }
+    if (16 * e % N == 0) {  // e = k N / 16, k = 1, 2, 3, 5, 6, 7
+        using R = decltype(d.x);
+        constexpr R h = R(0.70710678118654752440), c = R(0.92387953251128675613), s = R(0.38268343236508977173);
+        const int k = 16 * e / N, m = k < 4 ? k : 8 - k;
+        C w;
+        w.x = m == 1 ? c : (m == 2 ? h : s);
+        w.y = m == 1 ? -s : (m == 2 ? -h : -c);
+        if (k > 4) w.x = -w.x;
+        if (INV) w.y = -w.y;
+        return cmul(d, w);
     }
     return cmul(d, twid<C, INV>(tw, e * Lstride));
 }
@@ -244,6 +255,86 @@ G2_D void fft4step_pre(C *sm, int nl, int lg_nl, const C *tw, LoadF load, PreF p
 #pragma unroll
         for (int k1 = 0; k1 < NOUT; k1++) store(line, k2 + N2 * k1, a[brev_c(k1, Log2<N1>::v)], p[k1]);
     }
+}
+
+// 512-point lines in three steps of 8 x 8 x 8: 8 values per thread and step where 32 x 16 held 32, so that two blocks of
+// 512 threads fit an SM (the forward complex64 y pass of a 256x256x48 pair took 356 us as 32 x 16 and takes 237 us this
+// way, the inverse x pass 207 and 141 us; the inverse y and forward x passes are as before).  n = n0 + 64 n2, n0 = m0 + 8 m1; k = k2 + 8 (j1 + 8 j0).  Step 1 transforms n2 -> k2 and parks
+// (n0, k2) at off(line, n0, k2); step 2 transforms m1 -> j1 in place; step 3 transforms m0 -> j0.  pre and store as in
+// fft4step_pre.  Items: LF1, LF3 line index fastest in steps 1 and 3 (else n0, and the output index), in step 2 always.
+// tid, nthr, sync: as in fft4step_part.
+template <typename C, bool INV, bool PAD_IN, bool CROP_OUT, bool LF1, bool LF3, class LoadF, class PreF, class StoreF,
+          class OffF, class SyncF>
+G2_D void fft512_part(C *sm, int nl, int lg_nl, const C *tw, LoadF load, PreF pre, StoreF store, OffF off, int tid, int nthr,
+                      SyncF sync)
+{
+    constexpr int NOUT = CROP_OUT ? 4 : 8;
+    const int nlb = 1 << lg_nl;
+    // padded complex64 lines (four loads per item): the loads of two items together, before the first DFT
+    constexpr int IT = sizeof(C) == 8 && PAD_IN && LF1 ? 2 : 1;
+    for (int it0 = tid; it0 < nlb * 64; it0 += IT * nthr) {
+        C a[IT][8];
+#pragma unroll
+        for (int r = 0; r < IT; r++) {
+            const int it = it0 + r * nthr;
+            const int line = LF1 ? it & (nlb - 1) : it >> 6, n0 = LF1 ? (it >> lg_nl) & 63 : it & 63;
+            if (it >= nlb * 64 || line >= nl) continue;
+#pragma unroll
+            for (int n2 = 0; n2 < 8; n2++) {
+                if (PAD_IN && n2 >= 4) a[r][n2] = czero<C>();
+                else a[r][n2] = load(line, n0 + 64 * n2);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < IT; r++) {
+            const int it = it0 + r * nthr;
+            const int line = LF1 ? it & (nlb - 1) : it >> 6, n0 = LF1 ? (it >> lg_nl) & 63 : it & 63;
+            if (it >= nlb * 64 || line >= nl) continue;
+            reg_dft_dif<C, 8, INV, PAD_IN>(a[r], tw, 64);
+#pragma unroll
+            for (int k2 = 0; k2 < 8; k2++) {
+                C v = a[r][brev_c(k2, 3)];
+                if (k2 != 0) v = cmul(v, twid<C, INV>(tw, n0 * k2));
+                sm[off(line, n0, k2)] = v;
+            }
+        }
+    }
+    sync();
+    for (int it = tid; it < nlb * 64; it += nthr) {
+        const int line = it & (nlb - 1), q = (it >> lg_nl) & 63, m0 = q & 7, k2 = q >> 3;
+        if (line >= nl) continue;
+        C a[8];
+#pragma unroll
+        for (int m1 = 0; m1 < 8; m1++) a[m1] = sm[off(line, m0 + 8 * m1, k2)];
+        reg_dft_dif<C, 8, INV, false>(a, tw, 64);
+#pragma unroll
+        for (int j1 = 0; j1 < 8; j1++) {
+            C v = a[brev_c(j1, 3)];
+            if (j1 != 0) v = cmul(v, twid<C, INV>(tw, 8 * m0 * j1));
+            sm[off(line, m0 + 8 * j1, k2)] = v;
+        }
+    }
+    sync();
+    for (int it = tid; it < nlb * 64; it += nthr) {
+        const int line = LF3 ? it & (nlb - 1) : it >> 6, q = LF3 ? (it >> lg_nl) & 63 : it & 63, k2 = q & 7, j1 = q >> 3;
+        if (line >= nl) continue;
+        decltype(pre(0, 0)) p[NOUT];
+#pragma unroll
+        for (int j0 = 0; j0 < NOUT; j0++) p[j0] = pre(line, q + 64 * j0);
+        C a[8];
+#pragma unroll
+        for (int m0 = 0; m0 < 8; m0++) a[m0] = sm[off(line, m0 + 8 * j1, k2)];
+        reg_dft_dif<C, 8, INV, false>(a, tw, 64);
+#pragma unroll
+        for (int j0 = 0; j0 < NOUT; j0++) store(line, q + 64 * j0, a[brev_c(j0, 3)], p[j0]);
+    }
+}
+template <typename C, bool INV, bool PAD_IN, bool CROP_OUT, bool LF1, bool LF3, class LoadF, class PreF, class StoreF,
+          class OffF>
+G2_D void fft512(C *sm, int nl, int lg_nl, const C *tw, LoadF load, PreF pre, StoreF store, OffF off)
+{
+    fft512_part<C, INV, PAD_IN, CROP_OUT, LF1, LF3>(sm, nl, lg_nl, tw, load, pre, store, off, (int)threadIdx.x,
+                                                    (int)blockDim.x, [] { __syncthreads(); });
 }
 
 // The whole CTA transforms its line block.

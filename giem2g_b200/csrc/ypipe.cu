@@ -199,6 +199,9 @@ __global__ void __launch_bounds__(CfgY<R, L, NZ, NP, SL, NG, NSTAGE, PK, NFW, NL
                 C2 *col = U1 + (size_t)kx * Ny * ZL + zl0;
                 C2 *spec = Uh + (size_t)q * Ny * 4 * ZL + sx * 2 * ZL + zl0;
                 auto off = [&](int t2, int n1, int k2) { return t2 + NL * (n1 + Cfg::N1 * k2); };
+                auto off512 = [&](int t2, int n0, int k2) { return t2 + NL * (n0 + 64 * k2); };
+                (void)off;
+                (void)off512;
                 if (fwd) {
                     auto load = [&](int t2, int yy) -> C2 { return col[yy * ZL + t2]; };
                     auto store = [&](int t2, int ky, C2 v) {
@@ -208,8 +211,13 @@ __global__ void __launch_bounds__(CfgY<R, L, NZ, NP, SL, NG, NSTAGE, PK, NFW, NL
                         else { r = 2 * Ny - ky; sy = 1; }
                         spec[(r * 4 + sy) * ZL + t2] = v;
                     };
-                    fft4step_part_ilp<C2, Cfg::N1, Cfg::N2, Cfg::IPT, false, true, false>(
-                        fsm, nl, Cfg::LG_NL, ftw, load, store, off, ftid, Cfg::NF, fsync);
+                    if constexpr (L == 512)
+                        fft512_part<C2, false, true, false, true, true>(
+                            fsm, nl, Cfg::LG_NL, ftw, load, [](int, int) { return 0; },
+                            [&](int t2, int ky, C2 v, int) { store(t2, ky, v); }, off512, ftid, Cfg::NF, fsync);
+                    else
+                        fft4step_part_ilp<C2, Cfg::N1, Cfg::N2, Cfg::IPT, false, true, false>(
+                            fsm, nl, Cfg::LG_NL, ftw, load, store, off, ftid, Cfg::NF, fsync);
                 } else {
                     auto load = [&](int t2, int ky) -> C2 {
                         int r, sy;
@@ -219,8 +227,13 @@ __global__ void __launch_bounds__(CfgY<R, L, NZ, NP, SL, NG, NSTAGE, PK, NFW, NL
                         return ld_l2(&spec[(r * 4 + sy) * ZL + t2]);
                     };
                     auto store = [&](int t2, int yy, C2 v) { col[yy * ZL + t2] = v; };
-                    fft4step_part_ilp<C2, Cfg::N1, Cfg::N2, Cfg::IPT, true, false, true>(
-                        fsm, nl, Cfg::LG_NL, ftw, load, store, off, ftid, Cfg::NF, fsync);
+                    if constexpr (L == 512)
+                        fft512_part<C2, true, false, true, true, true>(
+                            fsm, nl, Cfg::LG_NL, ftw, load, [](int, int) { return 0; },
+                            [&](int t2, int yy, C2 v, int) { store(t2, yy, v); }, off512, ftid, Cfg::NF, fsync);
+                    else
+                        fft4step_part_ilp<C2, Cfg::N1, Cfg::N2, Cfg::IPT, true, false, true>(
+                            fsm, nl, Cfg::LG_NL, ftw, load, store, off, ftid, Cfg::NF, fsync);
                 }
             }
             if (fwd) __threadfence();
