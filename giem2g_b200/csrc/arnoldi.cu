@@ -6,45 +6,131 @@
 // for the whole step, reduces all partial sums of a pass itself (a fixed order, so the result does not depend on the
 // schedule) and takes the pass decision with the others.  blockIdx.y is the instance; the barrier joins the blocks of one
 // instance.  The launch is cooperative, so all blocks are resident; the waits are bounded (2 s, error code 51).
-// Whole solves, launches per sweep -> one launch: FP64 32x32x8 3.00 -> 2.66 ms, mixed pairs 64x64x16 9.75 -> 8.80 ms,
-// 128x128x32 75.3 -> 74.3 ms (bound by the sweeps' HBM and L2 traffic).
+// Whole solves, launches per sweep -> one launch with its barriers, the last scalar step beside the scaling and the scaling
+// four words at a time: FP64 32x32x8 3.31 -> 2.30 ms, mixed pairs 128x128x32 2 ms of 66 (bound by the sweeps' HBM and L2
+// traffic).
 #include <type_traits>
 #include "krylov_dev.cuh"
 
 namespace {
 
-// all blocks of an instance; bar[0] arrivals, bar[1] generation
+// All blocks of an instance.  Block 0 arrives with 2^31 - (n - 1), the others with 1: n arrivals flip the word's top bit
+// and leave the rest as it was, so nothing is reset and launches of any grid can follow one another.  One release, one
+// L2 round trip and an acquiring poll: about 2 k clocks with 48 blocks, where an arrival counter with a generation word
+// between full fences had taken 6.4-7.7 k, 3.5 us in each of the step's two or three barriers.
 G2_D bool grid_barrier(unsigned *bar, unsigned n, int *err)
 {
     __shared__ bool ok;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
         ok = true;
-        const unsigned gen = atomicAdd(bar + 1, 0u);  // cannot advance before this block arrives
-        __threadfence();
-        if (atomicAdd(bar, 1u) == n - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            volatile const unsigned *g = bar + 1;
-            unsigned long long t0 = 0, t1;
-            for (int spin = 0; *g == gen; spin++) {
-                if ((spin & 255) != 255) continue;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-                if (t0 == 0) t0 = t1;
-                if (t1 - t0 > 2000000000ull) {
-                    atomicCAS(err, 0, 51);
-                    ok = false;
-                    break;
-                }
+        const unsigned add = blockIdx.x == 0 ? 0x80000000u - (n - 1) : 1u;
+        unsigned old, cur;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(bar), "r"(add) : "memory");
+        unsigned long long t0 = 0, t1;
+        for (int spin = 0;; spin++) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(cur) : "l"(bar) : "memory");
+            if ((cur ^ old) & 0x80000000u) break;
+            if ((spin & 255) != 255) continue;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+            if (t0 == 0) t0 = t1;
+            if (t1 - t0 > 2000000000ull) {
+                atomicCAS(err, 0, 51);
+                ok = false;
+                break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return ok;
+}
+
+// end of Arnoldi step j (gmres.F90:283-326): column j of H from the summed dots hc, H(j+1,j) = ||w||, the rotations, the
+// Arnoldi misfit and the exit test, by the lanes of one warp; cs, sn, g and the scalars were fetched when the step began.
+struct Finish {
+    double cs[KMAX], bn;
+    double2 sn[KMAX], g[2];
+    int iter;
+};
+G2_D void finish_load(Finish &f, const Level &L, int j)
+{
+    const int t = threadIdx.x;
+    if (t < j) {
+        f.cs[t] = L.cs[t];
+        f.sn[t] = L.sn[t];
+    }
+    if (t >= 32 && t < 34) f.g[t - 32] = L.H[hix(j + t - 32, L.m, L.m)];
+    if (t == 64) f.bn = L.scal[S_BN];
+    if (t == 65) f.iter = L.flags[F_ITER];
+}
+G2_D void finish_step(Finish &f, double2 *hc, Level &L, int j, double nrm, double dloo, double tol)
+{
+    const int m = L.m, lane = threadIdx.x & 31;
+    const double dnormw = sqrt(nrm);
+    if (lane == 0) {
+        double2 h = hc[0];
+        for (int i = 0; i < j; i++) {
+            double2 nx = hc[i + 1];
+            zrot1(h, nx, f.cs[i], f.sn[i]);
+            hc[i] = h;
+            h = nx;
+        }
+        // netlib ZROTG of (h, ||w||); the second argument is real and not negative
+        double2 hn = make_double2(dnormw, 0.0), sn;
+        double c;
+        const double ah = cabs_(h);
+        if (ah == 0.0) {
+            c = 0.0;
+            sn = make_double2(1.0, 0.0);
+        } else {
+            const double scale = ah + dnormw, a1 = ah / scale, b1 = dnormw / scale, norm = scale * sqrt(a1 * a1 + b1 * b1);
+            const double2 alpha = cdivr(h, ah);
+            c = ah / norm;
+            sn = cdivr(make_double2(alpha.x * dnormw, alpha.y * dnormw), norm);
+        }
+        zrot1(f.g[0], f.g[1], c, sn);
+        zrot1(h, hn, c, sn);
+        hc[j] = h;
+        hc[j + 1] = make_double2(0.0, 0.0);
+        const double bea = cabs_(f.g[1]) / f.bn;
+        if (bea < tol || j + 1 >= m) L.flags[F_KRYLOV] = 0;
+        L.scal[S_BEA] = bea;
+        L.cs[j] = c;
+        L.sn[j] = sn;
+        L.H[hix(j, m, m)] = f.g[0];
+        L.H[hix(j + 1, m, m)] = f.g[1];
+        L.scal[S_NRM2] = nrm;
+        L.scal[S_DLOO] = dloo;
+        L.scal[S_DNORMW] = dnormw;
+        L.flags[F_ITER] = f.iter + 1;
+        L.flags[F_L] = j + 1;
+    }
+    __syncwarp();
+    for (int i = lane; i <= j + 1; i += 32) L.H[hix(i, j, m)] = hc[i];
+}
+
+// V_K = w / ||w||: rounds of U words per thread, loads first.  In block 0, where the first warp finishes the step
+// meanwhile, the other seven take its words too.
+template <typename T, typename F>
+G2_D void scale_rows(const T *w, T *v, size_t n, size_t S, F f)
+{
+    constexpr int U = 4;
+    const bool first = blockIdx.x == 0;
+    const size_t rows = (n + S - 1) / S, T0 = blockIdx.x * (size_t)kVT + threadIdx.x;
+    const size_t rounds = first ? (rows * kVT + kVT - 33) / (kVT - 32) : rows;
+    auto at = [&](size_t r) {
+        const size_t q = threadIdx.x - 32 + (kVT - 32) * r;
+        return first ? (q % kVT) + (q / kVT) * S : T0 + r * S;
+    };
+    for (size_t r = 0; r < rounds; r += U) {
+        T x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (at(r + u) < n) x[u] = w[at(r + u)];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (at(r + u) < n) v[at(r + u)] = f(x[u]);
+    }
 }
 
 template <typename C, int K>
@@ -58,7 +144,9 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
     constexpr int E = Wide<C>::E, j = K - 1;
     __shared__ double2 hs[KMAX + 1], hn[KMAX + 1], hsum[KMAX + 1];
     __shared__ double nrm;
+    __shared__ Finish fin;
     Level L = mm.L[y];
+    if (blockIdx.x == 0) finish_load(fin, L, j);
     C *V = mm.V[y], *w = mm.w[y];
     const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x;
     const size_t Nw = wide_words<C>(N, N), ldw = N / E;
@@ -115,7 +203,7 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
     }
     for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) dots_of(w[i], i);
     block_reduce_store_r<K, R>(ax, ay, mm.part[y]);
-    if (!grid_barrier(L.counter + 1, gridDim.x, err)) return;
+    if (!grid_barrier(L.bar, gridDim.x, err)) return;
     reduce_partials(mm.part[y], gridDim.x, K, hs, nullptr);
     if (threadIdx.x < K) hsum[threadIdx.x] = hs[threadIdx.x];
     __syncthreads();
@@ -169,7 +257,7 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
         }
         double2 *part = mm.part[y] + (p & 1) * set;  // the other set may still be read by a slower block
         block_reduce_store_r<K, R>(ax, ay, part);
-        if (!grid_barrier(L.counter + 1, gridDim.x, err)) return;
+        if (!grid_barrier(L.bar, gridDim.x, err)) return;
         reduce_partials(part, gridDim.x, K, hn, &nrm);
         // gmres.F90:277-280
         double dl = 0.0;
@@ -184,27 +272,16 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
         }
         __syncthreads();
     }
-    const double dnormw = sqrt(nrm), inv = 1.0 / dnormw;
-    // in the scaling every thread takes the words that it wrote
-    for (i = t0; HOLD && i < Nw; i += S) {
-        W x = ww[i];
+    // every block has read its gate, a flag that the step's end may clear: all of them passed the barriers above
+    if (blockIdx.x == 0 && threadIdx.x < 32) return finish_step(fin, hsum, L, j, nrm, dloo, tol);
+    const double inv = 1.0 / sqrt(nrm);
+    if (HOLD && Nw)
+        scale_rows(ww, reinterpret_cast<W *>(V) + (size_t)K * ldw, Nw, S, [&](W x) {
 #pragma unroll
-        for (int e = 0; e < E; e++) set_part(x, e, scaled(part_of(x, e), inv));
-        reinterpret_cast<W *>(V)[(size_t)K * ldw + i] = x;
-    }
-    for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) V[(size_t)K * N + i] = scaled(w[i], inv);
-    if (blockIdx.x != 0) return;
-    // every block has read its gate, a flag that the step below may clear: all of them passed the barriers above
-    if (threadIdx.x < K) L.H[hix(threadIdx.x, j, L.m)] = hsum[threadIdx.x];
-    if (threadIdx.x == 0) {
-        L.scal[S_NRM2] = nrm;
-        L.scal[S_DLOO] = dloo;
-        L.scal[S_DNORMW] = dnormw;
-        L.flags[F_PASS] = 0;
-    }
-    __threadfence_block();
-    __syncthreads();
-    arnoldi_finish_body(L, j, tol);
+            for (int e = 0; e < E; e++) set_part(x, e, scaled(part_of(x, e), inv));
+            return x;
+        });
+    else scale_rows(w, V + (size_t)K * N, N, S, [&](C x) { return scaled(x, inv); });
 }
 
 int sms()

@@ -74,39 +74,34 @@ __global__ void __launch_bounds__(kVT) k_norm2_fused(const C *__restrict__ w, si
 G2_D double2 widen(float2 a) { return make_double2(a.x, a.y); }
 G2_D double2 widen(double2 a) { return a; }
 
-// ConstructCurrentSolution's triangular solve (gmres.F90:441-445): y = H(0:L,0:L)^-1 g.  The block stages the
-// L x L triangle and g in shared memory with one coalesced load; thread 0 then substitutes in the same order
-// as the single-thread loop it replaces, so y is bit-for-bit the same (a chain of dependent L2 loads had made
-// this 13 us per call).  Launch with kTriThreads threads.
-constexpr int kTriThreads = 128;
-__global__ void __launch_bounds__(kTriThreads) k_trisolve(Level L, const int *gate)
+// ConstructCurrentSolution's triangular solve (gmres.F90:441-445): y = H(0:L,0:L)^-1 g by one warp, lane i holding row
+// i's right side: each y_i found is taken off all rows above it at once.  (One thread going over the L^2/2 products took
+// 9.7 k clocks at L = 10.)
+__global__ void __launch_bounds__(32) k_trisolve(Level L, const int *gate)
 {
     pdl_wait();
     if (gate && *gate == 0) return;
-    __shared__ double2 Hs[KMAX * (KMAX + 1)];  // column j < n of the triangle at j * KMAX, then g at n * KMAX
-    __shared__ double2 ys[KMAX];
-    const int m = L.m, n = L.flags[F_L];
-    for (int e = threadIdx.x; e < n * (n + 1); e += blockDim.x) {
-        const int i = e % n, j = e / n, col = j < n ? j : m;
-        Hs[i + j * KMAX] = L.H[hix(i, col, m)];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double2 *g = Hs + n * KMAX;
-        for (int i = n - 1; i >= 0; i--) {
-            double2 t = g[i];
-            for (int k = i + 1; k < n; k++) {
-                const double2 p = cmul_(Hs[i + k * KMAX], ys[k]);
-                t.x -= p.x;
-                t.y -= p.y;
-            }
-            const double2 d = Hs[i + i * KMAX];
-            const double den = d.x * d.x + d.y * d.y;
-            ys[i] = make_double2((t.x * d.x + t.y * d.y) / den, (t.y * d.x - t.x * d.y) / den);
+    __shared__ double2 Hs[KMAX * KMAX];  // column j < n of the triangle at j * KMAX
+    const int m = L.m, n = L.flags[F_L], lane = threadIdx.x;
+    for (int j = 0; j < n; j++)
+        if (lane <= j) Hs[lane + j * KMAX] = L.H[hix(lane, j, m)];
+    double2 t = make_double2(0.0, 0.0), d = make_double2(1.0, 0.0);
+    if (lane < n) t = L.H[hix(lane, m, m)];
+    __syncwarp();
+    if (lane < n) d = Hs[lane + lane * KMAX];
+    const double den = d.x * d.x + d.y * d.y;
+    for (int i = n - 1; i >= 0; i--) {
+        double2 y = make_double2((t.x * d.x + t.y * d.y) / den, (t.y * d.x - t.x * d.y) / den);  // lane i's is row i's
+        y.x = __shfl_sync(0xffffffffu, y.x, i);
+        y.y = __shfl_sync(0xffffffffu, y.y, i);
+        if (lane < i) {
+            const double2 p = cmul_(Hs[lane + i * KMAX], y);
+            t.x -= p.x;
+            t.y -= p.y;
+        } else if (lane == i) {
+            L.y[i] = y;
         }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) L.y[i] = ys[i];
 }
 
 // start of a cycle: H(0,m) = beta, H(1..m, m) = 0, krylov active (gmres.F90:172-185)
@@ -130,7 +125,6 @@ __global__ void k_set_bn(Level L)
     L.flags[F_ITER] = 0;
     L.flags[F_KRYLOV] = L.flags[F_SOLVER];
     L.flags[F_L] = 0;
-    L.flags[F_PASS] = 0;
 }
 __global__ void k_set_beta(Level L, double tol)
 {
@@ -148,7 +142,7 @@ __global__ void k_zero_level(Level L)
     pdl_wait();
     const int n = (L.m + 1) * (L.m + 1);
     for (int i = threadIdx.x; i < n; i += blockDim.x) L.H[i] = make_double2(0.0, 0.0);
-    if (threadIdx.x == 0) L.counter[1] = 0u;  // a step that gave up at its barrier may have left arrivals
+    if (threadIdx.x == 0) *L.bar = 0u;  // a step that gave up at its barrier may have left arrivals
 }
 
 // restart (gmres.F90:369-376): beta = |g_m|, g <- inverse rotations of (0..0, g_m)
@@ -375,13 +369,12 @@ static int alloc_level(Level &L, int m)
     G2_CUDA_CHECK(cudaMalloc(&L.H, sizeof(double2) * (m + 1) * (m + 1)));
     G2_CUDA_CHECK(cudaMalloc(&L.cs, sizeof(double) * (m + 1)));
     G2_CUDA_CHECK(cudaMalloc(&L.sn, sizeof(double2) * (m + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&L.hpass, sizeof(double2) * (KMAX + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&L.hnext, sizeof(double2) * (KMAX + 1)));
     G2_CUDA_CHECK(cudaMalloc(&L.y, sizeof(double2) * (KMAX + 1)));
     G2_CUDA_CHECK(cudaMalloc(&L.scal, sizeof(double) * S_NSCAL));
     G2_CUDA_CHECK(cudaMalloc(&L.flags, sizeof(int) * F_NFLAGS));
-    G2_CUDA_CHECK(cudaMalloc(&L.counter, 3 * sizeof(unsigned)));
-    G2_CUDA_CHECK(cudaMemset(L.counter, 0, 3 * sizeof(unsigned)));
+    G2_CUDA_CHECK(cudaMalloc(&L.counter, 2 * sizeof(unsigned)));
+    G2_CUDA_CHECK(cudaMemset(L.counter, 0, 2 * sizeof(unsigned)));
+    L.bar = L.counter + 1;
     G2_CUDA_CHECK(cudaMemset(L.flags, 0, sizeof(int) * F_NFLAGS));
     G2_CUDA_CHECK(cudaMemset(L.scal, 0, sizeof(double) * S_NSCAL));
     // the solver's kernels run on non-blocking streams, which are not ordered after the legacy stream
@@ -390,7 +383,7 @@ static int alloc_level(Level &L, int m)
 }
 static void free_level(Level &L)
 {
-    void *p[] = {L.H, L.cs, L.sn, L.hpass, L.hnext, L.y, L.scal, L.flags, L.counter};
+    void *p[] = {L.H, L.cs, L.sn, L.y, L.scal, L.flags, L.counter};
     for (void *q : p)
         if (q) cudaFree(q);
     L = Level();
@@ -525,7 +518,7 @@ static int inner_solve(IeOp *op, KrylovWork *k, const CI *v, const CI *x0, CI *x
         if ((rc = arnoldi_step1<CI>(k, L, Vi, j, wi, tol, krylov, st))) return rc;
     }
     // FinalActions -> ConstructCurrentSolution (gmres.F90:423-458): x = x0 + V y
-    g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, solver); g2_count_launches(1);
+    g2_launch(k_trisolve, 1, 32, 0, st, L, solver); g2_count_launches(1);
     g2_launch(k_lincomb<CI, CI>, g, kVT, 0, st, x, 1.0, x, Vi, N, L.y, L.flags + F_L, N, solver); g2_count_launches(1);
     if (true_residual) {  // gmres.F90:402-419, result unused by the outer solver
         rc = apply_prec<CI>(op, x, ri, st, solver);
@@ -702,7 +695,7 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
         iter++;
         if (iter >= ctl.fgmres_maxit) break;
         // PrepareRestart: x += Z y; w = V g' (gmres.F90:333-379)
-        g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, nullptr); g2_count_launches(1);
+        g2_launch(k_trisolve, 1, 32, 0, st, L, nullptr); g2_count_launches(1);
         g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, Z, N, L.y, L.flags + F_L, N, nullptr); g2_count_launches(1);
         g2_launch(k_restart_g, 1, 1, 0, st, L); g2_count_launches(1);
         g2_launch(k_copy_g, 1, 64, 0, st, L); g2_count_launches(1);
@@ -711,7 +704,7 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
     }
     (void)L_used;
     // FinalActions (gmres.F90:382-421)
-    g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, nullptr); g2_count_launches(1);
+    g2_launch(k_trisolve, 1, 32, 0, st, L, nullptr); g2_count_launches(1);
     g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, Z, N, L.y, L.flags + F_L, N, nullptr); g2_count_launches(1);
     if ((rc = ie_apply_device64(op, k->x, k->r0, st))) return rc;
     k->applies64++;
@@ -805,7 +798,6 @@ __global__ void k_set_bn_masked(Level L, const int *outer_go)
     L.flags[F_ITER] = 0;
     L.flags[F_KRYLOV] = L.flags[F_SOLVER];
     L.flags[F_L] = 0;
-    L.flags[F_PASS] = 0;
 }
 
 }  // namespace
@@ -1024,7 +1016,7 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
         const int g = vec_grid(k->N);
         const int *solver = L.flags + F_SOLVER;
         CI *x = reinterpret_cast<CI *>(k->xin);
-        g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, solver); g2_count_launches(1);
+        g2_launch(k_trisolve, 1, 32, 0, st, L, solver); g2_count_launches(1);
         g2_launch(k_lincomb<CI, CI>, g, kVT, 0, st, x, 1.0, x, reinterpret_cast<const CI *>(k->Vi), k->N, L.y, L.flags + F_L,
                                              k->N, solver); g2_count_launches(1);
     }
@@ -1173,7 +1165,7 @@ static void batch_final_launch(BatchWork *b, int i, cudaStream_t st, int &rc)
     Level &L = k->Lo;
     const int g = vec_grid(k->N);
     CI *Z = reinterpret_cast<CI *>(k->Zo);
-    g2_launch(k_trisolve, 1, kTriThreads, 0, st, L, nullptr); g2_count_launches(1);
+    g2_launch(k_trisolve, 1, 32, 0, st, L, nullptr); g2_count_launches(1);
     g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, Z, k->N, L.y, L.flags + F_L, k->N, nullptr); g2_count_launches(1);
     if ((rc = ie_apply_device64(b->ops[i], k->x, k->r0, st))) return;
     k->applies64++;
@@ -1363,7 +1355,7 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                 b->h_active[i] = 0;
                 continue;
             }
-            g2_launch(k_trisolve, 1, kTriThreads, 0, st, k->Lo, nullptr); g2_count_launches(1);
+            g2_launch(k_trisolve, 1, 32, 0, st, k->Lo, nullptr); g2_count_launches(1);
             g2_launch(k_lincomb<double2, CI>, g, kVT, 0, st, k->x, 1.0, k->x, reinterpret_cast<const CI *>(k->Zo), k->N,
                                                       k->Lo.y, k->Lo.flags + F_L, k->N, nullptr); g2_count_launches(1);
             g2_launch(k_restart_g, 1, 1, 0, st, k->Lo); g2_count_launches(1);

@@ -9,12 +9,11 @@ struct Level {
     double2 *H = nullptr;   // (m+1) x (m+1) column-major, column m holds g
     double *cs = nullptr;
     double2 *sn = nullptr;
-    double2 *hpass = nullptr, *hnext = nullptr, *y = nullptr;
+    double2 *y = nullptr;
     double *scal = nullptr;
     int *flags = nullptr;
-    // [0] blocks done, for the last-block reductions (back to 0 after each use); [1], [2] arrivals and generation of
-    // the grid barrier of arnoldi.cu
-    unsigned *counter = nullptr;
+    unsigned *counter = nullptr;  // blocks done, for the last-block reductions (back to 0 after each use)
+    unsigned *bar = nullptr;      // the grid barrier of arnoldi.cu
 };
 
 // Several instances of one batch in one launch (blockIdx.y = instance): vectors of one length, and per instance its
@@ -42,7 +41,7 @@ constexpr double ZERO_THRESHOLD = 1e-14;  // gmres.F90:21
 constexpr int N_IGS = 3;                  // gmres.F90:22
 constexpr double kHookGain = 0.5;         // an outer step through the hook must halve the misfit
 
-enum { F_KRYLOV = 0, F_PASS = 1, F_L = 2, F_ITER = 3, F_SOLVER = 4, F_NFLAGS = 8 };
+enum { F_KRYLOV = 0, F_L = 2, F_ITER = 3, F_SOLVER = 4, F_NFLAGS = 8 };
 enum { S_BN = 0, S_BETA = 1, S_DNORMW = 2, S_DLOO = 3, S_BEA = 4, S_NRM2 = 5, S_NSCAL = 8 };
 
 G2_HD int hix(int i, int j, int m) { return i + j * (m + 1); }
@@ -135,65 +134,6 @@ G2_D void zrot1(double2 &cx, double2 &cy, double c, double2 s)
     cy = make_double2(c * cy.x - (sc.x * cx.x - sc.y * cx.y), c * cy.y - (sc.x * cx.y + sc.y * cx.x));
     cx = t;
 }
-// netlib ZROTG
-G2_D void zrotg(double2 &ca, double2 cb, double &c, double2 &s)
-{
-    const double aca = cabs_(ca);
-    if (aca == 0.0) {
-        c = 0.0;
-        s = make_double2(1.0, 0.0);
-        ca = cb;
-    } else {
-        const double scale = aca + cabs_(cb);
-        const double a1 = cabs_(cdivr(ca, scale)), b1 = cabs_(cdivr(cb, scale));
-        const double norm = scale * sqrt(a1 * a1 + b1 * b1);
-        const double2 alpha = cdivr(ca, aca);
-        c = aca / norm;
-        s = cdivr(cmul_(alpha, make_double2(cb.x, -cb.y)), norm);
-        ca = make_double2(alpha.x * norm, alpha.y * norm);
-    }
-}
-
-// end of Arnoldi step j (gmres.F90:283-326): H(j+1,j), rotations, Arnoldi misfit, exit test
-G2_D void arnoldi_finish_body(Level &L, int j, double tol)
-{
-    // run by every thread of one block: column j of H, the rotations so far and g(j), g(j+1) are staged in
-    // shared memory with one round of loads; thread 0 then applies the same operations in the same order
-    // as a single thread on global memory would (a chain of dependent L2 loads otherwise)
-    __shared__ double2 hc[KMAX + 1], sn_s[KMAX], gs[2];
-    __shared__ double cs_s[KMAX];
-    const int m = L.m;
-    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) hc[i] = L.H[hix(i, j, m)];
-    for (int i = threadIdx.x; i < j; i += blockDim.x) {
-        cs_s[i] = L.cs[i];
-        sn_s[i] = L.sn[i];
-    }
-    if (threadIdx.x < 2) gs[threadIdx.x] = L.H[hix(j + threadIdx.x, m, m)];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const double dnormw = L.scal[S_DNORMW], bn = L.scal[S_BN];
-        hc[j + 1] = make_double2(dnormw, 0.0);
-        for (int i = 0; i < j; i++) zrot1(hc[i], hc[i + 1], cs_s[i], sn_s[i]);
-        double2 h1 = hc[j], sn;
-        double c;
-        zrotg(h1, hc[j + 1], c, sn);
-        zrot1(gs[0], gs[1], c, sn);
-        zrot1(hc[j], hc[j + 1], c, sn);
-        hc[j + 1] = make_double2(0.0, 0.0);
-        L.cs[j] = c;
-        L.sn[j] = sn;
-        L.H[hix(j, m, m)] = gs[0];
-        L.H[hix(j + 1, m, m)] = gs[1];
-        const double bea = cabs_(gs[1]) / bn;
-        L.scal[S_BEA] = bea;
-        L.flags[F_ITER] += 1;
-        L.flags[F_L] = j + 1;
-        if (bea < tol || j + 1 >= m) L.flags[F_KRYLOV] = 0;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) L.H[hix(i, j, m)] = hc[i];
-}
-
 // ---- fused reductions: the last block to finish sums every block's partials ----------------------
 // Each block stores its partials, then counts itself done; the block that counts last reduces all
 // partials in a fixed order (lane-strided sums, shuffle tree: the result does not depend on which block
@@ -208,12 +148,12 @@ G2_D bool last_block(unsigned *counter)
     if (threadIdx.x == 0) am_last = atomicAdd(counter, 1u) == gridDim.x - 1;
     __syncthreads();
     if (am_last && threadIdx.x == 0) *counter = 0u;
+    __threadfence();
     return am_last;
 }
-// sums of part[b][col] over blocks for columns 0..K-1 into h[], and of column KMAX into *nrm (one block)
+// (after a barrier or last_block, which order the loads) sums of part[b][col] over blocks for columns 0..K-1 into h[], and of column KMAX into *nrm (one block)
 G2_D void reduce_partials(const double2 *part, int nb, int K, double2 *h, double *nrm)
 {
-    __threadfence();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int k = warp; k <= K; k += nw) {
         const int col = (k == K) ? KMAX : k;
