@@ -10,6 +10,7 @@
 // four words at a time: FP64 32x32x8 3.31 -> 2.30 ms, mixed pairs 128x128x32 2 ms of 66 (bound by the sweeps' HBM and L2
 // traffic).
 #include <type_traits>
+#include <utility>
 #include "krylov_dev.cuh"
 
 namespace {
@@ -109,13 +110,13 @@ G2_D void finish_step(Finish &f, double2 *hc, Level &L, int j, double nrm, doubl
     for (int i = lane; i <= j + 1; i += 32) L.H[hix(i, j, m)] = hc[i];
 }
 
-// V_K = w / ||w||: rounds of U words per thread, loads first.  In block 0, where the first warp finishes the step
-// meanwhile, the other seven take its words too.
-template <typename T, typename F>
+// v = f(w): rounds of U words per thread, loads first.  FIN: in block 0, where the first warp finishes the step meanwhile,
+// the other seven take its words too.
+template <bool FIN, typename T, typename F>
 G2_D void scale_rows(const T *w, T *v, size_t n, size_t S, F f)
 {
     constexpr int U = 4;
-    const bool first = blockIdx.x == 0;
+    const bool first = FIN && blockIdx.x == 0;
     const size_t rows = (n + S - 1) / S, T0 = blockIdx.x * (size_t)kVT + threadIdx.x;
     const size_t rounds = first ? (rows * kVT + kVT - 33) / (kVT - 32) : rows;
     auto at = [&](size_t r) {
@@ -276,12 +277,138 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
     if (blockIdx.x == 0 && threadIdx.x < 32) return finish_step(fin, hsum, L, j, nrm, dloo, tol);
     const double inv = 1.0 / sqrt(nrm);
     if (HOLD && Nw)
-        scale_rows(ww, reinterpret_cast<W *>(V) + (size_t)K * ldw, Nw, S, [&](W x) {
+        scale_rows<true>(ww, reinterpret_cast<W *>(V) + (size_t)K * ldw, Nw, S, [&](W x) {
 #pragma unroll
             for (int e = 0; e < E; e++) set_part(x, e, scaled(part_of(x, e), inv));
             return x;
         });
-    else scale_rows(w, V + (size_t)K * N, N, S, [&](C x) { return scaled(x, inv); });
+    else scale_rows<true>(w, V + (size_t)K * N, N, S, [&](C x) { return scaled(x, inv); });
+}
+
+// ---- start of an inner cycle -----------------------------------------------------------------------
+// Two launches, one before and one after the apply that forms A x0, where a launch per operation (reset, norm, scalars,
+// copy; difference, norm, scalars, column g, scaling) had taken nine of 2-4 us each on a small grid.  Words, sums and
+// their order are those of k_norm2_fused.
+template <typename C>
+__global__ void __launch_bounds__(kVT) k_begin(Starts<C> s, size_t N, int *err)
+{
+    pdl_wait();
+    using R = typename RealOf<C>::T;
+    using W = typename Wide<C>::T;
+    constexpr int E = Wide<C>::E, U = 4;
+    const int y = blockIdx.y;
+    Level L = s.L[y];
+    const C *v = s.v[y], *x0 = s.x0[y];
+    C *x = s.x[y];
+    const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x, Nw = wide_words<C>(N, N);
+    R ax[1] = {R(0)}, ay[1] = {R(0)};
+    const W *vw = reinterpret_cast<const W *>(v);
+    for (size_t i = t0; i < Nw; i += U * S) {
+        W a[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u * S < Nw) a[u] = vw[i + u * S];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u * S < Nw)
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const C c = part_of(a[u], e);
+                    ax[0] += c.x * c.x + c.y * c.y;
+                }
+    }
+    for (size_t i = Nw * E + t0; i < N; i += S) ax[0] += v[i].x * v[i].x + v[i].y * v[i].y;
+    block_reduce_store_r<0, R>(ax, ay, s.part[y]);
+    if (!grid_barrier(L.bar, gridDim.x, err)) return;
+    __shared__ double nrm;
+    reduce_partials(s.part[y], gridDim.x, 0, nullptr, &nrm);
+    const double bn = sqrt(nrm);
+    const bool zero = bn < ZERO_THRESHOLD;
+    const W *xw = reinterpret_cast<const W *>(x0);
+    for (size_t i = t0; i < Nw; i += U * S) {
+        W a[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u * S < Nw) a[u] = zero ? W() : xw[i + u * S];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u * S < Nw) reinterpret_cast<W *>(x)[i + u * S] = a[u];
+    }
+    for (size_t i = Nw * E + t0; i < N; i += S) x[i] = zero ? C() : x0[i];
+    if (blockIdx.x != 0) return;
+    for (int i = threadIdx.x; i < (L.m + 1) * (L.m + 1); i += kVT) L.H[i] = make_double2(0.0, 0.0);
+    if (threadIdx.x == 0) {
+        L.scal[S_NRM2] = nrm;
+        L.scal[S_BN] = bn;
+        L.flags[F_SOLVER] = L.flags[F_KRYLOV] = zero || (s.go[y] && *s.go[y] == 0) ? 0 : 1;
+        L.flags[F_ITER] = 0;
+        L.flags[F_L] = 0;
+    }
+}
+
+template <typename C>
+__global__ void __launch_bounds__(kVT) k_residual(Starts<C> s, size_t N, double tol, int *err)
+{
+    pdl_wait();
+    using R = typename RealOf<C>::T;
+    using W = typename Wide<C>::T;
+    constexpr int E = Wide<C>::E, U = 4;
+    const int y = blockIdx.y;
+    Level L = s.L[y];
+    if (L.flags[F_SOLVER] == 0) return;
+    const double bn = L.scal[S_BN];
+    const C *v = s.v[y];
+    C *r = s.r[y];
+    const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x, Nw = wide_words<C>(N, N);
+    R ax[1] = {R(0)}, ay[1] = {R(0)};
+    auto diff = [&](C b, C a) {
+        b.x -= a.x;
+        b.y -= a.y;
+        ax[0] += b.x * b.x + b.y * b.y;
+        return b;
+    };
+    const W *vw = reinterpret_cast<const W *>(v);
+    W *rw = reinterpret_cast<W *>(r);
+    for (size_t i = t0; i < Nw; i += U * S) {
+        W a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u * S < Nw) {
+                a[u] = rw[i + u * S];
+                b[u] = vw[i + u * S];
+            }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i + u * S < Nw) {
+#pragma unroll
+                for (int e = 0; e < E; e++) set_part(a[u], e, diff(part_of(b[u], e), part_of(a[u], e)));
+                rw[i + u * S] = a[u];
+            }
+    }
+    for (size_t i = Nw * E + t0; i < N; i += S) r[i] = diff(v[i], r[i]);
+    block_reduce_store_r<0, R>(ax, ay, s.part[y]);
+    if (!grid_barrier(L.bar, gridDim.x, err)) return;
+    __shared__ double nrm;
+    reduce_partials(s.part[y], gridDim.x, 0, nullptr, &nrm);
+    const double beta = sqrt(nrm), inv = 1.0 / beta;
+    const bool done = beta / bn < tol;
+    if (!done && Nw)
+        scale_rows<false>(rw, reinterpret_cast<W *>(s.V[y]), Nw, S, [&](W a) {
+#pragma unroll
+            for (int e = 0; e < E; e++) set_part(a, e, scaled(part_of(a, e), inv));
+            return a;
+        });
+    else if (!done) scale_rows<false>(r, s.V[y], N, S, [&](C a) { return scaled(a, inv); });
+    if (blockIdx.x != 0) return;
+    const int m = L.m;
+    if (!done && threadIdx.x <= m) L.H[hix(threadIdx.x, m, m)] = make_double2(threadIdx.x ? 0.0 : beta, 0.0);
+    if (threadIdx.x == 0) {
+        L.scal[S_NRM2] = nrm;
+        L.scal[S_BETA] = beta;
+        if (done) L.flags[F_SOLVER] = 0;
+        L.flags[F_KRYLOV] = done ? 0 : 1;
+        L.flags[F_L] = 0;
+    }
 }
 
 int sms()
@@ -295,14 +422,11 @@ int sms()
     return n;
 }
 
-template <typename C, int K>
-int launch(const Multi<C> &mm, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st)
+// a cooperative launch of `kernel` for n instances: as many blocks each as are resident together, up to nparts
+template <typename... P, typename... A>
+int launch(void (*kernel)(P...), int per_sm, size_t words, int n, int nparts, cudaStream_t st, A &&...args)
 {
-    static const int per_sm = [] {
-        int b = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_arnoldi<C, K>, kVT, 0) == cudaSuccess && b > 0 ? b : 1;
-    }();
-    const size_t words = N / Wide<C>::E + 1, need = (words + kVT - 1) / kVT;
+    const size_t need = (words + kVT - 1) / kVT;
     int g = per_sm * sms() / n;
     g = g < nparts ? g : nparts;
     g = (size_t)g < need ? g : (int)need;
@@ -315,15 +439,28 @@ int launch(const Multi<C> &mm, int n, size_t N, int nparts, double tol, int *err
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    G2_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_arnoldi<C, K>, mm, N, tol, err));
+    G2_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+    g2_count_launches(1);
     return G2_OK;
+}
+template <typename F>
+int per_sm_of(F kernel)
+{
+    int b = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kVT, 0) == cudaSuccess && b > 0 ? b : 1;
+}
+template <typename C, int K>
+int launch_step(const Multi<C> &mm, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st)
+{
+    static const int per_sm = per_sm_of(k_arnoldi<C, K>);
+    return launch(k_arnoldi<C, K>, per_sm, N / Wide<C>::E + 1, n, nparts, st, mm, N, tol, err);
 }
 template <typename C>
 int dispatch(const Multi<C> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
 {
     switch (j + 1) {
 #define G2_K(k) \
-    case k: return launch<C, k>(mm, n, N, nparts, tol, err, st)
+    case k: return launch_step<C, k>(mm, n, N, nparts, tol, err, st)
         G2_K(1);
         G2_K(2);
         G2_K(3);
@@ -370,3 +507,19 @@ int arnoldi_step(const Multi<double2> &mm, int n, size_t N, int nparts, int j, d
 {
     return dispatch(mm, n, N, nparts, j, tol, err, st);
 }
+
+template <typename C> int krylov_begin(const Starts<C> &s, int n, size_t N, int nparts, int *err, cudaStream_t st)
+{
+    static const int per_sm = per_sm_of(k_begin<C>);
+    return launch(k_begin<C>, per_sm, N / Wide<C>::E + 1, n, nparts, st, s, N, err);
+}
+template <typename C>
+int krylov_residual(const Starts<C> &s, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st)
+{
+    static const int per_sm = per_sm_of(k_residual<C>);
+    return launch(k_residual<C>, per_sm, N / Wide<C>::E + 1, n, nparts, st, s, N, tol, err);
+}
+template int krylov_begin(const Starts<float2> &, int, size_t, int, int *, cudaStream_t);
+template int krylov_begin(const Starts<double2> &, int, size_t, int, int *, cudaStream_t);
+template int krylov_residual(const Starts<float2> &, int, size_t, int, double, int *, cudaStream_t);
+template int krylov_residual(const Starts<double2> &, int, size_t, int, double, int *, cudaStream_t);

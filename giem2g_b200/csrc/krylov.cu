@@ -137,12 +137,12 @@ __global__ void k_set_beta(Level L, double tol)
         L.flags[F_KRYLOV] = 0;
     }
 }
-__global__ void k_zero_level(Level L)
+__global__ void k_zero_level(Level L, unsigned *bar_inner)
 {
     pdl_wait();
     const int n = (L.m + 1) * (L.m + 1);
     for (int i = threadIdx.x; i < n; i += blockDim.x) L.H[i] = make_double2(0.0, 0.0);
-    if (threadIdx.x == 0) *L.bar = 0u;  // a step that gave up at its barrier may have left arrivals
+    if (threadIdx.x == 0) *L.bar = *bar_inner = 0u;  // a step that gave up at its barrier may have left arrivals
 }
 
 // restart (gmres.F90:369-376): beta = |g_m|, g <- inverse rotations of (0..0, g_m)
@@ -189,15 +189,6 @@ __global__ void __launch_bounds__(kVT) k_axpby(CO *out, double a, const CX *x, d
         for (int u = 0; u < kILP; u++) st2(out, i + u * S, elem(xv[u], yv[u]));
     }
     for (; i < N; i += S) st2(out, i, elem(ld2(x, i), y ? ld2(y, i) : make_double2(0.0, 0.0)));
-}
-// x = v, or x = 0 when ||v|| < ZERO_THRESHOLD (gmres.F90:139-145)
-template <typename C>
-__global__ void __launch_bounds__(kVT) k_copy_or_zero(C *x, const C *v, const double *scal, size_t N)
-{
-    pdl_wait();
-    const bool zero = scal[S_BN] < ZERO_THRESHOLD;
-    for (size_t i = blockIdx.x * (size_t)kVT + threadIdx.x; i < N; i += (size_t)gridDim.x * kVT)
-        st2(x, i, zero ? make_double2(0.0, 0.0) : ld2(v, i));
 }
 // v = w / scal[idx]
 template <typename C>
@@ -465,14 +456,12 @@ static int arnoldi_step1(KrylovWork *k, Level &L, C *V, int j, C *w, double tol,
     mm.part[0] = k->part;
     mm.L[0] = L;
     mm.gate[0] = gate;
-    g2_count_launches(1);
     return arnoldi_step(mm, 1, k->N, k->nparts, j, tol, k->err, st);
 }
 // the same for n lockstep instances (vector length N, nparts partial-sum slots each) in one launch
 template <typename C>
 static int arnoldi_step_multi(const Multi<C> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
 {
-    g2_count_launches(1);
     return arnoldi_step(mm, n, N, nparts, j, tol, err, st);
 }
 
@@ -496,19 +485,21 @@ static int inner_solve(IeOp *op, KrylovWork *k, const CI *v, const CI *x0, CI *x
     const int g = vec_grid(N);
     CI *Vi = reinterpret_cast<CI *>(k->Vi), *ri = reinterpret_cast<CI *>(k->ri), *wi = reinterpret_cast<CI *>(k->wi);
     const int *solver = L.flags + F_SOLVER, *krylov = L.flags + F_KRYLOV;
-    g2_launch(k_zero_level, 1, 256, 0, st, L); g2_count_launches(1);
-    norm2<CI>(k, v, L.scal + S_NRM2, nullptr, st);
-    g2_launch(k_set_bn, 1, 1, 0, st, L); g2_count_launches(1);
-    g2_launch(k_copy_or_zero<CI>, g, kVT, 0, st, x, x0, L.scal, N);  // x = x0, or 0 when ||b|| < 1e-14
-    int rc = apply_prec<CI>(op, x0, ri, st, solver);
+    Starts<CI> s{};
+    s.v[0] = v;
+    s.x0[0] = x0;
+    s.x[0] = x;
+    s.r[0] = ri;
+    s.V[0] = Vi;
+    s.part[0] = k->part;
+    s.L[0] = L;
+    int rc = krylov_begin(s, 1, N, k->nparts, k->err, st);
+    if (rc) return rc;
+    rc = apply_prec<CI>(op, x0, ri, st, solver);
     if (rc) return rc;
     k->applies32 += sizeof(CI) == 8 ? 1 : 0;
     k->applies64 += sizeof(CI) == 16 ? 1 : 0;
-    g2_launch(k_axpby<CI, CI, CI>, g, kVT, 0, st, ri, 1.0, v, -1.0, ri, N, solver);  // r0 = b - A x0
-    norm2<CI>(k, ri, L.scal + S_NRM2, solver, st);
-    g2_launch(k_set_beta, 1, 1, 0, st, L, tol); g2_count_launches(1);
-    g2_launch(k_cycle_start, 1, 1, 0, st, L, solver); g2_count_launches(1);
-    g2_launch(k_scale_by<CI>, g, kVT, 0, st, Vi, ri, L.scal, S_BETA, N, solver); g2_count_launches(1);
+    if ((rc = krylov_residual(s, 1, N, k->nparts, tol, k->err, st))) return rc;
     for (int j = 0; j < k->mi; j++) {
         CI *Vj = Vi + (size_t)j * N;
         rc = apply_prec<CI>(op, Vj, wi, st, krylov);
@@ -611,7 +602,7 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
     info->bea = -1.0;
     info->be = -1.0;
     // gmres.F90:129-168
-    g2_launch(k_zero_level, 1, 256, 0, st, L); g2_count_launches(1);
+    g2_launch(k_zero_level, 1, 256, 0, st, L, k->Li.bar); g2_count_launches(1);
     norm2<double2>(k, k->b, L.scal + S_NRM2, nullptr, st);
     g2_launch(k_set_bn, 1, 1, 0, st, L); g2_count_launches(1);
     int rc = pull();
@@ -785,23 +776,6 @@ int krylov_history(IeOp *op, double *out, int max_len)
 // the launch sequence of the single solve, so its iterates, iteration count and status are those of a
 // solve on its own.  Converged instances are masked: their inner-cycle kernels are gated off through a
 // device flag and the host stops launching their outer work.
-namespace {
-
-// outer_go: the instance's outer Krylov flag (F_KRYLOV of its outer level); an inner cycle enqueued after the
-// instance converged (one outer step ahead of the host, see batch_outer) does nothing.  (Masked instances
-// launch nothing: each mask has its own captured cycle.)
-__global__ void k_set_bn_masked(Level L, const int *outer_go)
-{
-    pdl_wait();
-    L.scal[S_BN] = sqrt(L.scal[S_NRM2]);
-    L.flags[F_SOLVER] = (L.scal[S_BN] < ZERO_THRESHOLD || *outer_go == 0) ? 0 : 1;
-    L.flags[F_ITER] = 0;
-    L.flags[F_KRYLOV] = L.flags[F_SOLVER];
-    L.flags[F_L] = 0;
-}
-
-}  // namespace
-
 struct BatchGroup {
     IeOp *op = nullptr;
     int first = 0, n = 0;  // instances first .. first+n-1 (n = 1 or 2)
@@ -935,34 +909,42 @@ template <typename CI>
 static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
 {
     const int n = b->n;
-    for (int i = 0; i < n; i++) {
-        if (!b->h_active[i]) continue;
-        KrylovWork *k = b->k[i];
-        Level &L = k->Li;
-        const int g = vec_grid(k->N);
-        g2_launch(k_zero_level, 1, 256, 0, st, L); g2_count_launches(1);
-        norm2<CI>(k, reinterpret_cast<const CI *>(k->vin), L.scal + S_NRM2, nullptr, st);
-        g2_launch(k_set_bn_masked, 1, 1, 0, st, L, k->Lo.flags + F_KRYLOV); g2_count_launches(1);
-        g2_launch(k_copy_or_zero<CI>, g, kVT, 0, st, reinterpret_cast<CI *>(k->xin), reinterpret_cast<const CI *>(k->vin),
-                                             L.scal, k->N); g2_count_launches(1);
-    }
+    // f on runs of up to KMI active instances of one vector length
+    auto starts_of = [&](auto f) -> int {
+        std::vector<int> act;
+        for (int i = 0; i < n; i++)
+            if (b->h_active[i]) act.push_back(i);
+        for (size_t c = 0; c < act.size();) {
+            KrylovWork *k0 = b->k[act[c]];
+            Starts<CI> s{};
+            int q = 0;
+            for (; c < act.size() && q < KMI; c++, q++) {
+                KrylovWork *k = b->k[act[c]];
+                if (k->N != k0->N || k->nparts != k0->nparts) break;
+                s.v[q] = s.x0[q] = reinterpret_cast<const CI *>(k->vin);
+                s.x[q] = reinterpret_cast<CI *>(k->xin);
+                s.r[q] = reinterpret_cast<CI *>(k->ri);
+                s.V[q] = reinterpret_cast<CI *>(k->Vi);
+                s.part[q] = k->part;
+                s.L[q] = k->Li;
+                // a cycle enqueued after its instance converged (one outer step ahead of the host, see batch_outer)
+                // does nothing; masked instances launch nothing, as each mask has its own captured cycle
+                s.go[q] = k->Lo.flags + F_KRYLOV;
+            }
+            if (const int r = f(s, q, k0)) return r;
+        }
+        return G2_OK;
+    };
+    int rc = starts_of([&](const Starts<CI> &s, int q, KrylovWork *k) { return krylov_begin(s, q, k->N, k->nparts, k->err, st); });
+    if (rc) return rc;
     auto vin = [&](int i) { return reinterpret_cast<const CI *>(b->k[i]->vin); };
     auto ri = [&](int i) { return reinterpret_cast<CI *>(b->k[i]->ri); };
-    int rc = batch_apply<CI>(b, vin, ri, F_SOLVER, st);
+    rc = batch_apply<CI>(b, vin, ri, F_SOLVER, st);
     if (rc) return rc;
-    for (int i = 0; i < n; i++) {
-        if (!b->h_active[i]) continue;
-        KrylovWork *k = b->k[i];
-        Level &L = k->Li;
-        const int g = vec_grid(k->N);
-        const int *solver = L.flags + F_SOLVER;
-        CI *r = reinterpret_cast<CI *>(k->ri);
-        g2_launch(k_axpby<CI, CI, CI>, g, kVT, 0, st, r, 1.0, reinterpret_cast<const CI *>(k->vin), -1.0, r, k->N, solver); g2_count_launches(1);
-        norm2<CI>(k, r, L.scal + S_NRM2, solver, st);
-        g2_launch(k_set_beta, 1, 1, 0, st, L, tol); g2_count_launches(1);
-        g2_launch(k_cycle_start, 1, 1, 0, st, L, solver); g2_count_launches(1);
-        g2_launch(k_scale_by<CI>, g, kVT, 0, st, reinterpret_cast<CI *>(k->Vi), r, L.scal, S_BETA, k->N, solver); g2_count_launches(1);
-    }
+    rc = starts_of([&](const Starts<CI> &s, int q, KrylovWork *k) {
+        return krylov_residual(s, q, k->N, k->nparts, tol, k->err, st);
+    });
+    if (rc) return rc;
     // Arnoldi step j of the active instances in `act`: runs of up to KMI instances with the same vector length
     // share each launch (each instance keeps its own blocks, partials and gates)
     auto arnoldi_of = [&](const std::vector<int> &act, int j) -> int {
@@ -1197,7 +1179,7 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
         KrylovWork *k = b->k[i];
         const int g = vec_grid(k->N);
         const int *solver = k->Lo.flags + F_SOLVER;
-        g2_launch(k_zero_level, 1, 256, 0, st, k->Lo); g2_count_launches(1);
+        g2_launch(k_zero_level, 1, 256, 0, st, k->Lo, k->Li.bar); g2_count_launches(1);
         norm2<double2>(k, k->b, k->Lo.scal + S_NRM2, nullptr, st);
         g2_launch(k_set_bn, 1, 1, 0, st, k->Lo); g2_count_launches(1);
         if ((rc = ie_apply_device64(b->ops[i], k->x, k->r0, st, solver))) return rc;

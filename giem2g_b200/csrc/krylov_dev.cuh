@@ -32,6 +32,22 @@ struct Multi {
 int arnoldi_step(const Multi<float2> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st);
 int arnoldi_step(const Multi<double2> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st);
 
+// The inner cycles of several instances that start together: v right side, x0 start (x: the copy the cycle's solution is
+// added to), r = A x0 on entry of krylov_residual, V the basis.  go: 0 makes the instance's cycle do nothing.
+template <typename C>
+struct Starts {
+    const C *v[KMI], *x0[KMI];
+    C *x[KMI], *r[KMI], *V[KMI];
+    double2 *part[KMI];
+    Level L[KMI];
+    const int *go[KMI];
+};
+// arnoldi.cu: bn = ||v||, x = x0 (0 where bn vanishes), the level's flags and H reset (gmres.F90:129-145)
+template <typename C> int krylov_begin(const Starts<C> &s, int n, size_t N, int nparts, int *err, cudaStream_t st);
+// r = v - r, beta = ||r||, exit or V_0 = r / beta and a started cycle (gmres.F90:147-185)
+template <typename C>
+int krylov_residual(const Starts<C> &s, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st);
+
 namespace {
 
 constexpr int kVT = 256;   // threads of the vector kernels
