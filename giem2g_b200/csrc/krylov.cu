@@ -280,6 +280,19 @@ __global__ void k_copy_g(Level L)
     for (int i = threadIdx.x; i <= m; i += blockDim.x) L.y[i] = L.H[hix(i, m, m)];
 }
 
+// a level's scalars and the operator's error word into pinned host memory: one launch before the host's wait, where three
+// copies to pageable memory had cost about 20 us in each outer step of a small solve
+struct Report {
+    double scal[S_NSCAL];
+    int err;
+};
+__global__ void k_report(Level L, const int *err, Report *out)
+{
+    pdl_wait();
+    if (threadIdx.x < S_NSCAL) out->scal[threadIdx.x] = L.scal[threadIdx.x];
+    if (threadIdx.x == 0) out->err = *err;
+}
+
 // SolveEquation helpers (ie_solver_module.F90:64-97); vectors are [c][cell], cell = z*NxNy + y*Nx + x
 __global__ void k_rhs(double2 *rhs, const double2 *Ebkg, const double *post, size_t plane, int Nz)
 {
@@ -349,35 +362,35 @@ struct KrylovWork {
     double2 *part = nullptr;  // partial sums of a sweep, two sets
     int nparts = 0;
     int *err = nullptr;       // the operator's device error word
+    void *mem = nullptr;      // all device buffers
+    Report *report = nullptr;  // pinned; allocated by the first solve of its own (a batch has one for all instances)
     std::vector<double> history;
     int applies64 = 0, applies32 = 0;
     int hook_steps = 0;  // outer steps preconditioned through the hook in the last solve
 };
 
-static int alloc_level(Level &L, int m)
+// Pieces of one allocation, 256 bytes apart: without a base only their total is counted.  (The 28 buffers of a solve, each
+// allocated on its own, took 3-4 ms of a new operator's first solve.)
+struct Slab {
+    char *base = nullptr;
+    size_t used = 0;
+    template <typename T> void take(T *&p, size_t bytes)
+    {
+        p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (bytes + 255) / 256 * 256;
+    }
+};
+static void place_level(Level &L, int m, Slab &s)
 {
     L.m = m;
-    G2_CUDA_CHECK(cudaMalloc(&L.H, sizeof(double2) * (m + 1) * (m + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&L.cs, sizeof(double) * (m + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&L.sn, sizeof(double2) * (m + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&L.y, sizeof(double2) * (KMAX + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&L.scal, sizeof(double) * S_NSCAL));
-    G2_CUDA_CHECK(cudaMalloc(&L.flags, sizeof(int) * F_NFLAGS));
-    G2_CUDA_CHECK(cudaMalloc(&L.counter, 2 * sizeof(unsigned)));
-    G2_CUDA_CHECK(cudaMemset(L.counter, 0, 2 * sizeof(unsigned)));
-    L.bar = L.counter + 1;
-    G2_CUDA_CHECK(cudaMemset(L.flags, 0, sizeof(int) * F_NFLAGS));
-    G2_CUDA_CHECK(cudaMemset(L.scal, 0, sizeof(double) * S_NSCAL));
-    // the solver's kernels run on non-blocking streams, which are not ordered after the legacy stream
-    G2_CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy));
-    return G2_OK;
-}
-static void free_level(Level &L)
-{
-    void *p[] = {L.H, L.cs, L.sn, L.y, L.scal, L.flags, L.counter};
-    for (void *q : p)
-        if (q) cudaFree(q);
-    L = Level();
+    s.take(L.H, sizeof(double2) * (m + 1) * (m + 1));
+    s.take(L.cs, sizeof(double) * (m + 1));
+    s.take(L.sn, sizeof(double2) * (m + 1));
+    s.take(L.y, sizeof(double2) * (KMAX + 1));
+    s.take(L.scal, sizeof(double) * S_NSCAL);
+    s.take(L.flags, sizeof(int) * F_NFLAGS);
+    s.take(L.counter, sizeof(unsigned));
+    s.take(L.bar, sizeof(unsigned));
 }
 
 static void kw_free(KrylovWork *k)
@@ -385,11 +398,8 @@ static void kw_free(KrylovWork *k)
     if (!k) return;
     for (int q = 0; q < 2; q++)
         if (k->inner_exec[q]) cudaGraphExecDestroy(k->inner_exec[q]);
-    void *p[] = {k->Vo, k->x, k->b, k->r0, k->w, k->tmp, k->Zo, k->Vi, k->ri, k->wi, k->vin, k->xin, k->part, k->x0in};
-    for (void *q : p)
-        if (q) cudaFree(q);
-    free_level(k->Lo);
-    free_level(k->Li);
+    if (k->mem) cudaFree(k->mem);
+    if (k->report) cudaFreeHost(k->report);
     delete k;
 }
 
@@ -407,24 +417,38 @@ static int kw_alloc(KrylovWork *k, size_t N, int mo, int mi, int precision)
     k->mi = mi;
     k->precision = precision;
     const size_t e64 = sizeof(double2), ei = precision ? sizeof(float2) : sizeof(double2);
-    G2_CUDA_CHECK(cudaMalloc(&k->Vo, e64 * N * (mo + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&k->x, e64 * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->b, e64 * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->r0, e64 * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->w, e64 * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->tmp, e64 * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->Zo, ei * N * mo));
-    G2_CUDA_CHECK(cudaMalloc(&k->Vi, ei * N * (mi + 1)));
-    G2_CUDA_CHECK(cudaMalloc(&k->ri, ei * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->wi, ei * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->vin, ei * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->xin, ei * N));
-    G2_CUDA_CHECK(cudaMalloc(&k->x0in, ei * N));
     k->nparts = sweep_grid(N);
-    G2_CUDA_CHECK(cudaMalloc(&k->part, 2 * sizeof(double2) * (size_t)k->nparts * (KMAX + 1)));
-    int rc = alloc_level(k->Lo, mo);
-    if (!rc) rc = alloc_level(k->Li, mi);
-    return rc;
+    Slab s;
+    for (int pass = 0; pass < 2; pass++) {
+        // the levels first: they are zeroed
+        s.used = 0;
+        place_level(k->Lo, mo, s);
+        place_level(k->Li, mi, s);
+        const size_t state = s.used;
+        s.take(k->Vo, e64 * N * (mo + 1));
+        s.take(k->x, e64 * N);
+        s.take(k->b, e64 * N);
+        s.take(k->r0, e64 * N);
+        s.take(k->w, e64 * N);
+        s.take(k->tmp, e64 * N);
+        s.take(k->Zo, ei * N * mo);
+        s.take(k->Vi, ei * N * (mi + 1));
+        s.take(k->ri, ei * N);
+        s.take(k->wi, ei * N);
+        s.take(k->vin, ei * N);
+        s.take(k->xin, ei * N);
+        s.take(k->x0in, ei * N);
+        s.take(k->part, 2 * sizeof(double2) * (size_t)k->nparts * (KMAX + 1));
+        if (pass) {
+            G2_CUDA_CHECK(cudaMemset(s.base, 0, state));
+        } else {
+            G2_CUDA_CHECK(cudaMalloc(&k->mem, s.used));
+            s.base = static_cast<char *>(k->mem);
+        }
+    }
+    // the solver's kernels run on non-blocking streams, which are not ordered after the legacy stream
+    G2_CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy));
+    return G2_OK;
 }
 
 static int krylov_alloc(IeOp *op, int mo, int mi, int precision)
@@ -435,7 +459,9 @@ static int krylov_alloc(IeOp *op, int mo, int mi, int precision)
     k = new KrylovWork();
     k->err = op->d_err;
     op->krylov = k;
-    return kw_alloc(k, op->nvec(), mo, mi, precision);
+    const int rc = kw_alloc(k, op->nvec(), mo, mi, precision);
+    if (rc) krylov_free(op);  // a later call with the same sizes must not take it for a complete workspace
+    return rc;
 }
 
 // ---- launch helpers ------------------------------------------------------------------------------
@@ -589,13 +615,12 @@ static int outer_solve(IeOp *op, KrylovWork *k, const GIEM2G_FGMRES_CTL &ctl, GI
     const bool true_res = tr && tr[0] == '1';
     CI *Z = reinterpret_cast<CI *>(k->Zo);
     CI *vin = reinterpret_cast<CI *>(k->vin);
-    double h_scal[S_NSCAL];
-    int h_flags[F_NFLAGS];
+    if (!k->report) G2_CUDA_CHECK(cudaMallocHost(&k->report, sizeof(Report)));
+    const double *h_scal = k->report->scal;
     auto pull = [&]() -> int {
-        G2_CUDA_CHECK(cudaMemcpyAsync(h_scal, L.scal, sizeof(h_scal), cudaMemcpyDeviceToHost, st));
-        G2_CUDA_CHECK(cudaMemcpyAsync(h_flags, L.flags, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
+        g2_launch(k_report, 1, 32, 0, st, L, k->err, k->report); g2_count_launches(1);
         G2_CUDA_CHECK(cudaStreamSynchronize(st));
-        return ie_check_device_error(op);
+        return k->report->err ? ie_check_device_error(op) : G2_OK;
     };
     k->history.clear();
     info->iterations = 0;
@@ -744,6 +769,7 @@ int krylov_solve_device(IeOp *op, const double2 *d_Ebkg, double2 *d_Esol, const 
     // Esol = a * chi (ie_solver_module.F90:85-97)
     g2_launch(k_scale_asig, g, 256, 0, st, d_Esol, k->x, op->d_asig64, cells, false); g2_count_launches(1);
     cudaEventRecord(e1, st);
+    g2_launch(k_report, 1, 32, 0, st, k->Lo, k->err, k->report); g2_count_launches(1);
     G2_CUDA_CHECK(cudaStreamSynchronize(st));
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
@@ -755,7 +781,7 @@ int krylov_solve_device(IeOp *op, const double2 *d_Ebkg, double2 *d_Esol, const 
     info->device_ms = ms;
     op->mult_num += k->applies64 + k->applies32;
     op->apply_seconds += ms * 1e-3;
-    return ie_check_device_error(op);
+    return k->report->err ? ie_check_device_error(op) : G2_OK;
 }
 
 int krylov_history(IeOp *op, double *out, int max_len)
