@@ -156,7 +156,7 @@ void g2_set_error(const char *file, int line, const char *msg);
 // Programmatic dependent launch for the solver's chains of short kernels.  pdl_wait() is the first statement of every
 // kernel launched with g2_launch: it returns when the preceding kernel of the stream has completed and its writes are
 // visible (so, by induction over the chain, everything before it too).  The wait also lets the next kernel's blocks be
-// set up while this one runs: at 32x32x8 the gap between two kernels fell from about 2 to under 1 us.
+// set up while this one runs: a complex128 apply of 32x32x8, five kernels, fell from 29 to 21.5 us.
 G2_D void pdl_wait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

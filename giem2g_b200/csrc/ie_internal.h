@@ -65,7 +65,8 @@ struct IeOp {
     bool use_fast_contract = true;     // GIEM2G_GENERIC_CONTRACT=1 selects the generic contraction kernel
     // contraction of FP64, complex64 and paired complex64 applies: a tile-shape variant of contract.cu, or -1 for
     // the tensor-core kernel (contract_mma.cu), the default: it takes every Nz, and at 128x128x32 it beats variant 0
-    // in every form (FP64 215 against 280 us, complex64 151 against 170 us, paired 172 against 291 us)
+    // in every form (FP64 221 against 280 us, complex64 154 against 174, paired 178 against 293); the best of its shapes, which the
+    // autotuner finds, take 207, 115 and 180 us there
     int contract_variant[3] = {-1, -1, -1};
     // fused y-transforms + contraction (ypipe.cu) per form: its variant, or -1 for the separate passes
     // (k_fy, contraction, k_by).  The separate passes are the default (faster at 128x128x32 on a B200);

@@ -99,9 +99,9 @@ int giem2g_get_ie_kernel_spectral(void *ie, void *symm_hat, void *asym_hat);
 int giem2g_apply_ie_operator_device(void *ie, const void *d_in, void *d_out, int precision);
 /* No counterpart in the reference.  The same apply as giem2g_apply_ie_operator_device, but it
  * allocates nothing: the apply's intermediates live in one static device array of the library
- * (32 MiB per device, shared by every call and operator on that device) instead of the operator's
- * buffers.  For hosts that must not allocate device memory after start-up.  Grids that need more
- * than 32 MiB of intermediates (18*Nx*Ny*Nz complex of the precision) are rejected with status
+ * (40 MiB per device, shared by every call and operator on that device) instead of the operator's
+ * buffers.  For hosts that must not allocate device memory after start-up.  Grids with more than
+ * 32 MiB of intermediates before padding (18*Nx*Ny*Nz complex of the precision) are rejected with status
  * -1 and a message.  The first call on a device sets up the array's address; make it before any stream
  * capture on that device (and again after a device reset, which repeats the set-up).  Calls that overlap
  * on the GPU race on the shared array: each operator has its own stream, so calls on two operators of one
@@ -111,10 +111,11 @@ int giem2g_apply_ie_operator_device_static(void *ie, const void *d_in, void *d_o
  * out) as a nonzero status. */
 int giem2g_check_device_error(void *ie);
 /* Contraction tile-shape variants available for a precision (0 or 1) at this Nz, and selection of one
- * (what the autotuner in giem2g_b200.autotune sets after timing them). */
+ * (what the autotuner in giem2g_b200.autotune sets after timing them).  Without a selection the contraction
+ * runs on the tensor cores, at every Nz; where there are variants that kernel is one of them. */
 int giem2g_contract_variants(void *ie, int precision);  /* precision 2: paired complex64 */
 int giem2g_set_contract_variant(void *ie, int precision, int variant);
-/* Lines per CTA of the FFT passes (4, 8, 16 or 32; default 32), also set by the autotuner: for both
+/* Lines per CTA of the FFT passes (4, 8, 16 or 32; default: 8 complex128, 16 complex64), also set by the autotuner: for both
  * precisions, or for one (0 complex128, 1 complex64, the paired apply included). */
 int giem2g_set_fft_lines(void *ie, int lines);
 int giem2g_set_fft_lines_precision(void *ie, int precision, int lines);
