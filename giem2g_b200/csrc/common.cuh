@@ -157,9 +157,13 @@ void g2_set_error(const char *file, int line, const char *msg);
 // kernel launched with g2_launch: it returns when the preceding kernel of the stream has completed and its writes are
 // visible (so, by induction over the chain, everything before it too).  The wait also lets the next kernel's blocks be
 // set up while this one runs: a complex128 apply of 32x32x8, five kernels, fell from 29 to 21.5 us.
-G2_D void pdl_wait()
+G2_D void pdl_wait_only()  // the next kernel starts when this one ends
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+G2_D void pdl_wait()
+{
+    pdl_wait_only();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... A>

@@ -27,7 +27,9 @@
 //
 // Persistent CTAs with a ring of stages (one unit each, tensor with an L2 evict_first hint, and its spectrum).  NG
 // groups of W warps take the units round-robin.  No barrier joins the warps: each waits for the stage, reads it,
-// releases it and stores its own rows.  All waits are bounded (2 s, error codes 41 to 43).
+// releases it and stores its own rows.  All waits are bounded (2 s, error codes 41 to 43).  The kernels do not let their
+// dependents start early: with k_by's blocks waiting from the first wave on, k_by and k_bx after it took 52 and 33 us
+// instead of 29 and 24 (complex128, 128x128x32; whole apply 343 -> 321 us, 64x128x27 151 -> 144, pair 277 -> 275).
 #include <cstdint>
 #include "common.cuh"
 #include "ie_internal.h"
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
     for (int kt = 0; kt < KT; kt++)
         off[kt] = (uint32_t)mma_offset<KT1>(rt, nl, kt, kl, Nz, P, T + u_elems) |
                   (uint32_t)mma_offset<KT1>(rt, nl, kt, kl + 4, Nz, P, T + u_elems) << 16;
-    pdl_wait();  // the offsets above need nothing of the kernels before this one
+    pdl_wait_only();  // the offsets above need nothing of the kernels before this one
     if (gate && *gate == 0) return;
     mma_ring<double2, W, NG_, true>(smem, G, Uhat, a, u_elems, T, err,
                               [&](const unsigned char *g, const unsigned char *us, long long unit, auto release) {
@@ -496,7 +498,7 @@ __global__ void __launch_bounds__(MmaCfg32<KZ, NG_>::NTHREADS, 1)
                         k1 < Nz ? 4 * P + full_pos<false>(k1, z, Nz) : zero);
         }
     }
-    pdl_wait();
+    pdl_wait_only();
     if (gate && *gate == 0) return;
     mma_ring<float2, KZ, NG_, false>(smem, G, Uhat, a, u_elems, T, err,
                               [&](const unsigned char *g, const unsigned char *us, long long unit, auto release) {
