@@ -798,9 +798,9 @@ int krylov_history(IeOp *op, double *out, int max_len)
 // nested FGMRES with its own workspace, advanced in lockstep on one stream.  Per outer step the host
 // launches every active instance's work, replays ONE captured inner cycle for all instances and reads
 // all instances' scalars with one synchronisation.  Consecutive instances of the same operator form
-// pairs whose complex64 applies share every tensor read (ie_apply_pair32).  Each instance follows exactly
-// the launch sequence of the single solve, so its iterates, iteration count and status are those of a
-// solve on its own.  Converged instances are masked: their inner-cycle kernels are gated off through a
+// pairs whose complex64 applies share every tensor read (ie_apply_pair32).  Each instance follows
+// the operations of the single solve, so its iteration count and status are those of a solve on its own; its
+// sums may be split over fewer blocks (arnoldi.cu), a difference of rounding.  Converged instances are masked: their inner-cycle kernels are gated off through a
 // device flag and the host stops launching their outer work.
 struct BatchGroup {
     IeOp *op = nullptr;
