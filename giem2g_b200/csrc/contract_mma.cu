@@ -11,10 +11,18 @@
 //     rows combine into the outputs;
 //   * complex128: mma.m8n8k4.f64, rows (point, part);
 //   * complex64: mma.m16n8k8.tf32 with each operand split into two TF32 numbers, x = hi + lo.  The hi hi products of
-//     one z'-tile start from zero and are added to the FP32 accumulator with a rounded add (the tensor core truncates
-//     when it accumulates, which would bias a long sum); the hi lo and lo hi products, 2^-11 smaller, accumulate in
-//     the tensor core.  Two vectors (NP = 2) fill the 16 rows with 8 points' parts; one vector (NP = 1) fills them
-//     with 4 points' parts, hi in rows 0-7 and lo in rows 8-15, so two instructions do the four products.
+//     one block and z'-tile start from zero and are added to the FP32 accumulator with a rounded add (the tensor core
+//     truncates when it accumulates, which would bias a long sum); the hi lo and lo hi products, 2^-11 smaller,
+//     accumulate in the tensor core.  Two vectors (NP = 2) fill the 16 rows with 8 points' parts; one vector (NP = 1)
+//     fills them with 4 points' parts, hi in rows 0-7 and lo in rows 8-15, so two instructions do the four products.
+//     Up to 12 z the operands are split into three numbers, which hold every bit: an FP32 sum that short has a smaller
+//     error than two numbers leave (the last bit of lo, for NP = 2 the lo lo products), and the launch is bound elsewhere
+//     (128x128x8: 22 and 26 us where two numbers take 16 and 19).
+// Error of a unit's products against 80-bit sums, FP32 FMA kernels (plain or contract.cu's) -> this one, single / pair:
+// random units Nz = 8 1.1e-7 / 1.4e-7 -> 0.6e-7 / 0.6e-7, Nz = 13 1.00e-7 -> 0.94e-7 / 1.03e-7, Nz = 32 1.20e-7 / 1.43e-7
+// -> 1.02e-7 / 1.12e-7, Nz = 48 1.7e-7 -> 1.1e-7 / 1.2e-7; a layered background's tensor (Nz = 32) 1.09e-7 / 1.29e-7 ->
+// 0.92e-7 / 1.01e-7; one non-zero component 0.95e-7 / 1.01e-7 -> 0.88e-7 / 0.98e-7; coherent signs 0.63e-7 / 0.82e-7 ->
+// 0.69e-7 / 0.70e-7; one non-zero layer 0.74e-7 -> 0.88e-7 / 0.98e-7.
 // M's elements are read straight from the packed unit in shared memory: their offsets depend on the lane alone, so every
 // lane keeps its offsets in registers for the whole kernel; padded columns point at a zero.  The spectrum has a row pitch
 // of 4 mod 8 elements, which spreads the points' columns over the shared-memory banks.  complex128 warps own eight rows
@@ -22,8 +30,8 @@
 // z rows of eight z, which lets one split of an xy tile serve two products.
 // What bounds it at 128x128x32 (16384 units): complex128 HBM (tensor and spectrum twice, 1.29 GB: 200 us at the measured
 // copy rate, 215-221 us measured); paired complex64 the TF32 pipe (864 instructions of 8-9 clocks per SM partition and unit,
-// 110 us) plus the splits' instructions, which overlap with it only in part (172-178 us; the FP32 kernels of contract.cu
-// take 180 to 293 us); single complex64 the same splits for half the products (154 us).
+// 110 us) plus the splits' instructions, which overlap with it only in part (178 us; the FP32 kernels of contract.cu
+// take 180 to 293 us); single complex64 the same splits for half the products (142 us).
 //
 // Persistent CTAs with a ring of stages (one unit each, tensor with an L2 evict_first hint, and its spectrum).  NG
 // groups of W warps take the units round-robin.  No barrier joins the warps: each waits for the stage, reads it,
@@ -80,18 +88,17 @@ G2_D float2 add2(float2 a, float2 b)
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(uc.u) : "l"(ua.u), "l"(ub.u));
     return uc.f;
 }
-// d = a b + (0, 0, c2, c3)
-template <bool HALF>
-G2_D void tmma_from(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c2, float c3)
+// d = a b
+template <bool HALF> G2_D void tmma_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
     if constexpr (HALF)
-        asm("mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%8,%9};"
+        asm("mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
             : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-            : "r"(a[0]), "r"(a[1]), "r"(b0), "f"(0.f), "f"(c2), "f"(c3));
+            : "r"(a[0]), "r"(a[1]), "r"(b0), "f"(0.f));
     else
-        asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%11,%12};"
+        asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
             : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f), "f"(c2), "f"(c3));
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 // x = hi + lo: hi rounded to TF32 (11 significant bits), lo the exact rest, whose last bit or two the tensor core
 // drops (2^-23 |x| at most, of either sign)
@@ -99,6 +106,13 @@ G2_D void split(float x, uint32_t &hi, uint32_t &lo)
 {
     hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     lo = __float_as_uint(x - __uint_as_float(hi));
+}
+// x = hi + lo + rest exactly: lo rounded to TF32 too, the rest the last bit or two
+G2_D void split3(float x, uint32_t &hi, uint32_t &lo, uint32_t &rest)
+{
+    uint32_t r;
+    split(x, hi, r);
+    split(__uint_as_float(r), lo, rest);
 }
 template <typename T> G2_D T at(const void *p, uint32_t bytes)
 {
@@ -249,12 +263,15 @@ G2_D bool is_nyquist(long long unit, int Ny, int slot_pt)
 }
 
 // Lanes l and l ^ 4 hold the real (comp 0) and imaginary (comp 1) rows of one point: from their rows' products with
-// Re M (r0, r1) and Im M (i0, i1) for outputs j, j + 1, the complex outputs; comp 0 stores j, comp 1 stores j + 1.
-template <typename C, typename R>
-G2_D void store_pair(C *row, int j, R r0, R r1, R i0, R i1, R g0, R g1, bool ok, int comp)
+// Re M (r) and Im M (i), the complex output's part comp
+template <typename R> G2_D R complex_part(R r, R i, int comp)
 {
-    const R p0 = __shfl_xor_sync(0xffffffffu, i0, 4), p1 = __shfl_xor_sync(0xffffffffu, i1, 4);
-    const R v0 = (comp ? r0 + p0 : r0 - p0) * g0, v1 = (comp ? r1 + p1 : r1 - p1) * g1;
+    const R p = __shfl_xor_sync(0xffffffffu, i, 4);
+    return comp ? r + p : r - p;
+}
+// v0, v1: the lane's parts of outputs j and j + 1; comp 0 stores j, comp 1 stores j + 1
+template <typename C, typename R> G2_D void store_pair(C *row, int j, R v0, R v1, bool ok, int comp)
+{
     const R x = __shfl_xor_sync(0xffffffffu, comp ? v0 : v1, 4);
     if (ok) row[j + comp] = comp ? C{x, v1} : C{v0, x};
 }
@@ -317,13 +334,13 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
             g1 = j + 1 < Nz ? 1.0 : sy;
         }
         if (is_nyquist(unit, a.Ny, pt)) ar[0] = ar[1] = ai[0] = ai[1] = 0.0;
-        store_pair(Uhat + unit * (long long)u_elems + pt * a.pitch, j, ar[0], ar[1], ai[0], ai[1], g0, g1,
-                   j + comp < lim, comp);
+        store_pair(Uhat + unit * (long long)u_elems + pt * a.pitch, j, complex_part(ar[0], ai[0], comp) * g0,
+                   complex_part(ar[1], ai[1], comp) * g1, j + comp < lim, comp);
     });
 }
 
 // ---- complex64 -------------------------------------------------------------------------------------------------
-// one real row component's sums: hi hi (FP32, rounded adds), the small products (in the tensor core)
+// one real row component's sums: hi hi (FP32, rounded adds), the smaller products (in the tensor core)
 template <int NP> struct Acc32 {
     float2 r[NP], i[NP];
     float sr[4], si[4];
@@ -337,79 +354,101 @@ template <int NP> struct Acc32 {
         tr = ti = make_float2(0.f, 0.f);
     }
 };
-// A fragment of one component of V (k-tile of 8 or 4)
-template <int NP> struct Vfrag {
-    uint32_t h[4], l[4];
+// A fragment of one component of V (k-tile of 8 or 4); t: the third parts (TERMS = 3)
+template <int NP, int TERMS> struct Vfrag {
+    uint32_t h[4], l[4], t[TERMS == 3 ? 4 : 1];
 };
-template <int NP, bool HALF> G2_D Vfrag<NP> load_v(const float2 *u, int k0, int k1, float s, int comp)
+template <int NP, int TERMS, bool HALF>
+G2_D Vfrag<NP, TERMS> load_v(const float2 *u, int k0, int k1, float s, int comp)
 {
-    Vfrag<NP> v;
+    Vfrag<NP, TERMS> v{};
+    // part q of the fragment's word (NP = 2), or of its words q and q + 1 (NP = 1: rows 0-7 hi, rows 8-15 lo)
+    auto put = [&](int q, float x) {
+        uint32_t h, l, t = 0u;
+        if constexpr (TERMS == 3) split3(x * s, h, l, t);
+        else split(x * s, h, l);
+        v.h[q] = h;
+        if constexpr (NP == 2) v.l[q] = l;
+        else v.h[q + 1] = l;
+        if constexpr (TERMS == 3) v.t[q] = t;
+    };
     if constexpr (NP == 2) {
         const float2 u0 = u[k0];
-        split(u0.x * s, v.h[0], v.l[0]);
-        split(u0.y * s, v.h[1], v.l[1]);
-        v.h[2] = v.h[3] = v.l[2] = v.l[3] = 0u;
+        put(0, u0.x);
+        put(1, u0.y);
         if constexpr (!HALF) {
             const float2 u1 = u[k1];
-            split(u1.x * s, v.h[2], v.l[2]);
-            split(u1.y * s, v.h[3], v.l[3]);
+            put(2, u1.x);
+            put(3, u1.y);
         }
-    } else {  // rows 0-7 hi, rows 8-15 lo of the lane's part
-        split(reinterpret_cast<const float *>(u + k0)[comp] * s, v.h[0], v.h[1]);
-        v.h[2] = v.h[3] = 0u;
-        if constexpr (!HALF) split(reinterpret_cast<const float *>(u + k1)[comp] * s, v.h[2], v.h[3]);
+    } else {
+        put(0, reinterpret_cast<const float *>(u + k0)[comp]);
+        if constexpr (!HALF) put(2, reinterpret_cast<const float *>(u + k1)[comp]);
     }
     return v;
 }
-template <int NP> G2_D Vfrag<NP> negate(const Vfrag<NP> &v)
+template <int NP, int TERMS> G2_D Vfrag<NP, TERMS> negate(const Vfrag<NP, TERMS> &v)
 {
-    Vfrag<NP> w;
+    Vfrag<NP, TERMS> w{};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         w.h[k] = v.h[k] ^ 0x80000000u;
         w.l[k] = v.l[k] ^ 0x80000000u;
+        if constexpr (TERMS == 3) w.t[k] = v.t[k] ^ 0x80000000u;
     }
     return w;
 }
-struct Mfrag {
-    uint32_t rh[2], rl[2], ih[2], il[2];
+template <int TERMS> struct Mfrag {
+    uint32_t rh[2], rl[2], ih[2], il[2], rt[TERMS == 3 ? 2 : 1], it[TERMS == 3 ? 2 : 1];
 };
-template <bool HALF> G2_D Mfrag load_m(const unsigned char *g, uint32_t o0, uint32_t o1)
+template <int TERMS, bool HALF> G2_D Mfrag<TERMS> load_m(const unsigned char *g, uint32_t o0, uint32_t o1)
 {
-    Mfrag m;
-    const float2 e0 = at<float2>(g, o0);
-    split(e0.x, m.rh[0], m.rl[0]);
-    split(e0.y, m.ih[0], m.il[0]);
-    m.rh[1] = m.rl[1] = m.ih[1] = m.il[1] = 0u;
-    if constexpr (!HALF) {
-        const float2 e1 = at<float2>(g, o1);
-        split(e1.x, m.rh[1], m.rl[1]);
-        split(e1.y, m.ih[1], m.il[1]);
-    }
+    Mfrag<TERMS> m{};
+    auto put = [&](int q, float2 e) {
+        if constexpr (TERMS == 3) {
+            split3(e.x, m.rh[q], m.rl[q], m.rt[q]);
+            split3(e.y, m.ih[q], m.il[q], m.it[q]);
+        } else {
+            split(e.x, m.rh[q], m.rl[q]);
+            split(e.y, m.ih[q], m.il[q]);
+        }
+    };
+    put(0, at<float2>(g, o0));
+    if constexpr (!HALF) put(1, at<float2>(g, o1));
     return m;
 }
-// The hi hi sums of one row component over one z'-tile: three products accumulate here, starting from zero, before
-// a rounded add takes them into Acc32.
+// The hi hi sums of one product over one z'-tile.  They start from zero and a rounded add takes them into Acc32, so a
+// product is truncated once, at its own size; a part of the tensor or of the vector that is small or zero costs nothing.
+// truncation: what that takes off on average, half a unit in the last place of a mantissa m of density 1 / (m ln 2),
+// 2^-24 E[1 / m] = 2^-24 / (2 ln 2) = 4.3e-8.  It is added with the smaller products, before the last rounding.  Measured
+// loss: random units and vectors 3.4e-8, one non-zero component 3.5e-8, a layered background's tensor 3.6e-8, coherent
+// signs 4.0e-8; a vector with one non-zero layer loses nothing, since the sum of one product is exact, and gains it.  Sums
+// of up to 12 z have part tiles whose few products leave fewer bits to lose: 2.4e-8 (Nz = 4) to 3.5e-8 (Nz = 8).
+template <int TERMS> constexpr float truncation = TERMS == 3 ? 3.3e-8f : 4.3e-8f;
 template <int NP> struct Sum32 {
     float r[4], i[4];
 };
-// s (+)= hi hi part, c += small parts of V M^T for one tile
-template <int NP, bool HALF, bool FIRST>
-G2_D void product(Sum32<NP> &s, Acc32<NP> &c, const Vfrag<NP> &v, const Mfrag &m)
+// s = hi hi part, c += smaller parts of V M^T for one tile
+template <int NP, int TERMS, bool HALF>
+G2_D void product(Sum32<NP> &s, Acc32<NP> &c, const Vfrag<NP, TERMS> &v, const Mfrag<TERMS> &m)
 {
-    if constexpr (FIRST) {
-        const float2 tr = NP == 2 ? make_float2(0.f, 0.f) : c.tr, ti = NP == 2 ? make_float2(0.f, 0.f) : c.ti;
-        tmma_from<HALF>(s.r, v.h, m.rh[0], m.rh[1], tr.x, tr.y);
-        tmma_from<HALF>(s.i, v.h, m.ih[0], m.ih[1], ti.x, ti.y);
-    } else {
-        tmma<HALF>(s.r, v.h, m.rh[0], m.rh[1]);
-        tmma<HALF>(s.i, v.h, m.ih[0], m.ih[1]);
-    }
+    tmma_zero<HALF>(s.r, v.h, m.rh[0], m.rh[1]);
+    tmma_zero<HALF>(s.i, v.h, m.ih[0], m.ih[1]);
     tmma<HALF>(c.sr, v.h, m.rl[0], m.rl[1]);
     tmma<HALF>(c.si, v.h, m.il[0], m.il[1]);
     if constexpr (NP == 2) {
         tmma<HALF>(c.sr, v.l, m.rh[0], m.rh[1]);
         tmma<HALF>(c.si, v.l, m.ih[0], m.ih[1]);
+    }
+    if constexpr (TERMS == 3) {
+        if constexpr (NP == 2) {
+            tmma<HALF>(c.sr, v.l, m.rl[0], m.rl[1]);
+            tmma<HALF>(c.si, v.l, m.il[0], m.il[1]);
+        }
+        tmma<HALF>(c.sr, v.h, m.rt[0], m.rt[1]);
+        tmma<HALF>(c.si, v.h, m.it[0], m.it[1]);
+        tmma<HALF>(c.sr, v.t, m.rh[0], m.rh[1]);
+        tmma<HALF>(c.si, v.t, m.ih[0], m.ih[1]);
     }
 }
 template <int NP> G2_D void take(Acc32<NP> &c, const Sum32<NP> &s)
@@ -420,8 +459,8 @@ template <int NP> G2_D void take(Acc32<NP> &c, const Sum32<NP> &s)
         c.r[1] = add2(c.r[1], make_float2(s.r[2], s.r[3]));
         c.i[1] = add2(c.i[1], make_float2(s.i[2], s.i[3]));
     } else {
-        c.tr = make_float2(s.r[2], s.r[3]);
-        c.ti = make_float2(s.i[2], s.i[3]);
+        c.tr = add2(c.tr, make_float2(s.r[2], s.r[3]));
+        c.ti = add2(c.ti, make_float2(s.i[2], s.i[3]));
     }
 }
 // A lane's tensor offsets for one z'-tile: the symmetric, the full and the transposed full tile, two k halves each;
@@ -443,7 +482,7 @@ template <bool PACK> struct Offs {
 // All nine products of z-tile (rows) and z'-tile (columns).  LAST: the tile may hold padded k, whose offsets point at
 // the zero z0 in every block (padded rows repeat the last row; they are not stored).  pb, fb: bytes of a symmetric and
 // of a full block.
-template <int NP, bool HALF, bool LAST, bool PACK>
+template <int NP, int TERMS, bool HALF, bool LAST, bool PACK>
 G2_D void tile_products(Acc32<NP> (&acc)[3], const unsigned char *g, const float2 *u, int k0, int k1, int Nz, float sy,
                         float sz, int comp, const Offs<PACK> &of, uint32_t z0, uint32_t pb, uint32_t fb)
 {
@@ -451,24 +490,33 @@ G2_D void tile_products(Acc32<NP> (&acc)[3], const unsigned char *g, const float
     const uint32_t p0 = LAST && o[0] == z0 ? 0u : pb, p1 = LAST && o[1] == z0 ? 0u : pb;
     const uint32_t f0 = LAST && o[2] == z0 ? 0u : fb, f1 = LAST && o[3] == z0 ? 0u : fb;
     const uint32_t t0 = f0, t1 = f1;
-    const Vfrag<NP> vx = load_v<NP, HALF>(u, k0, k1, 1.f, comp);
-    const Vfrag<NP> vy = load_v<NP, HALF>(u + Nz, k0, k1, sy, comp);
-    const Vfrag<NP> vz = load_v<NP, HALF>(u + 2 * Nz, k0, k1, sz, comp);
+    const Vfrag<NP, TERMS> vx = load_v<NP, TERMS, HALF>(u, k0, k1, 1.f, comp);
+    const Vfrag<NP, TERMS> vy = load_v<NP, TERMS, HALF>(u + Nz, k0, k1, sy, comp);
+    const Vfrag<NP, TERMS> vz = load_v<NP, TERMS, HALF>(u + 2 * Nz, k0, k1, sz, comp);
     Sum32<NP> s, t;
+    auto mul = [&](Sum32<NP> &d, Acc32<NP> &a, const Vfrag<NP, TERMS> &v, uint32_t e0, uint32_t e1) {
+        product<NP, TERMS, HALF>(d, a, v, load_m<TERMS, HALF>(g, e0, e1));
+    };
     {
-        const Mfrag m = load_m<HALF>(g, o[0] + p0, o[1] + p1);  // xy
-        product<NP, HALF, true>(s, acc[0], vy, m);
-        product<NP, HALF, true>(t, acc[1], vx, m);
+        const Mfrag<TERMS> m = load_m<TERMS, HALF>(g, o[0] + p0, o[1] + p1);  // xy
+        product<NP, TERMS, HALF>(s, acc[0], vy, m);
+        product<NP, TERMS, HALF>(t, acc[1], vx, m);
     }
-    product<NP, HALF, false>(s, acc[0], vx, load_m<HALF>(g, o[0], o[1]));
-    product<NP, HALF, false>(t, acc[1], vy, load_m<HALF>(g, o[0] + 2 * p0, o[1] + 2 * p1));
-    product<NP, HALF, false>(s, acc[0], vz, load_m<HALF>(g, o[2], o[3]));
-    product<NP, HALF, false>(t, acc[1], vz, load_m<HALF>(g, o[2] + f0, o[3] + f1));
     take(acc[0], s);
-    product<NP, HALF, true>(s, acc[2], vx, load_m<HALF>(g, o[4], o[5]));
     take(acc[1], t);
-    product<NP, HALF, false>(s, acc[2], vy, load_m<HALF>(g, o[4] + t0, o[5] + t1));
-    product<NP, HALF, false>(s, acc[2], negate(vz), load_m<HALF>(g, o[0] + 3 * p0, o[1] + 3 * p1));  // acc[2] = -out_z
+    mul(s, acc[0], vx, o[0], o[1]);
+    mul(t, acc[1], vy, o[0] + 2 * p0, o[1] + 2 * p1);
+    take(acc[0], s);
+    take(acc[1], t);
+    mul(s, acc[0], vz, o[2], o[3]);
+    mul(t, acc[1], vz, o[2] + f0, o[3] + f1);
+    take(acc[0], s);
+    take(acc[1], t);
+    mul(s, acc[2], vx, o[4], o[5]);
+    mul(t, acc[2], vy, o[4] + t0, o[5] + t1);
+    take(acc[2], s);
+    take(acc[2], t);
+    mul(s, acc[2], negate(vz), o[0] + 3 * p0, o[1] + 3 * p1);  // acc[2] = -out_z
     take(acc[2], s);
 }
 
@@ -485,6 +533,7 @@ __global__ void __launch_bounds__(MmaCfg32<KZ, NG_>::NTHREADS, 1)
     const float sz = (slot_pt & 2) ? -1.f : 1.f, sy = (slot_pt & 1) ? -sz : sz;  // sx, sx m
     const uint32_t z0 = sizeof(float2) * (T + u_elems), pb = sizeof(float2) * P, fb = sizeof(float2) * Nz * Nz;
     constexpr bool PACK = KZ >= 5;
+    constexpr int TERMS = KZ == 1 || (KZ == 2 && HALF) ? 3 : 2;  // Nz <= 12
     Offs<PACK> off[KZ];
     {
         const int z = min(rt * 8 + nl, Nz - 1), zero = T + u_elems;
@@ -508,16 +557,14 @@ __global__ void __launch_bounds__(MmaCfg32<KZ, NG_>::NTHREADS, 1)
         for (int c = 0; c < 3; c++) acc[c].clear();
 #pragma unroll
         for (int kt = 0; kt < KZ - 1; kt++)
-            tile_products<NP, false, false, PACK>(acc, g, u, kt * 8 + kl, kt * 8 + kl + 4, Nz, sy, sz, comp, off[kt], z0, pb, fb);
+            tile_products<NP, TERMS, false, false, PACK>(acc, g, u, kt * 8 + kl, kt * 8 + kl + 4, Nz, sy, sz, comp, off[kt], z0, pb, fb);
         // padded k read an element that exists (M is zero there)
-        tile_products<NP, HALF, true, PACK>(acc, g, u, min((KZ - 1) * 8 + kl, Nz - 1), min((KZ - 1) * 8 + kl + 4, Nz - 1),
+        tile_products<NP, TERMS, HALF, true, PACK>(acc, g, u, min((KZ - 1) * 8 + kl, Nz - 1), min((KZ - 1) * 8 + kl + 4, Nz - 1),
                                             Nz, sy, sz, comp, off[KZ - 1], z0, pb, fb);
         release();
         float2 *row = Uhat + unit * (long long)u_elems + pt * a.pitch;
         const int z = rt * 8 + 2 * kl;
-        // three truncated accumulations per z'-tile take 7e-8 of every sum on average (the same at every Nz on random
-        // units); giving that back takes the units' error from 1.26e-7 to 1.08e-7
-        auto grown = [](float v) { return fmaf(v, 7e-8f, v); };
+        auto total = [](float hi, float small) { return hi + fmaf(hi, truncation<TERMS>, small); };
         if (is_nyquist(unit, a.Ny, slot_pt))
 #pragma unroll
             for (int c = 0; c < 3; c++) acc[c].clear();
@@ -527,15 +574,18 @@ __global__ void __launch_bounds__(MmaCfg32<KZ, NG_>::NTHREADS, 1)
             const float s = c == 0 ? 1.f : (c == 1 ? sy : -sz);
             float2 *dst = row + c * Nz;
             if constexpr (NP == 2) {
-                const float tr[4] = {q.r[0].x + q.sr[0], q.r[0].y + q.sr[1], q.r[1].x + q.sr[2], q.r[1].y + q.sr[3]};
-                const float ti[4] = {q.i[0].x + q.si[0], q.i[0].y + q.si[1], q.i[1].x + q.si[2], q.i[1].y + q.si[3]};
-                if (z < Nz) dst[z] = make_float2(grown(tr[0] - ti[2]) * s, grown(tr[2] + ti[0]) * s);
-                if (z + 1 < Nz) dst[z + 1] = make_float2(grown(tr[1] - ti[3]) * s, grown(tr[3] + ti[1]) * s);
+                if (z < Nz)
+                    dst[z] = make_float2(total(q.r[0].x - q.i[1].x, q.sr[0] - q.si[2]) * s,
+                                         total(q.r[1].x + q.i[0].x, q.sr[2] + q.si[0]) * s);
+                if (z + 1 < Nz)
+                    dst[z + 1] = make_float2(total(q.r[0].y - q.i[1].y, q.sr[1] - q.si[3]) * s,
+                                             total(q.r[1].y + q.i[0].y, q.sr[3] + q.si[1]) * s);
             } else {
-                store_pair(dst, z, grown(q.r[0].x + (q.sr[0] + (q.sr[2] + q.tr.x))),
-                           grown(q.r[0].y + (q.sr[1] + (q.sr[3] + q.tr.y))),
-                           grown(q.i[0].x + (q.si[0] + (q.si[2] + q.ti.x))),
-                           grown(q.i[0].y + (q.si[1] + (q.si[3] + q.ti.y))), s, s, z + comp < Nz, comp);
+                const float v0 = total(complex_part(q.r[0].x, q.i[0].x, comp),
+                                       complex_part(q.sr[0] + (q.sr[2] + q.tr.x), q.si[0] + (q.si[2] + q.ti.x), comp));
+                const float v1 = total(complex_part(q.r[0].y, q.i[0].y, comp),
+                                       complex_part(q.sr[1] + (q.sr[3] + q.tr.y), q.si[1] + (q.si[3] + q.ti.y), comp));
+                store_pair(dst, z, v0 * s, v1 * s, z + comp < Nz, comp);
             }
         }
     });
