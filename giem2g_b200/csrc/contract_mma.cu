@@ -283,6 +283,12 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
 {
     using Cfg = MmaCfg64<KT1, KT2, NG_>;
     constexpr int KT = Cfg::KT, W = Cfg::W;
+    // A sum in one chain of FMAs has 1.2 to 1.5 times the error of the FP64 kernels it takes the place of.  Two chains (the
+    // k halves of each tile) have a smaller one; blocks of four tiles, each added to the total, a smaller one still.
+    // Time of one chain / two / blocks, 128x128: Nz = 20 91 / 91 / 99 us, 27 171 / 171 / 179, 32 216 / 219 / 218,
+    // 40 313 / 329 / 331, 48 606 / 623 / 632, 57 964 / 1007 / 966: blocks where they cost no more than two chains.  Error on
+    // random units: Nz = 32 3.3e-16 / 2.4e-16 / 2.1e-16 (contract.cu 2.2e-16), 48 4.0e-16 / 2.9e-16 / 2.1e-16 (3.1e-16).
+    constexpr bool BLOCKED = KT == 12 || KT == 23;
     extern __shared__ __align__(128) unsigned char smem[];
     const int Nz = a.Nz, P = Nz * (Nz + 1) / 2, T = 4 * P + 2 * Nz * Nz, u_elems = 4 * a.pitch;
     const int lane = threadIdx.x & 31, rt = (threadIdx.x >> 5) % W;
@@ -298,7 +304,7 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
     mma_ring<double2, W, NG_, true>(smem, G, Uhat, a, u_elems, T, err,
                               [&](const unsigned char *g, const unsigned char *us, long long unit, auto release) {
         const double *u = reinterpret_cast<const double *>(us) + 2 * pt * a.pitch + comp;
-        double ar[2] = {0.0, 0.0}, ai[2] = {0.0, 0.0};
+        double ar[2] = {0.0, 0.0}, ai[2] = {0.0, 0.0}, br[2] = {0.0, 0.0}, bi[2] = {0.0, 0.0};
 #pragma unroll
         for (int kt = 0; kt < KT; kt++) {
             if (kt == KT1 && rt >= KT1) {  // the transposed blocks of out_z
@@ -306,6 +312,12 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
                 ar[1] = -ar[1];
                 ai[0] = -ai[0];
                 ai[1] = -ai[1];
+                if constexpr (!BLOCKED) {
+                    br[0] = -br[0];
+                    br[1] = -br[1];
+                    bi[0] = -bi[0];
+                    bi[1] = -bi[1];
+                }
             }
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -322,8 +334,21 @@ __global__ void __launch_bounds__(MmaCfg64<KT1, KT2, NG_>::NTHREADS, 1)
                 }
                 const double x = u[2 * k] * s;
                 const double2 e = at<double2>(g, 16u * (h ? off[kt] >> 16 : off[kt] & 0xffffu));
-                dmma(ar, x, e.x);
-                dmma(ai, x, e.y);
+                if (BLOCKED || h) {
+                    dmma(br, x, e.x);
+                    dmma(bi, x, e.y);
+                } else {
+                    dmma(ar, x, e.x);
+                    dmma(ai, x, e.y);
+                }
+            }
+            if (kt == KT - 1 || (BLOCKED && (kt % 4 == 3 || kt == KT1 - 1))) {
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    ar[q] += br[q];
+                    ai[q] += bi[q];
+                    br[q] = bi[q] = 0.0;
+                }
             }
         }
         release();

@@ -113,3 +113,17 @@ def test_complex64_sums_keep_their_size(g2lib, orc, Nz, components):
                 den += float(np.sum(np.abs(e) ** 2))
             op.delete()
         assert abs(num / den) < 2.1e-8, (form, num / den)
+
+
+def test_complex128_sums_are_split(g2lib, orc):
+    """57 layers: one chain of FMAs per output has an error of 4.4e-16, two chains 3.2e-16; the apply's other roundings add
+    about 1e-16 in quadrature, so 4.5e-16 and 3.4e-16 for the whole."""
+    num, den = 0.0, 0.0
+    for seed in range(6):
+        m, op, symm, asym, csiga, csigb, v = _case(g2lib, orc, 57, 10 * seed + 5)
+        e = exact_apply(m, symm, asym, csiga, csigb, v)
+        got = _run(g2lib, op, [v], 0)[0].astype(np.clongdouble)
+        num += float(np.sum(np.abs(got - e) ** 2))
+        den += float(np.sum(np.abs(e) ** 2))
+        op.delete()
+    assert np.sqrt(num / den) < 3.9e-16, np.sqrt(num / den)
