@@ -9,6 +9,7 @@
 // Whole solves, launches per sweep -> one launch with its barriers, the last scalar step beside the scaling and the scaling
 // four words at a time: FP64 32x32x8 3.31 -> 2.30 ms, mixed pairs 128x128x32 2 ms of 66 (bound by the sweeps' HBM and L2
 // traffic).
+#include <atomic>
 #include <type_traits>
 #include <utility>
 #include "krylov_dev.cuh"
@@ -134,6 +135,15 @@ G2_D void scale_rows(const T *w, T *v, size_t n, size_t S, F f)
     }
 }
 
+// Sums of a complex64 sweep: a thread adds up to kChain elements in FP32, then that to FP64 sums of its own in shared
+// memory.  (A thread's part of a vector is 83 elements for a pair of 128x128x32 and 498 for one of 256x256x48; in one FP32
+// chain its error would grow with it.)
+constexpr int kChain = 16;
+template <typename C, int K> constexpr size_t sums_bytes()
+{
+    return sizeof(C) == sizeof(float2) ? (K + 1) * kVT * sizeof(double2) : 0;
+}
+
 template <typename C, int K>
 __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double tol, int *err)
 {
@@ -155,9 +165,37 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
     W *ww = reinterpret_cast<W *>(w);
     const size_t set = (size_t)gridDim.x * (KMAX + 1);
     R ax[K + 1], ay[K + 1];
-    auto clear = [&] {
+    extern __shared__ __align__(16) double2 sums[];  // [K + 1][kVT]
+    int added;  // elements in ax, ay
+    bool kept;  // the thread has sums in shared memory
+    auto zero = [&] {
 #pragma unroll
         for (int k = 0; k <= K; k++) ax[k] = ay[k] = R(0);
+        added = 0;
+    };
+    auto clear = [&] {
+        zero();
+        kept = false;
+    };
+    auto total = [&](int k) {
+        double2 v = make_double2(ax[k], ay[k]);
+        if constexpr (sums_bytes<C, K>() > 0)
+            if (kept) {
+                const double2 s = sums[k * kVT + threadIdx.x];
+                v.x += s.x;
+                v.y += s.y;
+            }
+        return v;
+    };
+    auto count = [&](int n) {  // after n more elements
+        if constexpr (sums_bytes<C, K>() > 0) {
+            added += n;
+            if (added + n <= kChain) return;
+#pragma unroll
+            for (int k = 0; k <= K; k++) sums[k * kVT + threadIdx.x] = total(k);
+            kept = true;
+            zero();
+        }
     };
     auto dots = [&](const C &a, const C *b) {
 #pragma unroll
@@ -198,12 +236,16 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
                     for (int k = 0; k < KH; k++) b[k] = part_of(v[k][u], e);
                     dots(part_of(wv[u], e), b);
                 }
+            count(NU * E);
         };
         for (; i + (U - 1) * S < Nw; i += U * S) round(std::integral_constant<int, U>());
         for (; i < Nw; i += S) round(std::integral_constant<int, 1>());
     }
-    for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) dots_of(w[i], i);
-    block_reduce_store_r<K, R>(ax, ay, mm.part[y]);
+    for (i = HOLD ? Nw * E + t0 : t0; i < N; i += S) {
+        dots_of(w[i], i);
+        count(1);
+    }
+    block_reduce_store<K>(total, mm.part[y]);
     if (!grid_barrier(L.bar, gridDim.x, err)) return;
     reduce_partials(mm.part[y], gridDim.x, K, hs, nullptr);
     if (threadIdx.x < K) hsum[threadIdx.x] = hs[threadIdx.x];
@@ -244,6 +286,7 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
                     }
                     ww[i + u * S] = wv[u];
                 }
+                count(NU * E);
             };
             // backwards after the forward sweep before it, whose last words are still in L2 (odd p): pairs 128x128x32, steps
             // of 10, 7 and 4 vectors 154 -> 142, 93 -> 82, 60 -> 53 us
@@ -266,9 +309,10 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
             w[i] = a;
             ax[K] += a.x * a.x + a.y * a.y;
             dots_of(a, i);
+            count(1);
         }
         double2 *part = mm.part[y] + (p & 1) * set;  // the other set may still be read by a slower block
-        block_reduce_store_r<K, R>(ax, ay, part);
+        block_reduce_store<K>(total, part);
         if (!grid_barrier(L.bar, gridDim.x, err)) return;
         reduce_partials(part, gridDim.x, K, hn, &nrm);
         // gmres.F90:277-280
@@ -298,8 +342,8 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
 
 // ---- start of an inner cycle -----------------------------------------------------------------------
 // Two launches, one before and one after the apply that forms A x0, where a launch per operation (reset, norm, scalars,
-// copy; difference, norm, scalars, column g, scaling) had taken nine of 2-4 us each on a small grid.  Words, sums and
-// their order are those of k_norm2_fused.
+// copy; difference, norm, scalars, column g, scaling) had taken nine of 2-4 us each on a small grid.  A thread sums the
+// words of a round in the vector's precision and the rounds in FP64.
 template <typename C>
 __global__ void __launch_bounds__(kVT) k_begin(Starts<C> s, size_t N, int *err)
 {
@@ -312,9 +356,10 @@ __global__ void __launch_bounds__(kVT) k_begin(Starts<C> s, size_t N, int *err)
     const C *v = s.v[y], *x0 = s.x0[y];
     C *x = s.x[y];
     const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x, Nw = wide_words<C>(N, N);
-    R ax[1] = {R(0)}, ay[1] = {R(0)};
+    double sum = 0.0;
     const W *vw = reinterpret_cast<const W *>(v);
     for (size_t i = t0; i < Nw; i += U * S) {
+        R r = R(0);
         W a[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
@@ -325,11 +370,12 @@ __global__ void __launch_bounds__(kVT) k_begin(Starts<C> s, size_t N, int *err)
 #pragma unroll
                 for (int e = 0; e < E; e++) {
                     const C c = part_of(a[u], e);
-                    ax[0] += c.x * c.x + c.y * c.y;
+                    r += c.x * c.x + c.y * c.y;
                 }
+        sum += r;
     }
-    for (size_t i = Nw * E + t0; i < N; i += S) ax[0] += v[i].x * v[i].x + v[i].y * v[i].y;
-    block_reduce_store_r<0, R>(ax, ay, s.part[y]);
+    for (size_t i = Nw * E + t0; i < N; i += S) sum += v[i].x * v[i].x + v[i].y * v[i].y;
+    block_reduce_store<0>([&](int) { return make_double2(sum, 0.0); }, s.part[y]);
     if (!grid_barrier(L.bar, gridDim.x, err)) return;
     __shared__ double nrm;
     reduce_partials(s.part[y], gridDim.x, 0, nullptr, &nrm);
@@ -371,12 +417,17 @@ __global__ void __launch_bounds__(kVT) k_residual(Starts<C> s, size_t N, double 
     const C *v = s.v[y];
     C *r = s.r[y];
     const size_t S = (size_t)gridDim.x * kVT, t0 = blockIdx.x * (size_t)kVT + threadIdx.x, Nw = wide_words<C>(N, N);
-    R ax[1] = {R(0)}, ay[1] = {R(0)};
+    double sum = 0.0;
+    R round = R(0);
     auto diff = [&](C b, C a) {
         b.x -= a.x;
         b.y -= a.y;
-        ax[0] += b.x * b.x + b.y * b.y;
+        round += b.x * b.x + b.y * b.y;
         return b;
+    };
+    auto add_round = [&] {
+        sum += round;
+        round = R(0);
     };
     const W *vw = reinterpret_cast<const W *>(v);
     W *rw = reinterpret_cast<W *>(r);
@@ -395,9 +446,13 @@ __global__ void __launch_bounds__(kVT) k_residual(Starts<C> s, size_t N, double 
                 for (int e = 0; e < E; e++) set_part(a[u], e, diff(part_of(b[u], e), part_of(a[u], e)));
                 rw[i + u * S] = a[u];
             }
+        add_round();
     }
-    for (size_t i = Nw * E + t0; i < N; i += S) r[i] = diff(v[i], r[i]);
-    block_reduce_store_r<0, R>(ax, ay, s.part[y]);
+    for (size_t i = Nw * E + t0; i < N; i += S) {
+        r[i] = diff(v[i], r[i]);
+        add_round();
+    }
+    block_reduce_store<0>([&](int) { return make_double2(sum, 0.0); }, s.part[y]);
     if (!grid_barrier(L.bar, gridDim.x, err)) return;
     __shared__ double nrm;
     reduce_partials(s.part[y], gridDim.x, 0, nullptr, &nrm);
@@ -435,7 +490,7 @@ int sms()
 
 // a cooperative launch of `kernel` for n instances: as many blocks each as are resident together, up to nparts
 template <typename... P, typename... A>
-int launch(void (*kernel)(P...), int per_sm, size_t words, int n, int nparts, cudaStream_t st, A &&...args)
+int launch(void (*kernel)(P...), int per_sm, size_t smem, size_t words, int n, int nparts, cudaStream_t st, A &&...args)
 {
     const size_t need = (words + kVT - 1) / kVT;
     int g = per_sm * sms() / n;
@@ -444,6 +499,7 @@ int launch(void (*kernel)(P...), int per_sm, size_t words, int n, int nparts, cu
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(g < 1 ? 1 : g, n);
     cfg.blockDim = dim3(kVT);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeCooperative;
@@ -454,17 +510,26 @@ int launch(void (*kernel)(P...), int per_sm, size_t words, int n, int nparts, cu
     g2_count_launches(1);
     return G2_OK;
 }
-template <typename F>
-int per_sm_of(F kernel)
+// resident blocks per SM; kept once the calls have succeeded
+template <typename F> int per_sm_of(F kernel, size_t smem, std::atomic<int> &kept, int *out)
 {
-    int b = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kVT, 0) == cudaSuccess && b > 0 ? b : 1;
+    if (!(*out = kept.load())) {
+        if (smem)
+            G2_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        G2_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(out, kernel, kVT, smem));
+        if (*out < 1) *out = 1;
+        kept = *out;
+    }
+    return G2_OK;
 }
 template <typename C, int K>
 int launch_step(const Multi<C> &mm, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st)
 {
-    static const int per_sm = per_sm_of(k_arnoldi<C, K>);
-    return launch(k_arnoldi<C, K>, per_sm, N / Wide<C>::E + 1, n, nparts, st, mm, N, tol, err);
+    constexpr size_t smem = sums_bytes<C, K>();
+    static std::atomic<int> kept{0};
+    int per_sm;
+    if (const int rc = per_sm_of(k_arnoldi<C, K>, smem, kept, &per_sm)) return rc;
+    return launch(k_arnoldi<C, K>, per_sm, smem, N / Wide<C>::E + 1, n, nparts, st, mm, N, tol, err);
 }
 template <typename C>
 int dispatch(const Multi<C> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
@@ -521,14 +586,18 @@ int arnoldi_step(const Multi<double2> &mm, int n, size_t N, int nparts, int j, d
 
 template <typename C> int krylov_begin(const Starts<C> &s, int n, size_t N, int nparts, int *err, cudaStream_t st)
 {
-    static const int per_sm = per_sm_of(k_begin<C>);
-    return launch(k_begin<C>, per_sm, N / Wide<C>::E + 1, n, nparts, st, s, N, err);
+    static std::atomic<int> kept{0};
+    int per_sm;
+    if (const int rc = per_sm_of(k_begin<C>, 0, kept, &per_sm)) return rc;
+    return launch(k_begin<C>, per_sm, 0, N / Wide<C>::E + 1, n, nparts, st, s, N, err);
 }
 template <typename C>
 int krylov_residual(const Starts<C> &s, int n, size_t N, int nparts, double tol, int *err, cudaStream_t st)
 {
-    static const int per_sm = per_sm_of(k_residual<C>);
-    return launch(k_residual<C>, per_sm, N / Wide<C>::E + 1, n, nparts, st, s, N, tol, err);
+    static std::atomic<int> kept{0};
+    int per_sm;
+    if (const int rc = per_sm_of(k_residual<C>, 0, kept, &per_sm)) return rc;
+    return launch(k_residual<C>, per_sm, 0, N / Wide<C>::E + 1, n, nparts, st, s, N, tol, err);
 }
 template int krylov_begin(const Starts<float2> &, int, size_t, int, int *, cudaStream_t);
 template int krylov_begin(const Starts<double2> &, int, size_t, int, int *, cudaStream_t);

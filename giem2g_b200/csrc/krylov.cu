@@ -9,7 +9,8 @@
 // passes, stop when 2||w|| > ||h_pass||; each pass after the first is ONE sweep over the basis that
 // subtracts V h, and accumulates the next pass's dots and ||w||^2.  Complex Givens rotations follow
 // the netlib ZROTG/ZROT definitions; restarts use the Arnoldi residual (RESTART_RESIDUAL = .FALSE.).
-// Dot products accumulate in FP64 for both precisions.
+// Dot products and norms: complex128 in FP64; complex64 up to 16 elements of a thread in FP32 (arnoldi.cu; the norms of
+// k_norm2_fused: a thread's part of the vector), their sums in FP64.
 //
 // The inner solve is a fixed launch sequence whose kernels are gated by device flags, so it needs no
 // host round trip; the outer loop reads two scalars back once per outer iteration (Inform callback).

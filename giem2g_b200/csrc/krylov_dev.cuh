@@ -110,22 +110,20 @@ template <typename C> struct RealOf;
 template <> struct RealOf<double2> { using T = double; };
 template <> struct RealOf<float2> { using T = float; };
 
-// per-thread partial sums in the vector's precision (a handful of elements each), block and grid
-// reductions in FP64
-template <int KM, typename R>
-G2_D void block_reduce_store_r(R (&ax)[KM + 1], R (&ay)[KM + 1], double2 *part)
+// Sums over a block and into its row of the grid's partial sums, in FP64; total(k) is the thread's k-th sum.
+template <int KM, class F> G2_D void block_reduce_store(F total, double2 *part)
 {
     __shared__ double2 red[kVT / 32][KM + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k <= KM; k++) {
-        double vx = ax[k], vy = ay[k];
+        double2 v = total(k);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            vx += __shfl_xor_sync(0xffffffffu, vx, o);
-            vy += __shfl_xor_sync(0xffffffffu, vy, o);
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
         }
-        if (lane == 0) red[warp][k] = make_double2(vx, vy);
+        if (lane == 0) red[warp][k] = v;
     }
     __syncthreads();
     if (threadIdx.x <= KM) {
@@ -136,6 +134,11 @@ G2_D void block_reduce_store_r(R (&ax)[KM + 1], R (&ay)[KM + 1], double2 *part)
         }
         part[(size_t)blockIdx.x * (KMAX + 1) + (threadIdx.x == KM ? KMAX : threadIdx.x)] = s;
     }
+}
+// per-thread sums in the vector's precision
+template <int KM, typename R> G2_D void block_reduce_store_r(R (&ax)[KM + 1], R (&ay)[KM + 1], double2 *part)
+{
+    block_reduce_store<KM>([&](int k) { return make_double2(ax[k], ay[k]); }, part);
 }
 
 // ---- scalar steps -------------------------------------------------------------------------------
