@@ -37,6 +37,15 @@ def _time_rounds(run, stream, reps: int, rounds: int) -> float:
     return best
 
 
+def _cached(cache: dict, key: str, nv: int):
+    """The pick kept under key, if it was made among as many variants as there are now: a pick among other variants
+    may name another kernel."""
+    pick = cache.get(key)
+    if isinstance(pick, dict) and len(pick.get("all_ms") or ()) == nv and pick.get("variant") in range(nv):
+        return pick
+    return None
+
+
 def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, rounds: int = 3) -> dict:
     import torch
 
@@ -56,9 +65,10 @@ def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, round
             picks[prec] = {"variant": 0, "ms": None}
             continue
         ck = f"{key}:{prec}"
-        if ck in cache:
-            op.set_contract_variant(prec, cache[ck]["variant"])
-            picks[prec] = cache[ck]
+        pick = _cached(cache, ck, nv)
+        if pick is not None:
+            op.set_contract_variant(prec, pick["variant"])
+            picks[prec] = pick
             continue
         x = torch.randn(op.nvec, dtype=dt, device="cuda")
         y = torch.empty_like(x)

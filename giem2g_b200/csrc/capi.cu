@@ -440,13 +440,12 @@ static GIEM2G_FGMRES_CTL resolve_precision(const IeOp *op, GIEM2G_FGMRES_CTL ctl
     return ctl;
 }
 
-// Where contract.cu has shapes for Nz, variants [0, n - 1) are those and n - 1 is the tensor-core kernel (the default of
-// a new operator, and the only contraction of other Nz); where the fused pass exists, variants
-// [n, n + ie_ypipe_variants) select it with its own shapes instead of the separate passes.
+// Variant numbers are kept by hosts and in the tuner's files, so they stay what they are.  Where contract.cu has shapes for
+// Nz: 0 is the default of a new operator, the tensor-core kernel; [1, n) are the shapes; [n, n + n_ypipe) the fused pass with
+// its own shapes, where it exists (the last numbers).  Where it does not, n is the default too.
 static int n_contract(const IeOp *op, int precision)
 {
-    const int n = precision == 2 ? ie_contract_pair_variants(op->Nz) : ie_contract_variants(precision, op->Nz);
-    return n ? n + 1 : 0;
+    return precision == 2 ? ie_contract_pair_variants(op->Nz) : ie_contract_variants(precision, op->Nz);
 }
 static int n_ypipe(const IeOp *op, int precision)
 {
@@ -457,13 +456,13 @@ int giem2g_set_contract_variant(void *ie, int precision, int variant)
 {
     IeOp *op = resolve(ie);
     if (!op || precision < 0 || precision > 2) return fail(G2_ERR_ARG, "giem2g_set_contract_variant: bad arguments");
-    const int n = n_contract(op, precision), ny = n_ypipe(op, precision);
-    if (variant < 0 || (variant > 0 && variant >= n + ny))
-        return fail(G2_ERR_ARG, "giem2g_set_contract_variant: variant %d of %d", variant, n + ny);
+    const int n = n_contract(op, precision), ny = n_ypipe(op, precision), all = giem2g_contract_variants(ie, precision);
+    if (variant < 0 || (variant > 0 && variant >= all))
+        return fail(G2_ERR_ARG, "giem2g_set_contract_variant: variant %d of %d", variant, all);
     if (variant >= n && ny > 0) {
         op->ypipe_mode[precision] = variant - n;
     } else {
-        op->contract_variant[precision] = variant >= n - 1 ? -1 : variant;
+        op->contract_variant[precision] = variant >= 1 && variant < n ? variant : -1;
         op->ypipe_mode[precision] = -1;
     }
     op->config_gen++;
@@ -513,7 +512,8 @@ int giem2g_contract_variants(void *ie, int precision)
 {
     IeOp *op = resolve(ie);
     if (!op || precision < 0 || precision > 2) return 0;
-    return n_contract(op, precision) + n_ypipe(op, precision);
+    const int n = n_contract(op, precision), ny = n_ypipe(op, precision);
+    return n && !ny ? n + 1 : n + ny;
 }
 
 int giem2g_check_device_error(void *ie)

@@ -684,6 +684,9 @@ int sm_count()
 
 // Tile-shape variants per (precision, Nz); variant 0 is the default.  The autotuner times the variants
 // on the operator's own buffers and stores its pick in the operator.
+// (0 stands for the tensor-core kernel in every count below: it took the place of the first shape, which was the slower one
+// at every Nz and in every form: 128x128 whole applies, default against that shape, FP64 / complex64 / pair: Nz = 8 64 / 50 /
+// 62 against 73 / 51 / 69 us, 16 116 / 80 / 111 against 142 / 89 / 150, 32 322 / 200 / 286 against 382 / 231 / 395.)
 int ie_contract_variants(int precision, int Nz)
 {
     if (precision == 0) return Nz == 32 ? 12 : (Nz == 8 || Nz == 16 || Nz == 48 ? 2 : 0);
@@ -698,13 +701,13 @@ int ie_contract_fast64(const double2 *G, double2 *Uhat, int Nx, int Ny, int Nz, 
     switch (Nz) {
     case 8:
         if (v == 1) return launch_wl<double, 8, 4, 8, 16>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<double, 8, 2, 8, 4>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 16:
         if (v == 1) return launch_wl<double, 16, 4, 4, 8>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<double, 16, 4, 4, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 48:
         if (v == 1) return launch_wl<double, 48, 4, 1, 1>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<double, 48, 4, 1, 1>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 32:
         if (v == 1) return launch_cfg<double, 32, 4, 1, 3>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_cfg<double, 32, 4, 1, 1, 1, false, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
@@ -717,7 +720,7 @@ int ie_contract_fast64(const double2 *G, double2 *Uhat, int Nx, int Ny, int Nz, 
         if (v == 9) return launch_wl<double, 32, 2, 4, 3>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 10) return launch_wl<double, 32, 4, 2, 3, 1, 1, true>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 11) return launch_wl<double, 32, 4, 2, 3, 1, 1, false, false, 1, 4>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<double, 32, 8, 1, 3>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     default: return G2_ERR_UNSUPPORTED;
     }
 }
@@ -731,12 +734,12 @@ int ie_contract_fast32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, in
         if (v == 1) return launch_w32<8, 2, 16, 3, 1>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_wl<float, 8, 4, 8, 16>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 3) return launch_wl<float, 8, 4, 8, 16, 1, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 8, 2, 16, 4>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 16:
         if (v == 1) return launch_w32<16, 4, 4, 4, 1>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_wl<float, 16, 2, 8, 8>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 3) return launch_wl<float, 16, 2, 8, 8, 1, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 16, 4, 4, 4>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 32:
         switch (v) {
         case 1: return launch_cfg<float, 32, 4, 1, 5>(G, Uhat, Nx, Ny, err, n, st, gate);
@@ -763,21 +766,20 @@ int ie_contract_fast32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, in
         case 22: return launch_wl<float, 32, 2, 4, 6, 1, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
         case 23: return launch_wl<float, 32, 4, 4, 6, 1, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
         case 24: return launch_wl<float, 32, 2, 6, 6, 1, 1, false, true, 1, 4>(G, Uhat, Nx, Ny, err, n, st, gate);
-        default: return launch_cfg<float, 32, 8, 1, 5>(G, Uhat, Nx, Ny, err, n, st, gate);
+        default: return G2_ERR_UNSUPPORTED;
         }
     case 48:
         if (v == 1) return launch_w32<48, 4, 1, 2, 1>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_wl<float, 48, 4, 2, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 3) return launch_wl<float, 48, 4, 2, 2, 1, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 48, 4, 1, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     default: return G2_ERR_UNSUPPORTED;
     }
 }
 
 // Two vectors of one operator per tensor read (complex64; both polarisations of a plane-wave source).
-// The spectrum holds [unit][slot][vector][3Nz].  Variants: 0 the direct kernel with the two vectors spread
-// over threads, 1 the direct kernel with both vectors in each thread's registers, 2 (and 3) the
-// Walsh-basis packed kernel.
+// The spectrum holds [unit][slot][vector][3Nz].  Variants: 1 the direct kernel with both vectors in each thread's
+// registers, 2 (and 3) the Walsh-basis packed kernel.
 int ie_contract_pair_variants(int Nz) { return Nz == 32 ? 21 : (Nz == 48 ? 6 : ((Nz == 8 || Nz == 16) ? 4 : 0)); }
 int ie_contract_pair32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, int *err, cudaStream_t st,
                        const int *gate, int v)
@@ -788,12 +790,12 @@ int ie_contract_pair32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, in
         if (v == 1) return launch_cfg<float, 8, 1, 16, 3, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_w32<8, 1, 16, 2, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 3) return launch_wl<float, 8, 4, 8, 16, 2, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 8, 1, 16, 3, 2, true>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 16:
         if (v == 1) return launch_cfg<float, 16, 2, 4, 4, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_w32<16, 2, 4, 4, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 3) return launch_wl<float, 16, 2, 4, 8, 2, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 16, 2, 4, 4, 2, true>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 32:
         if (v == 1) return launch_cfg<float, 32, 4, 1, 5, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_w32<32, 4, 2, 2, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
@@ -817,7 +819,7 @@ int ie_contract_pair32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, in
         if (v == 19) return launch_wl<float, 32, 4, 2, 5, 2, 1, false, true, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         // variant 14 with four j iterations unrolled together
         if (v == 20) return launch_wl<float, 32, 2, 4, 5, 2, 1, false, true, 1, 4>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 32, 4, 2, 2, 2, true>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     case 48:
         if (v == 1) return launch_cfg<float, 48, 4, 1, 2, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 2) return launch_w32<48, 4, 1, 2, 2>(G, Uhat, Nx, Ny, err, n, st, gate);
@@ -826,7 +828,7 @@ int ie_contract_pair32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, in
         // 256x256x48 (standalone timing of the contraction alone)
         if (v == 4) return launch_wl<float, 48, 4, 2, 2, 2, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
         if (v == 5) return launch_wl<float, 48, 8, 1, 2, 2, 1, false, true>(G, Uhat, Nx, Ny, err, n, st, gate);
-        return launch_cfg<float, 48, 4, 1, 2, 2, true>(G, Uhat, Nx, Ny, err, n, st, gate);
+        return G2_ERR_UNSUPPORTED;
     default: return G2_ERR_UNSUPPORTED;
     }
 }

@@ -111,8 +111,8 @@ int giem2g_apply_ie_operator_device_static(void *ie, const void *d_in, void *d_o
  * out) as a nonzero status. */
 int giem2g_check_device_error(void *ie);
 /* Contraction tile-shape variants available for a precision (0 or 1) at this Nz, and selection of one
- * (what the autotuner in giem2g_b200.autotune sets after timing them).  Without a selection the contraction
- * runs on the tensor cores, at every Nz; where there are variants that kernel is one of them. */
+ * (what the autotuner in giem2g_b200.autotune sets after timing them).  Variant 0 is the default, as
+ * without a selection: the tensor-core kernel, at every Nz. */
 int giem2g_contract_variants(void *ie, int precision);  /* precision 2: paired complex64 */
 int giem2g_set_contract_variant(void *ie, int precision, int variant);
 /* Lines per CTA of the FFT passes (4, 8, 16 or 32; default: 8 complex128, 16 complex64), also set by the autotuner: for both
