@@ -8,6 +8,11 @@ buffers and keeps the fastest in the operator; results are cached per (Nx, Ny, N
 file next to this module when one is given.  Each candidate is timed in `rounds` rounds of `reps` full
 applies and scored by its fastest round, so a transient slowdown (another process, a clock dip) during
 one round does not decide the pick.
+
+The tensor-core kernel (variant 0) reads another layout of the tensor than the shapes of the other kernels.  Where the
+complex64 and the paired apply are fastest with different ones, the operator holds a second complex64 tensor (0.5 GB at
+128x128x32, 4.9 GB at 256x256x48); the tuner takes that only where it is a small part of the free memory, and otherwise
+keeps both on the layout of the faster paired apply.
 """
 from __future__ import annotations
 
@@ -46,6 +51,21 @@ def _cached(cache: dict, key: str, nv: int):
     return None
 
 
+COPY_SHARE = 32  # a second complex64 tensor may take 1/COPY_SHARE of the free memory
+
+
+def _second_tensor_fits(op, free_bytes: int) -> bool:
+    return COPY_SHARE * 8 * op.Nx * op.Ny * 2 * op.Nz * (2 * op.Nz + 1) <= free_bytes
+
+
+def _one_layout(single_ms, pair_ms):
+    """The picks of the complex64 and the paired apply that read the same layout: the fastest paired one, and the fastest
+    single one of its layout (0 reads one, all others the other)."""
+    pair = min(range(len(pair_ms)), key=pair_ms.__getitem__)
+    group = [0] if pair == 0 else range(1, len(single_ms))
+    return min(group, key=single_ms.__getitem__), pair
+
+
 def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, rounds: int = 3) -> dict:
     import torch
 
@@ -58,7 +78,7 @@ def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, round
             cache = {}
     stream = torch.cuda.ExternalStream(op.stream)
     picks = {}
-    from . import apply_device_batch
+    from . import Giem2gError, apply_device_batch
     for prec, dt in ((0, torch.complex128), (1, torch.complex64), (2, torch.complex64)):
         nv = op.contract_variants(prec)
         if nv <= 1:
@@ -82,13 +102,25 @@ def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, round
 
         best, all_ms = None, []
         for v in range(nv):
-            op.set_contract_variant(prec, v)
+            try:
+                op.set_contract_variant(prec, v)
+            except Giem2gError:
+                if v == 0:
+                    raise
+                all_ms.append(float("inf"))  # no memory for its layout of the tensor
+                continue
             ms = _time_rounds(run, stream, reps, rounds)
             all_ms.append(round(ms, 5))
             if best is None or ms < best[1]:
                 best = (v, ms)
         op.set_contract_variant(prec, best[0])
         picks[prec] = {"variant": best[0], "ms": best[1], "all_ms": all_ms}
+        if prec == 2 and (picks[1]["variant"] == 0) != (best[0] == 0) and len(picks[1].get("all_ms") or ()) > 1 \
+                and not _second_tensor_fits(op, torch.cuda.mem_get_info()[0]):
+            for q, v in zip((1, 2), _one_layout(picks[1]["all_ms"], all_ms)):
+                op.set_contract_variant(q, v)
+                picks[q] = dict(picks[q], variant=v, ms=picks[q]["all_ms"][v])
+                cache[f"{key}:{q}"] = picks[q]
         cache[ck] = picks[prec]
     # FFT lines per CTA, per precision: complex64 timed on the paired apply (the inner solver's), complex128
     # on the FP64 apply; the shared-memory tile per line doubles with the element size, so they can differ

@@ -343,8 +343,7 @@ __global__ void k_sigma(const double2 *__restrict__ csiga, const double2 *__rest
 
 template <typename R> struct Bufs;
 template <> struct Bufs<double> {
-    static const double2 *G(IeOp *o) { return o->d_tensor64; }
-    static const double2 *plain(IeOp *o) { return o->d_plain64; }
+    static const double2 *G(IeOp *o, int layout) { return o->d_tensor64[layout]; }
     static const double2 *gsig(IeOp *o) { return o->d_gsig64; }
     static const double2 *asig(IeOp *o) { return o->d_asig64; }
     static const double *post(IeOp *o) { return o->d_post64; }
@@ -352,8 +351,7 @@ template <> struct Bufs<double> {
     static const double2 *twy(IeOp *o) { return o->d_twy64; }
 };
 template <> struct Bufs<float> {
-    static const float2 *G(IeOp *o) { return o->d_tensor32; }
-    static const float2 *plain(IeOp *o) { return o->d_plain32; }
+    static const float2 *G(IeOp *o, int layout) { return o->d_tensor32[layout]; }
     static const float2 *gsig(IeOp *o) { return o->d_gsig32; }
     static const float2 *asig(IeOp *o) { return o->d_asig32; }
     static const float *post(IeOp *o) { return o->d_post32; }
@@ -517,7 +515,7 @@ static int ie_apply_core(IeOp *op, const CT<R> *d_in, CT<R> *d_out, cudaStream_t
     const size_t es = sizeof(CT<R>);
     const int form = sizeof(R) == 8 ? 0 : 1;
     const bool mma = ie_uses_mma(op, form);
-    const CT<R> *G = mma ? Bufs<R>::G(op) : Bufs<R>::plain(op);
+    const CT<R> *G = Bufs<R>::G(op, mma ? L_TILED : L_PLAIN);
     if (!G || !U1 || !Uh) return G2_ERR_STATE;
     const int pitch = mma ? ie_spectrum_pitch(Nz) : Z3;
     VecSet<CT<R>> vs{{d_in, nullptr}, {d_out, nullptr}, 1};
@@ -741,7 +739,7 @@ int ie_apply_pair32(IeOp *op, const float2 *in0, const float2 *in1, float2 *out0
     const bool mma = ie_uses_mma(op, 2);
     if (!mma && (!op->use_fast_contract || !ie_contract_pair32_supported(op->Nx, op->Ny, op->Nz)))
         return G2_ERR_UNSUPPORTED;
-    const float2 *G = mma ? op->d_tensor32 : op->d_plain32;
+    const float2 *G = op->d_tensor32[mma ? L_TILED : L_PLAIN];
     if (!G || !U1 || !Uh) return G2_ERR_STATE;
     const int pitch = mma ? ie_spectrum_pitch(op->Nz) : 3 * op->Nz;
     VecSet<float2> vs{{in0, in1}, {out0, out1}, 2};

@@ -244,8 +244,8 @@ int giem2g_set_ie_kernel_spatial(void *ie, const void *symm, const void *asym)
     return set_status(0);
 }
 
-// the unit tensor d in the reference's arrays; tiled: d is the spectral tensor (unit_pos), else the spatial one
-static int get_units(IeOp *op, const double2 *d, void *symm, void *asym, bool tiled)
+// the unit tensor d in the reference's arrays; layout: the spectral tensor's, or -1 for the spatial one
+static int get_units(IeOp *op, const double2 *d, void *symm, void *asym, int layout)
 {
     const int P = op->P(), Nz = op->Nz, T = op->Tunit();
     const size_t U = op->units();
@@ -255,7 +255,7 @@ static int get_units(IeOp *op, const double2 *d, void *symm, void *asym, bool ti
         return fail(G2_ERR_CUDA, "tensor download failed");
     double2 *s = reinterpret_cast<double2 *>(symm), *a = reinterpret_cast<double2 *>(asym);
     std::vector<int> pos(T);
-    for (int e = 0; e < T; e++) pos[e] = tiled ? unit_pos<true>(e, Nz) : e;
+    for (int e = 0; e < T; e++) pos[e] = layout < 0 ? e : (layout == L_TILED ? unit_pos<true>(e, Nz) : plain_pos<true>(e, Nz));
     for (size_t u = 0; u < U; u++) {
         for (int e = 0; e < 4 * P; e++) s[u * 4 * P + e] = h[u * T + pos[e]];
         for (int e = 4 * P; e < T; e++) a[u * 2 * Nz * Nz + e - 4 * P] = h[u * T + pos[e]];
@@ -267,14 +267,15 @@ int giem2g_get_ie_kernel_spatial(void *ie, void *symm, void *asym)
 {
     IeOp *op = resolve(ie);
     if (!op || !op->have_spatial) return fail(G2_ERR_STATE, "giem2g_get_ie_kernel_spatial: no spatial tensor");
-    return get_units(op, op->d_spatial, symm, asym, false);
+    return get_units(op, op->d_spatial, symm, asym, -1);
 }
 
 int giem2g_get_ie_kernel_spectral(void *ie, void *symm, void *asym)
 {
     IeOp *op = resolve(ie);
     if (!op || !op->have_spectral) return fail(G2_ERR_STATE, "giem2g_get_ie_kernel_spectral: no spectral tensor");
-    return get_units(op, op->d_tensor64, symm, asym, true);
+    const int layout = op->d_tensor64[L_TILED] ? L_TILED : L_PLAIN;
+    return get_units(op, op->d_tensor64[layout], symm, asym, layout);
 }
 
 void giem2g_calc_fft_of_ie_kernel(void *ie)
@@ -306,6 +307,15 @@ void giem2g_set_anomaly_conductivity(void *ie, void *csiga)
     set_status(0);
 }
 
+// An apply that the host captures becomes part of a graph that the library does not know: from then on no tensor that the
+// graph may read is moved, re-laid or freed.
+static void note_capture(IeOp *op)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!op->captured && cudaStreamIsCapturing(op->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive)
+        op->captured = true;
+}
+
 static int check_ready(IeOp *op, const char *who)
 {
     if (!op) return fail(G2_ERR_STATE, "%s: no operator", who);
@@ -321,6 +331,7 @@ int giem2g_apply_ie_operator_device(void *ie, const void *d_in, void *d_out, int
     if (rc) return rc;
     if (precision != 0 && precision != 1)
         return fail(G2_ERR_ARG, "giem2g_apply_ie_operator_device: precision must be 0 or 1");
+    note_capture(op);
     cudaEventRecord(op->ev0, op->stream);
     if (precision == 0)
         rc = ie_apply_device64(op, reinterpret_cast<const double2 *>(d_in), reinterpret_cast<double2 *>(d_out), op->stream);
@@ -343,6 +354,7 @@ int giem2g_apply_ie_operator_device_static(void *ie, const void *d_in, void *d_o
     if (rc) return rc;
     if (precision != 0 && precision != 1)
         return fail(G2_ERR_ARG, "giem2g_apply_ie_operator_device_static: precision must be 0 or 1");
+    note_capture(op);
     void *base = nullptr;
     size_t cap = 0, n_u1 = 0;
     rc = ie_static_scratch(&base, &cap);
@@ -459,15 +471,20 @@ int giem2g_set_contract_variant(void *ie, int precision, int variant)
     const int n = n_contract(op, precision), ny = n_ypipe(op, precision), all = giem2g_contract_variants(ie, precision);
     if (variant < 0 || (variant > 0 && variant >= all))
         return fail(G2_ERR_ARG, "giem2g_set_contract_variant: variant %d of %d", variant, all);
+    const int old_variant = op->contract_variant[precision], old_ypipe = op->ypipe_mode[precision];
     if (variant >= n && ny > 0) {
         op->ypipe_mode[precision] = variant - n;
     } else {
         op->contract_variant[precision] = variant >= 1 && variant < n ? variant : -1;
         op->ypipe_mode[precision] = -1;
     }
+    const int rc = ie_sync_layouts(op);
+    if (rc) {  // the selection stays what it was
+        op->contract_variant[precision] = old_variant;
+        op->ypipe_mode[precision] = old_ypipe;
+        return fail(rc, "giem2g_set_contract_variant: %s", giem2g_last_error());
+    }
     op->config_gen++;
-    const int rc = ie_sync_plain(op);
-    if (rc) return fail(rc, "giem2g_set_contract_variant: %s", giem2g_last_error());
     return set_status(0);
 }
 
@@ -644,6 +661,7 @@ int giem2g_apply_ie_operator_device_batch(void *ie, int nv, const void *const *d
     if (rc) return rc;
     if (nv < 1 || !d_in || !d_out || (precision != 0 && precision != 1))
         return fail(G2_ERR_ARG, "giem2g_apply_ie_operator_device_batch: bad arguments");
+    note_capture(op);
     cudaEventRecord(op->ev0, op->stream);
     int i = 0;
     if (precision == 1) {
@@ -927,11 +945,10 @@ void giem2g_delete_ie_operator(void *ie)
     g2_pool_free(op->d_spatial, op->stream);
     if (op->stream) cudaStreamSynchronize(op->stream);
     if (op->pool) cudaMemPoolDestroy(op->pool);
-    void *ptrs[] = {op->d_tensor64, op->d_tensor32, op->d_csiga, op->d_gsig64, op->d_asig64,
+    void *ptrs[] = {op->d_tensor64[0], op->d_tensor64[1], op->d_tensor32[0], op->d_tensor32[1], op->d_csiga, op->d_gsig64, op->d_asig64,
                     op->d_gsig32, op->d_asig32, op->d_post64, op->d_post32, op->d_twx64, op->d_twy64,
                     op->d_twx32, op->d_twy32, op->scratch.U1, op->scratch.Uhat, op->pair_scratch.U1,
-                    op->pair_scratch.Uhat, op->d_vin, op->d_vout, op->d_err, op->d_vin32, op->d_vout32, op->d_pos, op->d_plain64,
-                    op->d_plain32};
+                    op->pair_scratch.Uhat, op->d_vin, op->d_vout, op->d_err, op->d_vin32, op->d_vout32, op->d_pos};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (op->ev0) cudaEventDestroy(op->ev0);

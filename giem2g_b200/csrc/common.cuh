@@ -133,7 +133,7 @@ template <bool F64> G2_HD int unit_pos(int e, int Nz)
     return 4 * P + blk * Nz * Nz + full_pos<F64>(rc % Nz, rc / Nz, Nz);
 }
 
-// Layout of the copy that the other contraction kernels read: packed upper blocks as they are, and
+// Layout of the units that the other contraction kernels read: packed upper blocks as they are, and
 // the full (xz, yz) Nz x Nz blocks column-major with the row index XOR-swizzled by
 // the low bits of the column, so lane-parallel reads of a row and of a column both hit distinct
 // shared-memory banks.  W = 1 is plain column-major.
@@ -141,6 +141,15 @@ G2_HD int asw(int r, int c, int N, int W) { return c * N + (r ^ (c & (W - 1))); 
 // swizzle widths used for the FP64 and FP32 device tensors
 __host__ __device__ constexpr int asw_width64(int Nz) { return (Nz % 8 == 0) ? 8 : 1; }
 __host__ __device__ constexpr int asw_width32(int Nz) { return (Nz % 16 == 0) ? 16 : ((Nz % 8 == 0) ? 8 : 1); }
+
+// position of the spatial tensor's element e in a unit of that layout
+template <bool F64> G2_HD int plain_pos(int e, int Nz)
+{
+    const int P4 = 2 * Nz * (Nz + 1);
+    if (e < P4) return e;
+    const int li = e - P4, blk = li / (Nz * Nz), rc = li - blk * Nz * Nz;
+    return P4 + blk * Nz * Nz + asw(rc % Nz, rc / Nz, Nz, F64 ? asw_width64(Nz) : asw_width32(Nz));
+}
 
 #define G2_CUDA_CHECK(expr)                                                                    \
     do {                                                                                       \

@@ -35,12 +35,13 @@ struct IeOp {
     // device data
     cudaMemPool_t pool = nullptr;      // temporaries of the set-up, and the spatial tensor
     double2 *d_spatial = nullptr;      // [Nx][Ny][Tunit] FP64 spatial tensor (from the pool)
-    double2 *d_tensor64 = nullptr;     // [Nx][Ny][Tunit] FP64 spectral tensor
-    float2 *d_tensor32 = nullptr;      // same, complex64 copy
-    // copies in the layout of the other contraction kernels, held while a form of that precision selects one
-    ushort2 *d_pos = nullptr;          // a unit element's place in d_tensor64 (x) and d_tensor32 (y)
-    double2 *d_plain64 = nullptr;
-    float2 *d_plain32 = nullptr;
+    // [Nx][Ny][Tunit] spectral tensor, FP64 and its complex64 copy, per layout of a unit: L_TILED for the tensor-core
+    // contraction, L_PLAIN for the others.  Each is held in the layout that the selected contractions read; in both, one
+    // per precision more, where the complex64 and the paired form read different ones or an apply was captured before.
+    double2 *d_tensor64[2] = {nullptr, nullptr};
+    float2 *d_tensor32[2] = {nullptr, nullptr};
+    ushort4 *d_pos = nullptr;          // a unit element's places: tiled FP64, tiled complex64, plain FP64, plain complex64
+    bool captured = false;             // the host captured an apply: a graph of its own may read the tensors
     double2 *d_csiga = nullptr;        // [Nz][Ny][Nx]
     double2 *d_gsig64 = nullptr, *d_asig64 = nullptr;  // per-cell pre/post coefficients
     float2 *d_gsig32 = nullptr, *d_asig32 = nullptr;
@@ -156,8 +157,10 @@ int ie_contract_variants(int precision, int Nz);
 // spectrum rows (one point of one vector: 3Nz elements) are ie_spectrum_pitch(Nz) elements apart.
 int ie_spectrum_pitch(int Nz);
 bool ie_uses_mma(const IeOp *op, int form);
-// Makes or frees the plain-layout copies (d_plain64, d_plain32) for the selected contractions; not during a capture.
-int ie_sync_plain(IeOp *op);
+enum { L_TILED = 0, L_PLAIN = 1 };
+// Brings the tensors into the layouts that the selected contractions read; not during a capture.  alloc: makes them
+// first, where there are none.  On failure the tensors are as they were.
+int ie_sync_layouts(IeOp *op, bool alloc = false);
 int ie_contract_mma(int form, const void *G, void *Uhat, int Nx, int Ny, int Nz, int *err, cudaStream_t st,
                     const int *gate);
 
