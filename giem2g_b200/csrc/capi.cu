@@ -944,7 +944,7 @@ void giem2g_delete_ie_operator(void *ie)
     krylov_free(op);
     g2_pool_free(op->d_spatial, op->stream);
     if (op->stream) cudaStreamSynchronize(op->stream);
-    if (op->pool) cudaMemPoolDestroy(op->pool);
+    g2_pool_release(&op->pool);
     void *ptrs[] = {op->d_tensor64[0], op->d_tensor64[1], op->d_tensor32[0], op->d_tensor32[1], op->d_csiga, op->d_gsig64, op->d_asig64,
                     op->d_gsig32, op->d_asig32, op->d_post64, op->d_post32, op->d_twx64, op->d_twy64,
                     op->d_twx32, op->d_twy32, op->scratch.U1, op->scratch.Uhat, op->pair_scratch.U1,

@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 #include "common.cuh"
 #include "ie_internal.h"
@@ -511,7 +512,7 @@ struct RcOp {
     double2 *d_E = nullptr, *d_Ea = nullptr, *d_Ha = nullptr;  // staging of the host-buffer entry
     std::vector<double2> csigb;  // per cell
     cudaStream_t stream = nullptr;
-    cudaMemPool_t pool = nullptr;  // temporaries of the tensor
+    G2Pool *pool = nullptr;  // temporaries of the tensor
 
     size_t npts() const { return (size_t)4 * Nx * Ny; }
     size_t E() const { return (size_t)RC_NCOMP * Nr * Nz; }
@@ -575,7 +576,7 @@ void rc_delete(RcOp *op)
                     op->d_E, op->d_Ea, op->d_Ha};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    if (op->pool) cudaMemPoolDestroy(op->pool);
+    g2_pool_release(&op->pool);
     if (op->stream) cudaStreamDestroy(op->stream);
     delete op;
 }
@@ -650,7 +651,8 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
     for (int iz = 1; iz <= Nz; iz++) op->csigb[iz - 1] = csigma[Lnumber[iz]];  // FinalizeRCOperator :178-181
     std::vector<RcRecvDev> rv(Nr);
     for (int r = 0; r < Nr; r++) rv[r] = RcRecvDev{op->recv[r].zrecv, op->recv[r].recv_layer, op->recv[r].anom_cell};
-    VbtTab *tab = new VbtTab();
+    const std::unique_ptr<VbtTab> table(new VbtTab());
+    VbtTab *tab = table.get();
     // VBTransformInit(rmin) with rmin = sqrt(dx^2 + dy^2) / 2 (calc_rc_tensor_module.F90:79-80)
     make_vbt(std::sqrt(op->dx * op->dx + op->dy * op->dy) / 2.0, *tab);
 
@@ -669,7 +671,6 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
         g2_pool_free(d_B, st);
         g2_pool_free(d_W, st);
         g2_pool_free(d_range, st);
-        delete tab;
     };
 #define RC_TRY2(expr)                                                     \
     do {                                                                  \
@@ -749,9 +750,9 @@ int rc_calc_kernel(RcOp *op, int Nl, const double2 *csigma, const double *thick,
         RC_TRY2(launch_gemm(jobs, NT, d_range, (int)npts, op->d_G, E, sc, st));
         launches++;
     }
-    RC_TRY2(cudaStreamSynchronize(st));
+    cleanup();  // before the synchronisation, which gives back what the pool does not keep
+    RC_TRY(cudaStreamSynchronize(st));
     g2_count_launches(launches);
-    cleanup();
 #undef RC_TRY2
 #undef RC_TRY2_RC
     op->have_tensor = true;

@@ -18,6 +18,7 @@
 // A lambda that the reference skips for a lag has all six weights zero here, so the sums hold the
 // same terms; only the order of the floating-point additions differs.
 #include <cmath>
+#include <memory>
 #include <vector>
 #include <cuda/std/complex>
 #include "common.cuh"
@@ -374,7 +375,8 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
         h.z[i] = op->z[i];
     }
     for (int i = 1; i <= Nz; i++) h.dz[i] = op->z[i] - op->z[i - 1];
-    VbtTab *tab = new VbtTab();
+    const std::unique_ptr<VbtTab> table(new VbtTab());
+    VbtTab *tab = table.get();
     make_vbt(std::sqrt(op->dx * op->dx + op->dy * op->dy) / 2.0, *tab);  // calc_ie_tensor_module.F90:102-103
 
     Bkg *d_bkg = nullptr;
@@ -389,7 +391,6 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
         for (auto p : M) g2_pool_free(p, st);
         g2_pool_free(W, st);
         g2_pool_free(krange, st);
-        delete tab;
     };
 #define G2_TRY(expr)                                                      \
     do {                                                                  \
@@ -438,8 +439,8 @@ int ie_green_tensor(IeOp *op, cudaStream_t st)
     add_job(jobs, NT, Wt(IE_DY), M[2], nullptr, nullptr, Nz * Nz, 4 * P + Nz * Nz);     // yz
     G2_TRY(launch_gemm(jobs, NT, krange, (int)lags, op->d_spatial, T, sc, st));
     G2_TRY(cudaGetLastError());
-    G2_TRY(cudaStreamSynchronize(st));
-    cleanup();
+    cleanup();  // before the synchronisation, which gives back what the pool does not keep
+    G2_CUDA_CHECK(cudaStreamSynchronize(st));
 #undef G2_TRY
 #undef G2_TRY_RC
     return rc;

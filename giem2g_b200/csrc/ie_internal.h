@@ -8,9 +8,12 @@
 enum { G2_OK = 0, G2_ERR_ARG = -1, G2_ERR_CUDA = -2, G2_ERR_STATE = -3, G2_ERR_UNSUPPORTED = -4,
        G2_ERR_NUMERIC = -5, G2_ERR_NOMEM = -6 };
 
-// mem_pool.cu: stream-ordered temporaries of one operator (the pool is made on first use)
-int g2_pool_alloc(cudaMemPool_t *pool, void **p, size_t bytes, cudaStream_t st);
+// mem_pool.cu: stream-ordered temporaries from the device's pool, which an operator (ref) holds from its first use to its end.
+// A buffer is freed on the stream it is used on; free before the call's last synchronisation, which gives memory back.
+struct G2Pool;
+int g2_pool_alloc(G2Pool **ref, void **p, size_t bytes, cudaStream_t st);
 void g2_pool_free(void *p, cudaStream_t st);
+void g2_pool_release(G2Pool **ref);
 
 struct ApplyScratch {
     void *U1 = nullptr;    // [2Nx][3Nz][Ny]   x-spectrum / inverse-y output
@@ -33,7 +36,7 @@ struct IeOp {
     bool have_background = false;
     bool have_spatial = false, have_spectral = false, have_sigma = false;
     // device data
-    cudaMemPool_t pool = nullptr;      // temporaries of the set-up, and the spatial tensor
+    G2Pool *pool = nullptr;            // temporaries of the set-up, and the spatial tensor
     double2 *d_spatial = nullptr;      // [Nx][Ny][Tunit] FP64 spatial tensor (from the pool)
     // [Nx][Ny][Tunit] spectral tensor, FP64 and its complex64 copy, per layout of a unit: L_TILED for the tensor-core
     // contraction, L_PLAIN for the others.  Each is held in the layout that the selected contractions read; in both, one
