@@ -38,6 +38,7 @@
 // releases it and stores its own rows.  All waits are bounded (2 s, error codes 41 to 43).  The kernels do not let their
 // dependents start early: with k_by's blocks waiting from the first wave on, k_by and k_bx after it took 52 and 33 us
 // instead of 29 and 24 (complex128, 128x128x32; whole apply 343 -> 321 us, 64x128x27 151 -> 144, pair 277 -> 275).
+#include <atomic>
 #include <cstdint>
 #include "common.cuh"
 #include "ie_internal.h"
@@ -638,6 +639,16 @@ constexpr int stages_of(int bytes)
     return n > 16 ? 16 : n;
 }
 
+// all shared memory for a kernel, asked for until the call has succeeded once
+template <class K> int allow_smem(K kern, std::atomic<bool> &ready)
+{
+    if (!ready) {
+        G2_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+        ready = true;
+    }
+    return G2_OK;
+}
+
 template <typename C, class K>
 int launch_mma(K kern, int nthreads, int multiple, int pts, const void *G, void *Uhat, int Nx, int Ny, int Nz, int *err,
                cudaStream_t st, const int *gate)
@@ -660,16 +671,16 @@ template <int KT1, int KT2, int NG>
 int launch_mma64(const void *G, void *U, int Nx, int Ny, int Nz, int *err, cudaStream_t st, const int *gate)
 {
     auto kern = k_contract_mma64<KT1, KT2, NG>;
-    static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-    G2_CUDA_CHECK(attr);
+    static std::atomic<bool> ready{false};
+    if (const int rc = allow_smem(kern, ready)) return rc;
     return launch_mma<double2>(kern, MmaCfg64<KT1, KT2, NG>::NTHREADS, NG, 4, G, U, Nx, Ny, Nz, err, st, gate);
 }
 template <int NP, int KZ, bool HALF, int NG>
 int launch_mma32(const void *G, void *U, int Nx, int Ny, int Nz, int *err, cudaStream_t st, const int *gate)
 {
     auto kern = k_contract_mma32<NP, KZ, HALF, NG>;
-    static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-    G2_CUDA_CHECK(attr);
+    static std::atomic<bool> ready{false};
+    if (const int rc = allow_smem(kern, ready)) return rc;
     return launch_mma<float2>(kern, MmaCfg32<KZ, NG>::NTHREADS, 1, 4 * NP, G, U, Nx, Ny, Nz, err, st, gate);
 }
 // groups for about `want` warps, at most `most`
