@@ -65,7 +65,7 @@ G2_D void finish_load(Finish &f, const Level &L, int j)
     if (t == 64) f.bn = L.scal[S_BN];
     if (t == 65) f.iter = L.flags[F_ITER];
 }
-G2_D void finish_step(Finish &f, double2 *hc, Level &L, int j, double nrm, double dloo, double tol)
+G2_D void finish_step(Finish &f, double2 *hc, Level &L, int j, double nrm, double tol)
 {
     const int m = L.m, lane = threadIdx.x & 31;
     const double dnormw = sqrt(nrm);
@@ -102,8 +102,6 @@ G2_D void finish_step(Finish &f, double2 *hc, Level &L, int j, double nrm, doubl
         L.H[hix(j, m, m)] = f.g[0];
         L.H[hix(j + 1, m, m)] = f.g[1];
         L.scal[S_NRM2] = nrm;
-        L.scal[S_DLOO] = dloo;
-        L.scal[S_DNORMW] = dnormw;
         L.flags[F_ITER] = f.iter + 1;
         L.flags[F_L] = j + 1;
     }
@@ -250,7 +248,6 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
     reduce_partials(mm.part[y], gridDim.x, K, hs, nullptr);
     if (threadIdx.x < K) hsum[threadIdx.x] = hs[threadIdx.x];
     __syncthreads();
-    double dloo;
     for (int p = 1;; p++) {
         // w -= V hs; dots and norm of the new w
         clear();
@@ -318,8 +315,7 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
         // gmres.F90:277-280
         double dl = 0.0;
         for (int k = 0; k < K; k++) dl += hs[k].x * hs[k].x + hs[k].y * hs[k].y;
-        dloo = sqrt(dl);
-        if (2.0 * sqrt(nrm) > dloo || p > N_IGS) break;
+        if (2.0 * sqrt(nrm) > sqrt(dl) || p > N_IGS) break;
         __syncthreads();
         if (threadIdx.x < K) {
             hsum[threadIdx.x].x += hn[threadIdx.x].x;
@@ -329,7 +325,7 @@ __global__ void __launch_bounds__(kVT) k_arnoldi(Multi<C> mm, size_t N, double t
         __syncthreads();
     }
     // every block has read its gate, a flag that the step's end may clear: all of them passed the barriers above
-    if (blockIdx.x == 0 && threadIdx.x < 32) return finish_step(fin, hsum, L, j, nrm, dloo, tol);
+    if (blockIdx.x == 0 && threadIdx.x < 32) return finish_step(fin, hsum, L, j, nrm, tol);
     const double inv = 1.0 / sqrt(nrm);
     if (HOLD && Nw)
         scale_rows<true>(ww, reinterpret_cast<W *>(V) + (size_t)K * ldw, Nw, S, [&](W x) {

@@ -485,13 +485,6 @@ static int arnoldi_step1(KrylovWork *k, Level &L, C *V, int j, C *w, double tol,
     mm.gate[0] = gate;
     return arnoldi_step(mm, 1, k->N, k->nparts, j, tol, k->err, st);
 }
-// the same for n lockstep instances (vector length N, nparts partial-sum slots each) in one launch
-template <typename C>
-static int arnoldi_step_multi(const Multi<C> &mm, int n, size_t N, int nparts, int j, double tol, int *err, cudaStream_t st)
-{
-    return arnoldi_step(mm, n, N, nparts, j, tol, err, st);
-}
-
 template <typename C> static int apply_prec(IeOp *op, const C *in, C *out, cudaStream_t st, const int *gate);
 template <> int apply_prec<double2>(IeOp *op, const double2 *in, double2 *out, cudaStream_t st, const int *gate)
 {
@@ -995,7 +988,7 @@ static int batch_inner(BatchWork *b, double tol, cudaStream_t st)
                     mm.L[q] = k->Li;
                     mm.gate[q] = k->Li.flags + F_KRYLOV;
                 }
-                const int r = arnoldi_step_multi<CI>(mm, (int)(e - c), k0->N, k0->nparts, j, tol, k0->err, st);
+                const int r = arnoldi_step(mm, (int)(e - c), k0->N, k0->nparts, j, tol, k0->err, st);
                 if (r) return r;
             }
             c = e;
@@ -1299,7 +1292,7 @@ static int batch_outer(BatchWork *b, const GIEM2G_FGMRES_CTL &ctl, GIEM2G_RESULT
                         mm.gate[q] = k->Lo.flags + F_KRYLOV;
                     }
                     KrylovWork *k0 = b->k[act[0]];
-                    if ((r = arnoldi_step_multi<double2>(mm, 2, k0->N, k0->nparts, j, tol, k0->err, st))) return r;
+                    if ((r = arnoldi_step(mm, 2, k0->N, k0->nparts, j, tol, k0->err, st))) return r;
                 } else {
                     for (int i : act) {
                         KrylovWork *k = b->k[i];

@@ -58,7 +58,7 @@ constexpr int N_IGS = 3;                  // gmres.F90:22
 constexpr double kHookGain = 0.5;         // an outer step through the hook must halve the misfit
 
 enum { F_KRYLOV = 0, F_L = 2, F_ITER = 3, F_SOLVER = 4, F_NFLAGS = 8 };
-enum { S_BN = 0, S_BETA = 1, S_DNORMW = 2, S_DLOO = 3, S_BEA = 4, S_NRM2 = 5, S_NSCAL = 8 };
+enum { S_BN = 0, S_BETA = 1, S_BEA = 4, S_NRM2 = 5, S_NSCAL = 8 };
 
 G2_HD int hix(int i, int j, int m) { return i + j * (m + 1); }
 
