@@ -356,14 +356,14 @@ int giem2g_apply_ie_operator_device_static(void *ie, const void *d_in, void *d_o
         return fail(G2_ERR_ARG, "giem2g_apply_ie_operator_device_static: precision must be 0 or 1");
     note_capture(op);
     void *base = nullptr;
-    size_t cap = 0, n_u1 = 0;
-    rc = ie_static_scratch(&base, &cap);
+    size_t cap = 0, array = 0, n_u1 = 0;
+    rc = ie_static_scratch(&base, &cap, &array);
     if (rc) return fail(rc, "giem2g_apply_ie_operator_device_static: static scratch set-up failed: %s",
                         giem2g_last_error());
     const size_t es = precision == 0 ? sizeof(double2) : sizeof(float2);
     const size_t n_all = ie_apply_scratch_elems(op, &n_u1);
     const size_t off_uh = (n_u1 * es + 255) / 256 * 256;
-    // the limit counts the rows of the spectrum without their padding, which the array has room for
+    // the limit counts the rows of the spectrum without their padding
     const size_t pad = op->units() * 4 * (ie_spectrum_pitch(op->Nz) - 3 * op->Nz);
     const size_t need = off_uh + (n_all - n_u1 - pad) * es;
     if (need > cap)
@@ -371,6 +371,12 @@ int giem2g_apply_ie_operator_device_static(void *ie, const void *d_in, void *d_o
                     "giem2g_apply_ie_operator_device_static: grid %dx%dx%d needs %zu bytes of scratch at precision "
                     "%d, above the static maximum of %zu bytes; use giem2g_apply_ie_operator_device",
                     op->Nx, op->Ny, op->Nz, need, precision, cap);
+    const size_t padded = off_uh + (n_all - n_u1) * es;
+    if (padded > array)
+        return fail(G2_ERR_ARG,
+                    "giem2g_apply_ie_operator_device_static: grid %dx%dx%d needs %zu bytes of scratch at precision "
+                    "%d, more than the static array's %zu; use giem2g_apply_ie_operator_device",
+                    op->Nx, op->Ny, op->Nz, padded, precision, array);
     unsigned char *b = static_cast<unsigned char *>(base);
     cudaEventRecord(op->ev0, op->stream);
     if (precision == 0)

@@ -121,7 +121,7 @@ int ie_contract_pair32(const float2 *G, float2 *Uhat, int Nx, int Ny, int Nz, in
 int ie_contract_pair_variants(int Nz);
 // Process-wide static scratch of the static-scratch apply: device address (set-up on first use per
 // device) and capacity in bytes.
-int ie_static_scratch(void **ptr, size_t *capacity);
+int ie_static_scratch(void **ptr, size_t *limit, size_t *array);  // of unpadded intermediates; bytes there are
 // 3x3x3 convolution data movement (channels-last): im2col (bf16) and its gather-form adjoint (fp32)
 int ie_im2col3d(const void *x, void *cols, int N, int D, int H, int W, int C, int s, int Kp, cudaStream_t st);
 int ie_col2im3d(const float *dcols, float *dx, int N, int D, int H, int W, int C, int s, int Kp, cudaStream_t st);

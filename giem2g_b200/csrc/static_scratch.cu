@@ -14,9 +14,12 @@
 // Limits and rules:
 //   - capacity kStaticScratchBytes (32 MiB).  The apply needs 18*Nx*Ny*Nz complex elements
 //     (U1 6*Nx*Ny*Nz, Uhat 12*Nx*Ny*Nz): 16 B each for precision 0, 8 B for precision 1, so e.g.
-//     64x64x16 fits at both precisions and 128x128x32 fits at neither.  (The array itself is 40 MiB:
-//     the tensor-core contraction pads the spectrum's rows of 3Nz elements, at Nz = 1 to 22 for 18.)  Larger grids are rejected
+//     64x64x16 fits at both precisions and 128x128x32 fits at neither.  Larger grids are rejected
 //     with G2_ERR_ARG and a message; they keep using giem2g_apply_ie_operator_device.
+//   - the array itself is 40 MiB: the tensor-core contraction pads the spectrum's rows of 3Nz elements to 4 mod 8 (Nz = 2:
+//     6 to 12, 30 for 18 in all).  A grid of the limit would need up to 53 MiB that way, but the lateral counts are powers of
+//     two, and the most that a grid within the limit needs is 38.5 MiB (Nz = 7).  The caller compares the padded need with
+//     the array all the same.
 //   - every call on a device shares the one array.  Nothing in it has to start at zero (every
 //     element is written before it is read within a call), but two calls whose executions overlap
 //     on the GPU race on it and both results are undefined.  Every operator owns its own stream, so
@@ -65,10 +68,11 @@ CtxGetCurrentFn ctx_get_current()
 
 }  // namespace
 
-int ie_static_scratch(void **ptr, size_t *capacity)
+int ie_static_scratch(void **ptr, size_t *limit, size_t *array)
 {
     *ptr = nullptr;
-    *capacity = kStaticScratchBytes;
+    *limit = kStaticScratchBytes;
+    *array = kStaticArrayBytes;
     int dev = -1;
     G2_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) return G2_ERR_UNSUPPORTED;
