@@ -8,7 +8,8 @@
 // instance.  The launch is cooperative, so all blocks are resident; the waits are bounded (2 s, error code 51).
 // Whole solves, launches per sweep -> one launch with its barriers, the last scalar step beside the scaling and the scaling
 // four words at a time: FP64 32x32x8 3.31 -> 2.30 ms, mixed pairs 128x128x32 2 ms of 66 (bound by the sweeps' HBM and L2
-// traffic).
+// traffic); with the correction sweep backwards, the cycle start in two launches and sums in FP64 beyond 16 elements 2.0 ms
+// and, of such a pair's 60 ms, 11.3.
 #include <atomic>
 #include <type_traits>
 #include <utility>

@@ -29,7 +29,7 @@
 // of M (padded within (x, y) and within z, so that the sign of out_z is one per tile); complex64 warps own the x, y and
 // z rows of eight z, which lets one split of an xy tile serve two products.
 // What bounds it at 128x128x32 (16384 units): complex128 HBM (tensor and spectrum twice, 1.29 GB: 200 us at the measured
-// copy rate, 215-221 us measured); paired complex64 the TF32 pipe (864 instructions of 8-9 clocks per SM partition and unit,
+// copy rate, 218 us measured); paired complex64 the TF32 pipe (864 instructions of 8-9 clocks per SM partition and unit,
 // 110 us) plus the splits' instructions, which overlap with it only in part (178 us; the FP32 kernels of contract.cu
 // take 180 to 293 us); single complex64 the same splits for half the products (142 us).
 //

@@ -68,9 +68,10 @@ struct IeOp {
     int precision_mode = 0;            // 0 plain FP64, 1 mixed (c64 inner)
     bool use_fast_contract = true;     // GIEM2G_GENERIC_CONTRACT=1 selects the generic contraction kernel
     // contraction of FP64, complex64 and paired complex64 applies: a tile-shape variant of contract.cu, or -1 for
-    // the tensor-core kernel (contract_mma.cu), the default: it takes every Nz, and at 128x128x32 it beats variant 0
-    // in every form (FP64 221 against 280 us, complex64 154 against 174, paired 178 against 293); the best of its shapes, which the
-    // autotuner finds, take 207, 115 and 180 us there
+    // the tensor-core kernel (contract_mma.cu), the default.  It takes every Nz.  Where contract.cu has shapes, whole applies
+    // with it are the fastest or within 4 % of the fastest in FP64 and in pairs, and 9 to 18 % behind in single complex64
+    // (Nz = 16, 48, 32; contraction alone at 128x128x32, default and best shape: FP64 218 and 207 us, complex64 142 and 115,
+    // paired 178 and 180), where the autotuner finds the other one.
     int contract_variant[3] = {-1, -1, -1};
     // fused y-transforms + contraction (ypipe.cu) per form: its variant, or -1 for the separate passes
     // (k_fy, contraction, k_by).  The separate passes are the default (faster at 128x128x32 on a B200);
