@@ -60,10 +60,15 @@ def _second_tensor_fits(op, free_bytes: int) -> bool:
 
 def _one_layout(single_ms, pair_ms):
     """The picks of the complex64 and the paired apply that read the same layout: the fastest paired one, and the fastest
-    single one of its layout (0 reads one, all others the other)."""
-    pair = min(range(len(pair_ms)), key=pair_ms.__getitem__)
-    group = [0] if pair == 0 else range(1, len(single_ms))
-    return min(group, key=single_ms.__getitem__), pair
+    single one of its layout (0 reads one, all others the other).  None: not timed."""
+    def fastest(group, ms):
+        return min((v for v in group if ms[v] is not None), key=ms.__getitem__)
+
+    pair = fastest(range(len(pair_ms)), pair_ms)
+    try:
+        return fastest([0] if pair == 0 else range(1, len(single_ms)), single_ms), pair
+    except ValueError:  # no single shape of the pair's layout could be timed
+        return 0, 0
 
 
 def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, rounds: int = 3) -> dict:
@@ -78,6 +83,7 @@ def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, round
             cache = {}
     stream = torch.cuda.ExternalStream(op.stream)
     picks = {}
+    fused = None  # whether the grid has the fused pass
     from . import Giem2gError, apply_device_batch
     for prec, dt in ((0, torch.complex128), (1, torch.complex64), (2, torch.complex64)):
         nv = op.contract_variants(prec)
@@ -102,14 +108,22 @@ def autotune_contraction(op, reps: int = 5, cache_path: str | None = None, round
 
         best, all_ms = None, []
         for v in range(nv):
+            if v == nv - 1 and fused is False:
+                all_ms.append(None)  # the default's second name
+                continue
             try:
                 op.set_contract_variant(prec, v)
             except Giem2gError:
                 if v == 0:
                     raise
-                all_ms.append(float("inf"))  # no memory for its layout of the tensor
+                all_ms.append(None)  # no memory for its layout of the tensor
                 continue
             ms = _time_rounds(run, stream, reps, rounds)
+            if v == nv - 1 and prec == 0:  # the last number: the fused pass (three launches), or the default again
+                fused = op.last_kernel_launches() == 3
+                if not fused:
+                    all_ms.append(None)
+                    continue
             all_ms.append(round(ms, 5))
             if best is None or ms < best[1]:
                 best = (v, ms)

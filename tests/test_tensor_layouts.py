@@ -16,6 +16,8 @@ def test_tuner_weighs_the_second_tensor():
     # the paired apply decides, the single one follows in its layout
     assert _one_layout([0.20, 0.25, 0.17], [0.28, 0.40, 0.30]) == (0, 0)
     assert _one_layout([0.10, 0.25, 0.17], [0.28, 0.40, 0.27]) == (2, 2)
+    assert _one_layout([0.10, 0.25, None], [0.28, 0.27, None]) == (1, 1)
+    assert _one_layout([0.10, None, None], [0.28, 0.27, None]) == (0, 0)
 
 
 def _op(g2, m, seed=13):
@@ -140,4 +142,21 @@ def test_captured_apply_outlives_selections_and_new_tensors(g2lib, variant):
     torch.cuda.synchronize()
     assert np.array_equal(yd.cpu().numpy(), second) and not np.array_equal(second, first)
     del graph
+    op.delete()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fits", [True, False])
+def test_tuner_keeps_one_layout_when_memory_is_short(g2lib, monkeypatch, fits):
+    """A grid without the fused pass: its last number is the default again and is not picked; without room for a second
+    tensor the complex64 and the paired apply get kernels of one layout."""
+    import giem2g_b200.autotune as at
+    monkeypatch.setattr(at, "_second_tensor_fits", lambda op, free: fits)
+    m = tiny_model(32, 32, 16)
+    op = _op(g2lib, m)
+    picks = at.autotune_contraction(op, reps=2, rounds=1)
+    for form in (0, 1, 2):
+        assert 0 <= picks[str(form)]["variant"] < op.contract_variants(form) - 1
+    if not fits:
+        assert (picks["1"]["variant"] == 0) == (picks["2"]["variant"] == 0)
     op.delete()
